@@ -47,7 +47,7 @@ def build(force: bool = False) -> None:
     os.makedirs(os.path.dirname(LIB), exist_ok=True)
     if force or not os.path.exists(LIB) or os.path.getmtime(LIB) < os.path.getmtime(src):
         subprocess.run(["gcc", "-O2", "-shared", "-fPIC", "-o", LIB, src, "-lm"], check=True)
-    if os.path.isdir(REFERENCE_DIR):
+    if os.path.isfile(os.path.join(REFERENCE_DIR, "Algorithms", "BFS", "bfs.cu")):
         root = os.path.dirname(HERE)
         deps = [os.path.join(HERE, "ref_wrap.cpp"), os.path.join(HERE, "build_ref.sh"),
                 os.path.join(root, "tests", "cpp", "gas_ref_programs.cu"),
