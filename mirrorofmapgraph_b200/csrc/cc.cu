@@ -10,15 +10,18 @@
 // larger root under the smaller one with atomicCAS: parent pointers only
 // decrease, so every root is its component's minimum and the final labels equal
 // the reference's bit for bit. The edge work follows the sampling scheme of
-// Afforest (Sutton et al., IPDPS 2018):
-//   1. mg_tuning.cc_rounds rounds (1 by default) link every vertex to its first
-//      neighbours, then compress;
-//   2. one CTA samples 1024 vertices and takes the most frequent root c (on
+// Afforest (Sutton et al., IPDPS 2018), started from a forest that costs no
+// atomics:
+//   1. every vertex points at the smallest of itself and its first CC_FIRST
+//      neighbours, then the trees are compressed;
+//   2. mg_tuning.cc_rounds rounds (1 by default) unite every vertex with its
+//      first neighbours, then compress;
+//   3. one CTA samples 1024 vertices and takes the most frequent root c (on
 //      power-law graphs, the giant component);
-//   3. only vertices outside c process their remaining edges (and, without a
+//   4. only vertices outside c process their remaining edges (and, without a
 //      symmetric adjacency, their in-edges too); then compress.
 // Any edge with both endpoints skipped joins two members of c's tree already, so
-// the result does not depend on the sample.
+// the result does not depend on the sample or on the first forest.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -32,6 +35,8 @@ namespace mg {
 constexpr int CC_NT = 256;
 constexpr int CC_CTA_TH = 1024;
 constexpr int CC_SAMPLES = 1024;
+constexpr int CC_V = 4;      // vertices a thread holds in flight
+constexpr int CC_FIRST = 4;  // neighbours the first forest looks at
 
 // Root of x with path halving. Parent entries are read from L2 (ld.cg): they are
 // rewritten concurrently, and every value ever stored is an ancestor, so a
@@ -47,8 +52,14 @@ __device__ __forceinline__ int32_t uf_find(int32_t *p, int32_t x) {
   return x;
 }
 
+// Unites the trees of a and b. Two vertices with the same parent are in one tree
+// already: after a compression that is nearly every edge, and it costs two loads
+// where two finds cost four.
 __device__ __forceinline__ void uf_union(int32_t *p, int32_t a, int32_t b) {
-  int32_t ra = uf_find(p, a), rb = uf_find(p, b);
+  int32_t ra = __ldcg(p + a), rb = __ldcg(p + b);
+  if (ra == rb) return;
+  ra = uf_find(p, ra);
+  rb = uf_find(p, rb);
   while (ra != rb) {
     const int32_t hi = max(ra, rb), lo = min(ra, rb);
     const int32_t old = atomicCAS(p + hi, hi, lo);
@@ -64,11 +75,30 @@ __global__ void cc_init_kernel(int32_t *p, int64_t n) {
     p[i] = (int32_t)i;
 }
 
+// The first forest: p[v] = min(v, v's first CC_FIRST neighbours). Every vertex
+// writes only its own entry and pointers decrease, so there is no atomic and no
+// cycle. It matters where a row's first neighbour is arbitrary (rows in edge-list
+// order): one sampling round from singletons then leaves many middle-sized trees
+// (42-58% of the edges outside the largest on R-MAT graphs, every one of which the
+// last pass walks), one round from this forest under 0.1%.
+__global__ void __launch_bounds__(CC_NT) cc_first_kernel(const int32_t *__restrict__ ro,
+                                                         const int32_t *__restrict__ ci, int64_t n, int32_t *p) {
+  for (int64_t v = (int64_t)blockIdx.x * CC_NT + threadIdx.x; v < n; v += (int64_t)gridDim.x * CC_NT) {
+    const int32_t b = ro[v], e = ro[v + 1];
+    int32_t mn = (int32_t)v;
+#pragma unroll
+    for (int k = 0; k < CC_FIRST; k++)
+      if (b + k < e) mn = min(mn, ci[b + k]);
+    p[v] = mn;
+  }
+}
+
 // Sampling rounds r0 .. r1 - 1: v is united with its r-th neighbour in each
 // (the union-find result does not depend on the order of the unions).
-__global__ void cc_sample_link_kernel(const int32_t *__restrict__ ro, const int32_t *__restrict__ ci, int64_t n,
-                                      int32_t *p, int r0, int r1) {
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(CC_NT) cc_sample_link_kernel(const int32_t *__restrict__ ro,
+                                                               const int32_t *__restrict__ ci, int64_t n, int32_t *p,
+                                                               int r0, int r1) {
+  for (int64_t v = (int64_t)blockIdx.x * CC_NT + threadIdx.x; v < n; v += (int64_t)gridDim.x * CC_NT) {
     const int32_t b = ro[v], e = ro[v + 1];
     for (int r = r0; r < r1 && b + r < e; r++) {
       const int32_t u = ci[b + r];
@@ -77,59 +107,71 @@ __global__ void cc_sample_link_kernel(const int32_t *__restrict__ ro, const int3
   }
 }
 
-__global__ void cc_compress_kernel(int32_t *p, int32_t *label, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t r = (int32_t)i;
-    int32_t par = __ldcg(p + r);
-    while (par != r) {
-      r = par;
-      par = __ldcg(p + r);
+// Points every vertex at its root (into p, or into label for the final pass).
+// CC_V independent walks per thread, with path halving on the way: the first
+// forest of a lattice is chains as long as a column.
+__global__ void __launch_bounds__(CC_NT) cc_compress_kernel(int32_t *p, int32_t *label, int64_t n) {
+  for (int64_t t0 = (int64_t)blockIdx.x * CC_NT * CC_V; t0 < n; t0 += (int64_t)gridDim.x * CC_NT * CC_V) {
+    int32_t par[CC_V], gp[CC_V];
+#pragma unroll
+    for (int k = 0; k < CC_V; k++) {
+      const int64_t i = t0 + k * CC_NT + threadIdx.x;
+      par[k] = i < n ? __ldcg(p + i) : 0;
     }
-    if (label) label[i] = r;
-    else __stcg(p + i, r);
+#pragma unroll
+    for (int k = 0; k < CC_V; k++) gp[k] = __ldcg(p + par[k]);
+#pragma unroll
+    for (int k = 0; k < CC_V; k++) {
+      const int64_t i = t0 + k * CC_NT + threadIdx.x;
+      if (i >= n) continue;
+      const int32_t r = gp[k] == par[k] ? par[k] : uf_find(p, gp[k]);
+      if (label) label[i] = r;
+      else if (r != par[k]) __stcg(p + i, r);
+    }
   }
 }
 
 // Most frequent root among CC_SAMPLES hashed vertices (one CTA of CC_SAMPLES
-// threads); writes it to *out.
+// threads), counted in an open-addressed table in shared memory; writes it to *out.
 __global__ void __launch_bounds__(CC_SAMPLES) cc_mode_kernel(const int32_t *p, int64_t n, int32_t *out) {
-  __shared__ int32_t s[CC_SAMPLES];
+  __shared__ int32_t key[2 * CC_SAMPLES], cnt[2 * CC_SAMPLES];
   __shared__ unsigned long long best;
   const int t = threadIdx.x;
+  for (int i = t; i < 2 * CC_SAMPLES; i += CC_SAMPLES) {
+    key[i] = -1;
+    cnt[i] = 0;
+  }
+  if (t == 0) best = 0ull;
   uint64_t h = (uint64_t)t * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull;
   h ^= h >> 31;
   h *= 0xBF58476D1CE4E5B9ull;
   h ^= h >> 29;
-  s[t] = __ldcg(p + (int64_t)(h % (uint64_t)n));
-  if (t == 0) best = 0ull;
+  const int32_t r = __ldcg(p + (int64_t)(h % (uint64_t)n));
   __syncthreads();
-  for (int size = 2; size <= CC_SAMPLES; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const int j = t ^ stride;
-      if (j > t) {
-        const bool up = (t & size) == 0;
-        const int32_t a = s[t], b = s[j];
-        if ((a > b) == up) {
-          s[t] = b;
-          s[j] = a;
-        }
-      }
-      __syncthreads();
+  // lanes with the same root add once
+  const unsigned same = __match_any_sync(FULL, r);
+  const bool lead = (same & lanemask_lt()) == 0;
+  if (lead) {
+    unsigned at = ((unsigned)r * 2654435761u) >> 21;  // 2048 slots for at most 1024 keys
+    for (;;) {
+      const int32_t k = atomicCAS(key + at, -1, r);
+      if (k == -1 || k == r) break;
+      at = (at + 1) & (2 * CC_SAMPLES - 1);
     }
+    atomicAdd(cnt + at, __popc(same));
   }
-  if (t == 0 || s[t] != s[t - 1]) {
-    int len = 1;
-    while (t + len < CC_SAMPLES && s[t + len] == s[t]) len++;
-    // larger count first, then the smaller root
-    const unsigned long long key = ((unsigned long long)len << 32) | (unsigned)(INT_MAX - s[t]);
-    atomicMax(&best, key);
-  }
+  __syncthreads();
+  for (int i = t; i < 2 * CC_SAMPLES; i += CC_SAMPLES)
+    if (cnt[i] > 0)  // larger count first, then the smaller root
+      atomicMax(&best, ((unsigned long long)cnt[i] << 32) | (unsigned)(INT_MAX - key[i]));
   __syncthreads();
   if (t == 0) *out = INT_MAX - (int32_t)(best & 0xffffffffu);
 }
 
-// Phase 3: every vertex whose root is not c unites all its remaining edges
-// (from index `skip` of its CSR row; all in-edges too when `both`).
+// Phase 4: every vertex whose root is not c unites all its remaining edges
+// (from index `skip` of its CSR row; all in-edges too when `both`). A CTA looks at
+// CC_NT x CC_V vertices at a time and gathers the few that are outside c and have
+// edges left before it expands them.
 __global__ void __launch_bounds__(CC_NT) cc_finish_kernel(const int32_t *__restrict__ ro,
                                                           const int32_t *__restrict__ ci,
                                                           const int32_t *__restrict__ co,
@@ -138,22 +180,40 @@ __global__ void __launch_bounds__(CC_NT) cc_finish_kernel(const int32_t *__restr
                                                           unsigned long long *insp_out) {
   __shared__ ExpandSmem<CC_NT> sm;
   __shared__ int64_t s_sum[CC_NT / 32 + 1];
+  __shared__ int32_t s_list[CC_NT * CC_V], s_len;
   const int32_t c = *cptr;
   int64_t insp = 0;
-  for (int64_t tile = (int64_t)blockIdx.x * CC_NT; tile < n; tile += (int64_t)gridDim.x * CC_NT) {
-    const int64_t i = tile + threadIdx.x;
-    int32_t v = i < n ? (int32_t)i : -1;
-    if (v >= 0 && __ldcg(p + v) == c) v = -1;
-    expand_tile<CC_NT, CC_CTA_TH>(sm, ro, v, insp, [&](int32_t sv, int32_t k) {
-      if (k - __ldg(ro + sv) < skip) return;
-      const int32_t u = ci[k];
-      if (u != sv) uf_union(p, sv, u);
-    });
-    if (both)
-      expand_tile<CC_NT, CC_CTA_TH>(sm, co, v, insp, [&](int32_t sv, int32_t k) {
-        const int32_t u = ri[k];
+  for (int64_t t0 = (int64_t)blockIdx.x * CC_NT * CC_V; t0 < n; t0 += (int64_t)gridDim.x * CC_NT * CC_V) {
+    if (threadIdx.x == 0) s_len = 0;
+    __syncthreads();
+    int32_t par[CC_V];
+#pragma unroll
+    for (int k = 0; k < CC_V; k++) {
+      const int64_t i = t0 + k * CC_NT + threadIdx.x;
+      par[k] = i < n ? __ldcg(p + i) : c;
+    }
+#pragma unroll
+    for (int k = 0; k < CC_V; k++) {
+      const int64_t i = t0 + k * CC_NT + threadIdx.x;
+      if (par[k] != c && (ro[i + 1] - ro[i] > skip || (both && co[i + 1] > co[i])))
+        s_list[atomicAdd(&s_len, 1)] = (int32_t)i;
+    }
+    __syncthreads();
+    const int32_t len = s_len;
+    for (int32_t l0 = 0; l0 < len; l0 += CC_NT) {
+      const int32_t v = l0 + threadIdx.x < len ? s_list[l0 + threadIdx.x] : -1;
+      expand_tile<CC_NT, CC_CTA_TH>(sm, ro, v, insp, [&](int32_t sv, int32_t k) {
+        if (k - __ldg(ro + sv) < skip) return;
+        const int32_t u = ci[k];
         if (u != sv) uf_union(p, sv, u);
       });
+      if (both)
+        expand_tile<CC_NT, CC_CTA_TH>(sm, co, v, insp, [&](int32_t sv, int32_t k) {
+          const int32_t u = ri[k];
+          if (u != sv) uf_union(p, sv, u);
+        });
+    }
+    __syncthreads();
   }
   const int64_t b = block_sum<CC_NT>(insp, s_sum);
   if (threadIdx.x == 0 && b) atomicAdd(insp_out, (unsigned long long)b);
@@ -207,26 +267,29 @@ extern "C" mg_status mg_cc(mg_graph *g, int32_t *label, const mg_opts *opts, mg_
   MG_CUDA_TRY(cudaEventRecord(g->ev0, s));
   const int grid = g->num_sms * 8;
   int64_t launches = 0;
-  cc_init_kernel<<<grid, 256, 0, s>>>(parent, n);
-  launches++;
-  // Neighbour-sampling rounds before the giant component is picked: R-MAT s22
-  // 0.33 / 0.41 / 0.48 ms with 1 / 2 / 3 rounds. With none, only the sampled
-  // root's own self-loops are skipped, so every count gives the same labels.
+  // Neighbour-sampling rounds before the giant component is picked. With none,
+  // the largest tree of the first forest is skipped, so every count gives the same
+  // labels.
   const int32_t rounds = g->tune.cc_rounds;
+  const int64_t per = (int64_t)CC_NT * CC_V;
+  const int gv = (int)std::min<int64_t>(std::max<int64_t>((n + per - 1) / per, 1), g->num_sms * 8);
   if (n > 0 && sampling) {
+    cc_first_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent);
+    cc_compress_kernel<<<gv, CC_NT, 0, s>>>(parent, nullptr, n);
     // one launch per round: every vertex's first link lands before any second
     // (two rounds in one pass measured 0.51 against 0.41 ms on R-MAT s22)
-    for (int r = 0; r < rounds; r++) cc_sample_link_kernel<<<grid, 256, 0, s>>>(g->ro, g->ci, n, parent, r, r + 1);
-    cc_compress_kernel<<<grid, 256, 0, s>>>(parent, nullptr, n);
+    for (int r = 0; r < rounds; r++) cc_sample_link_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent, r, r + 1);
+    cc_compress_kernel<<<gv, CC_NT, 0, s>>>(parent, nullptr, n);
     cc_mode_kernel<<<1, CC_SAMPLES, 0, s>>>(parent, n, cmode);
-    cc_finish_kernel<<<g->num_sms * 4, CC_NT, 0, s>>>(g->ro, g->ci, g->co, g->ri, n, parent, cmode, rounds,
-                                                      symmetric ? 0 : 1, insp);
-    launches += rounds + 3;
+    cc_finish_kernel<<<gv, CC_NT, 0, s>>>(g->ro, g->ci, g->co, g->ri, n, parent, cmode, rounds, symmetric ? 0 : 1,
+                                          insp);
+    launches += rounds + 5;
   } else if (n > 0) {
+    cc_init_kernel<<<grid, 256, 0, s>>>(parent, n);
     cc_all_edges_kernel<<<g->num_sms * 4, CC_NT, 0, s>>>(g->ro, g->ci, n, parent, insp);
-    launches++;
+    launches += 2;
   }
-  cc_compress_kernel<<<grid, 256, 0, s>>>(parent, out, n);
+  cc_compress_kernel<<<gv, CC_NT, 0, s>>>(parent, out, n);
   launches++;
   MG_CUDA_TRY(cudaGetLastError());
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
