@@ -10,18 +10,20 @@
 // larger root under the smaller one with atomicCAS: parent pointers only
 // decrease, so every root is its component's minimum and the final labels equal
 // the reference's bit for bit. The edge work follows the sampling scheme of
-// Afforest (Sutton et al., IPDPS 2018), started from a forest that costs no
-// atomics:
+// Afforest (Sutton et al., IPDPS 2018): a cheap forest over a few edges of every
+// vertex first, and only what lies outside its largest tree walks all its edges.
+// The forest needs no union to succeed, so it is built without compare-and-swap:
 //   1. every vertex points at the smallest of itself and its first CC_FIRST
 //      neighbours, then the trees are compressed;
-//   2. mg_tuning.cc_rounds rounds (1 by default) unite every vertex with its
-//      first neighbours, then compress;
+//   2. 1 + mg_tuning.cc_rounds passes over the next CC_HOOK neighbours hook the
+//      larger of the two roots under the smaller one by a fire-and-forget minimum,
+//      each followed by a compression; a root hooked twice keeps the smaller link;
 //   3. one CTA samples 1024 vertices and takes the most frequent root c (on
 //      power-law graphs, the giant component);
-//   4. only vertices outside c process their remaining edges (and, without a
-//      symmetric adjacency, their in-edges too); then compress.
+//   4. only vertices outside c unite all their edges (and, without a symmetric
+//      adjacency, their in-edges too), by union-find; then compress.
 // Any edge with both endpoints skipped joins two members of c's tree already, so
-// the result does not depend on the sample or on the first forest.
+// the result does not depend on the sample or on the forest.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -37,6 +39,7 @@ constexpr int CC_CTA_TH = 1024;
 constexpr int CC_SAMPLES = 1024;
 constexpr int CC_V = 4;      // vertices a thread holds in flight
 constexpr int CC_FIRST = 4;  // neighbours the first forest looks at
+constexpr int CC_HOOK = 2;   // neighbours a hooking pass looks at
 
 // Root of x with path halving. Parent entries are read from L2 (ld.cg): they are
 // rewritten concurrently, and every value ever stored is an ancestor, so a
@@ -77,10 +80,7 @@ __global__ void cc_init_kernel(int32_t *p, int64_t n) {
 
 // The first forest: p[v] = min(v, v's first CC_FIRST neighbours). Every vertex
 // writes only its own entry and pointers decrease, so there is no atomic and no
-// cycle. It matters where a row's first neighbour is arbitrary (rows in edge-list
-// order): one sampling round from singletons then leaves many middle-sized trees
-// (42-58% of the edges outside the largest on R-MAT graphs, every one of which the
-// last pass walks), one round from this forest under 0.1%.
+// cycle.
 __global__ void __launch_bounds__(CC_NT) cc_first_kernel(const int32_t *__restrict__ ro,
                                                          const int32_t *__restrict__ ci, int64_t n, int32_t *p) {
   for (int64_t v = (int64_t)blockIdx.x * CC_NT + threadIdx.x; v < n; v += (int64_t)gridDim.x * CC_NT) {
@@ -93,23 +93,39 @@ __global__ void __launch_bounds__(CC_NT) cc_first_kernel(const int32_t *__restri
   }
 }
 
-// Sampling rounds r0 .. r1 - 1: v is united with its r-th neighbour in each
-// (the union-find result does not depend on the order of the unions).
-__global__ void __launch_bounds__(CC_NT) cc_sample_link_kernel(const int32_t *__restrict__ ro,
-                                                               const int32_t *__restrict__ ci, int64_t n, int32_t *p,
-                                                               int r0, int r1) {
+// Hooking pass over neighbours [r0, r0 + CC_HOOK) of every vertex, on compressed
+// trees. Bound by its random parent reads. With atomicCAS unions in its place (one
+// neighbour each) the sampled roots are few and hot: R-MAT s22, rows in edge-list
+// order, 466 us from singletons and 737 us from the first forest; two passes of
+// this kernel and the whole run take 300 us.
+// Rows whose first neighbours are arbitrary need the minimum to spread: from
+// singletons one round leaves 42-58% of an R-MAT graph's edges outside the largest
+// tree (every one walked by the last pass, 10 ms at s22), the first forest and one
+// hooking pass 0.4%, two passes nothing but the small components.
+__global__ void __launch_bounds__(CC_NT) cc_hook_kernel(const int32_t *__restrict__ ro,
+                                                        const int32_t *__restrict__ ci, int64_t n, int32_t *p,
+                                                        int r0) {
   for (int64_t v = (int64_t)blockIdx.x * CC_NT + threadIdx.x; v < n; v += (int64_t)gridDim.x * CC_NT) {
-    const int32_t b = ro[v], e = ro[v + 1];
-    for (int r = r0; r < r1 && b + r < e; r++) {
-      const int32_t u = ci[b + r];
-      if (u != v) uf_union(p, (int32_t)v, u);
+    const int32_t b = ro[v] + r0, e = ro[v + 1];
+    if (b >= e) continue;
+    const int32_t pv = __ldcg(p + v);
+    int32_t pu[CC_HOOK];
+#pragma unroll
+    for (int k = 0; k < CC_HOOK; k++) pu[k] = b + k < e ? __ldca(p + ci[b + k]) : pv;
+#pragma unroll
+    for (int k = 0; k < CC_HOOK; k++) {
+      const int32_t hi = max(pv, pu[k]), lo = min(pv, pu[k]);
+      if (lo < __ldca(p + hi) && lo < __ldcg(p + hi)) red_min(p + hi, lo);
     }
   }
 }
 
 // Points every vertex at its root (into p, or into label for the final pass).
 // CC_V independent walks per thread, with path halving on the way: the first
-// forest of a lattice is chains as long as a column.
+// forest of a lattice is chains as long as a column. Parents are read through L1:
+// a stale one is an older ancestor, roots do not change here, and nearly every
+// walk ends at the same root, whose one L2 sector 130,000 warps would queue for
+// (the last pass on R-MAT s22 43 us from L2).
 __global__ void __launch_bounds__(CC_NT) cc_compress_kernel(int32_t *p, int32_t *label, int64_t n) {
   for (int64_t t0 = (int64_t)blockIdx.x * CC_NT * CC_V; t0 < n; t0 += (int64_t)gridDim.x * CC_NT * CC_V) {
     int32_t par[CC_V], gp[CC_V];
@@ -119,7 +135,7 @@ __global__ void __launch_bounds__(CC_NT) cc_compress_kernel(int32_t *p, int32_t 
       par[k] = i < n ? __ldcg(p + i) : 0;
     }
 #pragma unroll
-    for (int k = 0; k < CC_V; k++) gp[k] = __ldcg(p + par[k]);
+    for (int k = 0; k < CC_V; k++) gp[k] = __ldca(p + par[k]);
 #pragma unroll
     for (int k = 0; k < CC_V; k++) {
       const int64_t i = t0 + k * CC_NT + threadIdx.x;
@@ -168,15 +184,14 @@ __global__ void __launch_bounds__(CC_SAMPLES) cc_mode_kernel(const int32_t *p, i
   if (t == 0) *out = INT_MAX - (int32_t)(best & 0xffffffffu);
 }
 
-// Phase 4: every vertex whose root is not c unites all its remaining edges
-// (from index `skip` of its CSR row; all in-edges too when `both`). A CTA looks at
-// CC_NT x CC_V vertices at a time and gathers the few that are outside c and have
-// edges left before it expands them.
+// Phase 4: every vertex whose root is not c unites all its edges (all in-edges
+// too when `both`). A CTA looks at CC_NT x CC_V vertices at a time and gathers the
+// few that are outside c and have edges before it expands them.
 __global__ void __launch_bounds__(CC_NT) cc_finish_kernel(const int32_t *__restrict__ ro,
                                                           const int32_t *__restrict__ ci,
                                                           const int32_t *__restrict__ co,
                                                           const int32_t *__restrict__ ri, int64_t n, int32_t *p,
-                                                          const int32_t *cptr, int skip, int both,
+                                                          const int32_t *cptr, int both,
                                                           unsigned long long *insp_out) {
   __shared__ ExpandSmem<CC_NT> sm;
   __shared__ int64_t s_sum[CC_NT / 32 + 1];
@@ -195,7 +210,7 @@ __global__ void __launch_bounds__(CC_NT) cc_finish_kernel(const int32_t *__restr
 #pragma unroll
     for (int k = 0; k < CC_V; k++) {
       const int64_t i = t0 + k * CC_NT + threadIdx.x;
-      if (par[k] != c && (ro[i + 1] - ro[i] > skip || (both && co[i + 1] > co[i])))
+      if (par[k] != c && (ro[i + 1] > ro[i] || (both && co[i + 1] > co[i])))
         s_list[atomicAdd(&s_len, 1)] = (int32_t)i;
     }
     __syncthreads();
@@ -203,7 +218,6 @@ __global__ void __launch_bounds__(CC_NT) cc_finish_kernel(const int32_t *__restr
     for (int32_t l0 = 0; l0 < len; l0 += CC_NT) {
       const int32_t v = l0 + threadIdx.x < len ? s_list[l0 + threadIdx.x] : -1;
       expand_tile<CC_NT, CC_CTA_TH>(sm, ro, v, insp, [&](int32_t sv, int32_t k) {
-        if (k - __ldg(ro + sv) < skip) return;
         const int32_t u = ci[k];
         if (u != sv) uf_union(p, sv, u);
       });
@@ -267,23 +281,21 @@ extern "C" mg_status mg_cc(mg_graph *g, int32_t *label, const mg_opts *opts, mg_
   MG_CUDA_TRY(cudaEventRecord(g->ev0, s));
   const int grid = g->num_sms * 8;
   int64_t launches = 0;
-  // Neighbour-sampling rounds before the giant component is picked. With none,
-  // the largest tree of the first forest is skipped, so every count gives the same
-  // labels.
+  // Hooking passes beyond the first before the giant component is picked; every
+  // count gives the same labels.
   const int32_t rounds = g->tune.cc_rounds;
   const int64_t per = (int64_t)CC_NT * CC_V;
   const int gv = (int)std::min<int64_t>(std::max<int64_t>((n + per - 1) / per, 1), g->num_sms * 8);
   if (n > 0 && sampling) {
     cc_first_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent);
     cc_compress_kernel<<<gv, CC_NT, 0, s>>>(parent, nullptr, n);
-    // one launch per round: every vertex's first link lands before any second
-    // (two rounds in one pass measured 0.51 against 0.41 ms on R-MAT s22)
-    for (int r = 0; r < rounds; r++) cc_sample_link_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent, r, r + 1);
-    cc_compress_kernel<<<gv, CC_NT, 0, s>>>(parent, nullptr, n);
+    for (int r = 0; r <= rounds; r++) {
+      cc_hook_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent, r * CC_HOOK);
+      cc_compress_kernel<<<gv, CC_NT, 0, s>>>(parent, nullptr, n);
+    }
     cc_mode_kernel<<<1, CC_SAMPLES, 0, s>>>(parent, n, cmode);
-    cc_finish_kernel<<<gv, CC_NT, 0, s>>>(g->ro, g->ci, g->co, g->ri, n, parent, cmode, rounds, symmetric ? 0 : 1,
-                                          insp);
-    launches += rounds + 5;
+    cc_finish_kernel<<<gv, CC_NT, 0, s>>>(g->ro, g->ci, g->co, g->ri, n, parent, cmode, symmetric ? 0 : 1, insp);
+    launches += 2 * rounds + 6;
   } else if (n > 0) {
     cc_init_kernel<<<grid, 256, 0, s>>>(parent, n);
     cc_all_edges_kernel<<<g->num_sms * 4, CC_NT, 0, s>>>(g->ro, g->ci, n, parent, insp);
@@ -299,7 +311,7 @@ extern "C" mg_status mg_cc(mg_graph *g, int32_t *label, const mg_opts *opts, mg_
     std::memset(stats, 0, sizeof(*stats));
     stats->iterations = 1;
     stats->edges_traversed = g->m;
-    stats->edges_inspected = g->ctl_host->edges_inspected + (sampling ? (int64_t)rounds * n : 0);
+    stats->edges_inspected = g->ctl_host->edges_inspected + (sampling ? (int64_t)(rounds + 1) * n : 0);
     // offsets and sampled neighbours, the remaining edges actually read, parent
     // init / compress passes
     stats->bytes_compulsory = 4 * (n + 1) + 4 * stats->edges_inspected + 16 * n;
