@@ -137,24 +137,23 @@ static mg_status bin_plan_build_impl(cudaStream_t s, const int32_t *off, int64_t
   int64_t *totals = counts + nchunks * (PRB_BINS + 1);
   int64_t *dboff = totals + (PRB_BINS + 1);
   prb_count_kernel<<<(unsigned)nchunks, PRB_NT, 0, s>>>(off, n, counts, heavy);
-  prb_offsets_kernel<<<1, 32, 0, s>>>(counts, nchunks, totals);
+  prb_offsets_kernel<<<1, 32 * (PRB_BINS + 1), 0, s>>>(counts, nchunks, totals);
   int64_t cnt[PRB_BINS + 1];
   MG_CUDA_TRY(cudaMemcpyAsync(cnt, totals, sizeof(cnt), cudaMemcpyDeviceToHost, s));
   MG_CUDA_TRY(cudaStreamSynchronize(s));
   int64_t acc = 0;
   for (int b = 0; b < PRB_BINS; b++) {
     bp.boff[b] = acc;
-    if (b < 6) acc += cnt[b];
+    if (b < PRB_HUB) acc += cnt[b];
   }
   bp.boff[PRB_BINS] = acc;
-  bp.boff[6] = acc;
-  bp.nheavy = cnt[6];
+  bp.nheavy = cnt[PRB_HUB];
   bp.ntasks = cnt[PRB_BINS];
-  // One warp assignment per 32 rows of bins 0..5, one per hub chunk.
+  // Warp assignments: the bins' rows, then one per hub chunk.
   int64_t w = 0;
   for (int b = 0; b < PRB_BINS; b++) {
     bp.wstart[b] = w;
-    if (b < 6) w += (cnt[b] + 31) / 32;
+    if (b < PRB_HUB) w += (cnt[b] + prb_rows_per(b) - 1) / prb_rows_per(b);
     else w += bp.ntasks;
   }
   bp.wstart[PRB_BINS] = w;
@@ -458,13 +457,6 @@ __global__ void __launch_bounds__(PRB_NT, PRB_MIN_BLOCKS) solve_binned_kernel(So
 #ifndef PRB_HUB_CAP
 #define PRB_HUB_CAP 40960
 #endif
-// Rounds of the warp-per-row gather sized to the row's tail (prb_warp_range's
-// ADAPT) in the column-cache kernel. Measured on R-MAT s22 (us per iteration,
-// static schedule): 640 threads with ADAPT 591, 768 with ADAPT 628, 768 without
-// 599, 640 without 774.
-#ifndef PRB_HUB_ADAPT
-#define PRB_HUB_ADAPT true
-#endif
 constexpr int PRB_HUB_NT = PRB_HUB_THREADS;
 
 template <bool WEIGHTED>
@@ -494,8 +486,7 @@ __global__ void __launch_bounds__(PRB_HUB_NT, PRB_HUB_MINB) solve_binned_hub_ker
     p.hcontrib[2 * h + 1] = hu.red2;
     __threadfence();
   };
-  prb_run<WEIGHTED, PRB_HUB_ADAPT>(p, [&](int32_t col) { return col < 0 ? s_hub[col & 0x7fffffff] : __ldg(gold + col); }, up,
-                    hub);
+  prb_run<WEIGHTED>(p, [&](int32_t col) { return col < 0 ? s_hub[col & 0x7fffffff] : __ldg(gold + col); }, up, hub);
   const double r = block_sum<PRB_HUB_NT>(up.resid, s_red);
   const double d = block_sum<PRB_HUB_NT>(up.red2, s_red);
   if (threadIdx.x == 0) {
@@ -1371,7 +1362,7 @@ static mg_status solve_setup(mg_graph *g, bool adjoint, bool weighted, const flo
       sp.p.idx = seg->sidx;
       if (weighted) sp.p.wts = seg->swts;
       sp.p.grab = bins->grab;  // phase 2 always takes items from the counter
-      sp.p.wstart[PRB_BINS] = sp.p.wstart[6];  // hub rows are phase 1's, not work items of phase 2
+      sp.p.wstart[PRB_BINS] = sp.p.wstart[PRB_HUB];  // hub rows are phase 1's, not work items of phase 2
       sp.sg = SegArgs{seg->ent,  seg->gofs, seg->pidx,   seg->pwts,  seg->bgrp,  seg->cta,
                       seg->bdense, (n + 31) & ~(int64_t)31, seg->S, seg->nblocks, seg->rrow, seg->rgofs,
                       seg->ridx, seg->rwts, seg->rgrab, seg->nrgroups, seg->nrgroups_e, seg->nrgroups_l,
@@ -1995,7 +1986,7 @@ static mg_status pagerank_ppr(mg_graph *g, const float *tele_dev, int32_t nvec, 
   a.idx = g->ri;
   a.wts = weighted ? (const float *)g->cvals : nullptr;
   a.rows = bins->rows;
-  a.nlight = bins->boff[6];
+  a.nlight = bins->boff[PRB_HUB];
   a.hrows = bins->hrows;
   a.hbase = bins->hbase;
   a.nheavy = nheavy;
@@ -2202,22 +2193,46 @@ __global__ void __launch_bounds__(PRB_NT) adj_rows_kernel(PrbArgs p, const float
                     [&](int64_t, int32_t row, Comp v) { st(row, v); });
 }
 
-// dL/da_uv = coef[u] * (lambda_v - pl[u]) for every CSR edge, rows expanded with
-// the degree-binned tile expansion (coalesced index loads and gradient stores).
-__global__ void __launch_bounds__(256) adj_edge_grad_kernel(const int32_t *__restrict__ ro,
-                                                            const int32_t *__restrict__ ci, int64_t n,
-                                                            const float *__restrict__ lam,
-                                                            const double *__restrict__ pl,
-                                                            const double *__restrict__ coef, float *__restrict__ grad) {
-  __shared__ ExpandSmem<256> sm;
-  int64_t insp = 0;
-  for (int64_t tile = (int64_t)blockIdx.x * 256; tile < n; tile += (int64_t)gridDim.x * 256) {
-    const int64_t i = tile + threadIdx.x;
-    const int32_t v = i < n ? (int32_t)i : -1;
-    expand_tile<256, 1024>(sm, ro, v, insp, [&](int32_t u, int32_t k) {
-      grad[k] = (float)(coef[u] * ((double)__ldg(lam + ci[k]) - pl[u]));
-    });
-  }
+// dL/da_uv = coef[u] * (lambda_v - pl[u]) for every CSR edge, over the rows of the
+// bin plan: a lane takes 8 edges of its row at a time (16-byte index loads and, on
+// an aligned gradient array, 16-byte stores). The random lambda reads bound it; in
+// tiles of 256 consecutive vertices the few tiles with the hubs ran alone at the
+// end (R-MAT s22 directed, 67 M edges: 5.4 ms).
+__global__ void __launch_bounds__(PRB_NT) adj_edge_grad_kernel(PrbArgs p, const float *__restrict__ lam,
+                                                               const double *__restrict__ pl,
+                                                               const double *__restrict__ coef,
+                                                               float *__restrict__ grad) {
+  const bool vec = (reinterpret_cast<uintptr_t>(grad) & 15) == 0;
+  prb_walk(p, [&](auto lanes, int32_t row, int32_t b, int32_t e, int sub, int64_t, int64_t) {
+    constexpr int L = decltype(lanes)::value > 0 ? decltype(lanes)::value : 1;
+    const double cf = row >= 0 ? coef[row] : 0.0, mean = row >= 0 ? pl[row] : 0.0;
+    for (int32_t k0 = (b & ~3) + 4 * sub; k0 < e; k0 += 8 * L) {
+      const int32_t k1 = k0 + 4 * L;
+      int4 c[2];
+      c[0] = prb_stream(reinterpret_cast<const int4 *>(p.idx + k0));
+      c[1] = k1 < e ? prb_stream(reinterpret_cast<const int4 *>(p.idx + k1)) : make_int4(0, 0, 0, 0);
+      float x[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int32_t k = j < 4 ? k0 + j : k1 + j - 4;
+        const int4 &q = c[j >> 2];
+        x[j] = k >= b && k < e ? __ldg(lam + ((j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w)) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) x[j] = (float)(cf * ((double)x[j] - mean));
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int32_t k = h ? k1 : k0;
+        if (vec && k >= b && k + 3 < e) {
+          __stcs(reinterpret_cast<float4 *>(grad + k), make_float4(x[4 * h], x[4 * h + 1], x[4 * h + 2], x[4 * h + 3]));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (k + j >= b && k + j < e) grad[k + j] = x[4 * h + j];
+        }
+      }
+    }
+  });
 }
 
 // Dangling rank mass of x: per-block partials, then one block.
@@ -2327,7 +2342,7 @@ extern "C" mg_status mg_pagerank_backward(mg_graph *g, const float *teleport, co
     AdjRowStore st{a.srow, x_dev, pl, coef, a.alpha};
     if (weighted) adj_rows_kernel<true><<<g->num_sms * 8, PRB_NT, 0, s>>>(rp, lam, st);
     else adj_rows_kernel<false><<<g->num_sms * 8, PRB_NT, 0, s>>>(rp, lam, st);
-    adj_edge_grad_kernel<<<g->num_sms * 8, 256, 0, s>>>(g->ro, g->ci, n, lam, pl, coef, gw);
+    adj_edge_grad_kernel<<<g->num_sms * 8, PRB_NT, 0, s>>>(rp, lam, pl, coef, gw);
     launches += 2;
   }
   if (dL_dteleport) {

@@ -1,23 +1,33 @@
 // pr_binned.cuh -- degree-binned gather over a CSR-shaped adjacency, the default
 // PageRank / adjoint gather.
 //
-// Rows are binned once per adjacency by degree and each bin gets the lane count
-// that covers its rows in one pass:
-//   bin 0..4  degree <= 1, 2, 4, 8, 16: groups of 1, 2, 4, 8, 16 lanes per row
-//             (32 / G rows per warp), each group reads its row's edges with
-//             consecutive lanes and reduces with a shuffle tree of log2 G steps;
-//   bin 5     degree < PRB_HEAVY: one warp per row, 32 consecutive edges per step;
-//   bin 6     degree >= PRB_HEAVY (hubs): split into chunks of PRB_CHUNK edges; a
-//             warp reduces one chunk into a partial; the warp that completes a
-//             hub's last chunk (per-row arrival counter) adds the partials in
-//             chunk order and finishes the row.
-// Warps are independent (no CTA barriers while gathering) and every edge load is
-// a coalesced stream. The per-row sums are compensated (TwoSum per addend,
-// FMA-based TwoProduct for weights) and every row's sum has a fixed order, so the
-// result does not depend on scheduling. A persistent grid walks the assignments
-// with a fixed stride, so each CTA's FP64 partials (residual, dangling mass) are
-// deterministic too; hub rows keep their contributions in a per-hub array.
+// Rows are binned once per adjacency by degree, and each bin gets the lane count
+// that keeps a warp's loads in flight without idle lanes:
+//   bin 0       no edges: only the row update;
+//   bin 1       1 or 2 edges: one lane per row, plain loads;
+//   bins 2..9   up to 64 edges: one lane per row, classes narrow enough that the
+//               32 rows of a warp end together. A lane reads its row's indices as
+//               16-byte vectors and gathers 8 values before its first add, so a
+//               warp keeps up to 256 gathers in flight, with no shuffles;
+//   bin 10      65..256 edges: 4 lanes per row, 8 rows per warp;
+//   bin 11      up to PRB_HEAVY: one warp per row, 256 edges per step;
+//   bin 12      degree >= PRB_HEAVY (hubs): split into chunks of PRB_CHUNK edges; a
+//               warp reduces one chunk into a partial; the warp that completes a
+//               hub's last chunk (per-row arrival counter) adds the partials in
+//               chunk order and finishes the row.
+// The random gathers bound it, and before them the number in flight: with a warp
+// per row above 16 edges and 32 such rows per work item, a warp waited for two
+// round trips per row and the items of the heaviest rows ran last and alone
+// (R-MAT s22 directed, weighted, 67 M edges: 451 us per iteration, 380 with these
+// bins; symmetric, unweighted, 134 M edges: 542 and 530).
+// Warps are independent (no CTA barriers while gathering). The per-row sums are
+// compensated (TwoSum per addend, FMA-based TwoProduct for weights) and every
+// row's sum has a fixed order, so the result does not depend on scheduling. A
+// persistent grid takes the assignments from a counter (or with a fixed stride);
+// hub rows keep their FP64 contributions in a per-hub array.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "pr_gather.cuh"
@@ -25,18 +35,15 @@
 namespace mg {
 
 constexpr int PRB_NT = 256;
-constexpr int PRB_BINS = 7;
-// Resident CTAs per SM the iteration kernel is compiled for, and how many passes
-// of a light bin issue their loads before the first reduction.
+constexpr int PRB_BINS = 13;
+constexpr int PRB_QUAD = 10;  // first bin of more than one lane per row (4 lanes)
+constexpr int PRB_WARP = 11;  // a warp per row
+constexpr int PRB_HUB = 12;   // hub rows
+// Rows of one warp assignment of a bin.
+__host__ __device__ constexpr int prb_rows_per(int bin) { return bin < PRB_QUAD ? 32 : bin == PRB_QUAD ? 8 : 2; }
+// Resident CTAs per SM the iteration kernel is compiled for.
 #ifndef PRB_MIN_BLOCKS
-#define PRB_MIN_BLOCKS 6
-#endif
-#ifndef PRB_BATCH
-#define PRB_BATCH 8
-#endif
-// Strides of 32 edges a warp-per-row gather loads before its first add.
-#ifndef PRB_UNROLL
-#define PRB_UNROLL 8
+#define PRB_MIN_BLOCKS 5
 #endif
 // Index (and weight) streams are read once per iteration: loads marked
 // evict-first (ld.global.cs) keep them from displacing the gathered vector in
@@ -55,34 +62,24 @@ __device__ __forceinline__ T prb_stream(const T *p) {
 #ifndef PRB_HEAVY_EDGES
 #define PRB_HEAVY_EDGES 2048
 #endif
-// Assignment order of a persistent warp: 1 walks the plan from the hub chunks and
-// the heaviest bins down to the lightest (longest items first shortens the
-// tail); 0 walks bins 0..6 in order.
 // Solve kernels take their work items from a shared counter (1) or by a fixed
 // grid stride (0).
 #ifndef PRB_DYNAMIC
 #define PRB_DYNAMIC 1
-#endif
-// Work items a warp takes per grab of the dynamic schedule.
-#ifndef PRB_GRAB
-#define PRB_GRAB 1
-#endif
-#ifndef PRB_HEAVY_FIRST
-#define PRB_HEAVY_FIRST 1
 #endif
 constexpr int32_t PRB_HEAVY = PRB_HEAVY_EDGES;
 constexpr int32_t PRB_CHUNK = 2048;
 
 // Plan of one adjacency.
 struct BinPlan {
-  int32_t *rows = nullptr;      // rows grouped by bin (bins 0..5), bin b at rows[boff[b]..]
-  int32_t *hrows = nullptr;     // hub rows (bin 6)
+  int32_t *rows = nullptr;      // rows grouped by bin (hubs apart), bin b at rows[boff[b]..]
+  int32_t *hrows = nullptr;     // hub rows
   int32_t *hbase = nullptr;     // first chunk task of each hub, nheavy + 1 entries
   int32_t *hcount = nullptr;    // arrival counters of the hubs (reset by the finishing warp)
   Comp *hpart = nullptr;        // partial sums of the hub chunks
   double *hcontrib = nullptr;   // per-hub FP64 contributions (residual, second reduction)
   int32_t *grab = nullptr;      // work-item counter of the dynamic schedule (zero between launches)
-  int64_t boff[PRB_BINS + 1] = {0};  // bin offsets into rows (bin 6 unused)
+  int64_t boff[PRB_BINS + 1] = {0};  // bin offsets into rows
   int64_t nheavy = 0, ntasks = 0;
   int64_t wstart[PRB_BINS + 1] = {0};  // first warp assignment of each bin
 };
@@ -97,15 +94,14 @@ void bin_plan_release(cudaStream_t s, mg::BinPlan &bp);
 
 namespace mg {
 
-// Bin of a row of `deg` edges; rows of at least `heavy` edges are hubs (bin 6).
+// Bin of a row of `deg` edges; rows of at least `heavy` edges are hubs.
 __device__ __forceinline__ int prb_bin_of(int32_t deg, int32_t heavy = PRB_HEAVY) {
-  if (deg >= heavy) return 6;
-  if (deg <= 1) return 0;
-  if (deg <= 2) return 1;
-  if (deg <= 4) return 2;
-  if (deg <= 8) return 3;
-  if (deg <= 16) return 4;
-  return 5;
+  if (deg >= heavy) return PRB_HUB;
+  if (deg <= 8) return deg <= 2 ? (deg + 1) >> 1 : deg <= 4 ? 2 : 3;
+  if (deg <= 16) return deg <= 12 ? 4 : 5;
+  if (deg <= 32) return deg <= 24 ? 6 : 7;
+  if (deg <= 64) return deg <= 48 ? 8 : 9;
+  return deg <= 256 ? PRB_QUAD : PRB_WARP;
 }
 
 // Ordered binning. Rows are cut into chunks of PRB_NT * PRB_RPT rows, one per
@@ -117,67 +113,101 @@ constexpr int PRB_RPT = 8;
 constexpr int PRB_CHUNK_ROWS = PRB_NT * PRB_RPT;
 
 #ifndef MG_PRB_NO_PLAN_KERNELS  // plan building runs in pagerank.cu only
+// Bins of a thread's PRB_RPT consecutive rows from r0 (-1 past the end).
+__device__ __forceinline__ void prb_bins_of(const int32_t *__restrict__ off, int64_t n, int64_t r0, int32_t heavy,
+                                            int (&bins)[PRB_RPT], int32_t &chunks) {
+  int32_t o[PRB_RPT + 1];
+#pragma unroll
+  for (int k = 0; k <= PRB_RPT; k++) o[k] = off[min(r0 + k, n)];
+  chunks = 0;
+#pragma unroll
+  for (int k = 0; k < PRB_RPT; k++) {
+    const int32_t d = o[k + 1] - o[k];
+    bins[k] = r0 + k < n ? prb_bin_of(d, heavy) : -1;
+    if (bins[k] == PRB_HUB) chunks += (d + PRB_CHUNK - 1) / PRB_CHUNK;
+  }
+}
+
+// Counts are summed over a warp packed seven to a word (9 bits each: a warp has
+// 256 rows), then added to the CTA's counters by one lane per warp and bin.
 __global__ void __launch_bounds__(PRB_NT) prb_count_kernel(const int32_t *__restrict__ off, int64_t n,
                                                            int64_t *__restrict__ counts /* [chunk][BINS+1] */,
                                                            int32_t heavy) {
-  __shared__ int64_t s[PRB_BINS + 1];
+  __shared__ int32_t s[PRB_BINS + 1];
   if (threadIdx.x <= PRB_BINS) s[threadIdx.x] = 0;
   __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * PRB_CHUNK_ROWS;
+  int bins[PRB_RPT];
+  int32_t chunks;
+  prb_bins_of(off, n, (int64_t)blockIdx.x * PRB_CHUNK_ROWS + (int64_t)threadIdx.x * PRB_RPT, heavy, bins, chunks);
+  unsigned long long w0 = 0, w1 = 0;
+#pragma unroll
   for (int k = 0; k < PRB_RPT; k++) {
-    const int64_t r = base + (int64_t)threadIdx.x * PRB_RPT + k;
-    if (r < n) {
-      const int32_t d = off[r + 1] - off[r];
-      const int b = prb_bin_of(d, heavy);
-      atomicAdd((unsigned long long *)&s[b], 1ull);
-      if (b == 6) atomicAdd((unsigned long long *)&s[PRB_BINS], (unsigned long long)((d + PRB_CHUNK - 1) / PRB_CHUNK));
-    }
+    if (bins[k] >= 7) w1 += 1ull << (9 * (bins[k] - 7));
+    else if (bins[k] >= 0) w0 += 1ull << (9 * bins[k]);
   }
+  w0 = warp_sum(w0);
+  w1 = warp_sum(w1);
+  const int lane = lane_id();
+  if (lane < PRB_BINS) {
+    const int32_t v = (int32_t)((lane < 7 ? w0 >> (9 * lane) : w1 >> (9 * (lane - 7))) & 511);
+    if (v) atomicAdd(s + lane, v);
+  }
+  if (chunks) atomicAdd(s + PRB_BINS, chunks);
   __syncthreads();
   if (threadIdx.x <= PRB_BINS) counts[(int64_t)blockIdx.x * (PRB_BINS + 1) + threadIdx.x] = s[threadIdx.x];
 }
 
-// Exclusive prefix over chunks of every bin, in place; totals[b] = bin sizes.
-__global__ void prb_offsets_kernel(int64_t *counts, int64_t nchunks, int64_t *totals) {
-  const int b = threadIdx.x;
-  if (b > PRB_BINS) return;
+// Exclusive prefix over chunks of every bin, in place (a warp per bin);
+// totals[b] = bin sizes.
+__global__ void __launch_bounds__(32 * (PRB_BINS + 1)) prb_offsets_kernel(int64_t *counts, int64_t nchunks,
+                                                                          int64_t *totals) {
+  const int b = warp_id(), lane = lane_id();
   int64_t acc = 0;
-  for (int64_t c = 0; c < nchunks; c++) {
-    const int64_t v = counts[c * (PRB_BINS + 1) + b];
-    counts[c * (PRB_BINS + 1) + b] = acc;
-    acc += v;
+  for (int64_t c0 = 0; c0 < nchunks; c0 += 32) {
+    const int64_t c = c0 + lane;
+    const int64_t v = c < nchunks ? counts[c * (PRB_BINS + 1) + b] : 0;
+    const int64_t inc = warp_inclusive_scan(v);
+    if (c < nchunks) counts[c * (PRB_BINS + 1) + b] = acc + inc - v;
+    acc += __shfl_sync(FULL, inc, 31);
   }
-  totals[b] = acc;
+  if (lane == 0) totals[b] = acc;
 }
 
 __global__ void __launch_bounds__(PRB_NT) prb_scatter_kernel(const int32_t *__restrict__ off, int64_t n,
                                                              const int64_t *__restrict__ offsets,
                                                              const int64_t *__restrict__ boff, int32_t *rows,
                                                              int32_t *hrows, int32_t heavy) {
-  __shared__ int32_t red[PRB_NT / 32 + 1];
-  const int64_t base = (int64_t)blockIdx.x * PRB_CHUNK_ROWS;
+  // a CTA has 2048 rows: four bins to a 64-bit word, 16 bits each
+  constexpr int NW = (PRB_BINS + 3) / 4;
+  __shared__ unsigned long long red[PRB_NT / 32 + 1];
+  const int64_t r0 = (int64_t)blockIdx.x * PRB_CHUNK_ROWS + (int64_t)threadIdx.x * PRB_RPT;
   int bins[PRB_RPT];
+  int32_t chunks;
+  prb_bins_of(off, n, r0, heavy, bins, chunks);
+  unsigned long long pos[NW];
+#pragma unroll
+  for (int w = 0; w < NW; w++) {
+    unsigned long long c = 0, tot;
+#pragma unroll
+    for (int k = 0; k < PRB_RPT; k++)
+      if (bins[k] >= 0 && (bins[k] >> 2) == w) c += 1ull << (16 * (bins[k] & 3));
+    pos[w] = block_exclusive_scan<PRB_NT>(c, red, &tot);
+  }
 #pragma unroll
   for (int k = 0; k < PRB_RPT; k++) {
-    const int64_t r = base + (int64_t)threadIdx.x * PRB_RPT + k;
-    bins[k] = r < n ? prb_bin_of(off[r + 1] - off[r], heavy) : -1;
-  }
-  for (int b = 0; b < PRB_BINS; b++) {
-    int cnt = 0;
+    const int b = bins[k];
+    if (b < 0) continue;
+    int32_t at = 0;
 #pragma unroll
-    for (int k = 0; k < PRB_RPT; k++) cnt += bins[k] == b;
-    int32_t tot;
-    int pos = block_exclusive_scan<PRB_NT>(cnt, red, &tot);
-    const int64_t o = offsets[(int64_t)blockIdx.x * (PRB_BINS + 1) + b];
-#pragma unroll
-    for (int k = 0; k < PRB_RPT; k++) {
-      if (bins[k] == b) {
-        const int32_t r = (int32_t)(base + (int64_t)threadIdx.x * PRB_RPT + k);
-        if (b < 6) rows[boff[b] + o + pos] = r;
-        else hrows[o + pos] = r;
-        pos++;
+    for (int w = 0; w < NW; w++) {
+      if ((b >> 2) == w) {
+        at = (int32_t)((pos[w] >> (16 * (b & 3))) & 0xffff);
+        pos[w] += 1ull << (16 * (b & 3));
       }
     }
+    const int64_t o = offsets[(int64_t)blockIdx.x * (PRB_BINS + 1) + b] + at;
+    if (b == PRB_HUB) hrows[o] = (int32_t)(r0 + k);
+    else rows[boff[b] + o] = (int32_t)(r0 + k);
   }
 }
 
@@ -219,18 +249,6 @@ struct PrbArgs {
   int64_t nheavy;
 };
 
-template <bool WEIGHTED>
-__device__ __forceinline__ void prb_add(Comp &acc, float g, const float *__restrict__ wts, int32_t k) {
-  if (WEIGHTED) {
-    const float a = prb_stream(wts + k);
-    const float p = a * g;
-    two_sum_add(acc, p);
-    acc.lo += __fmaf_rn(a, g, -p);
-  } else {
-    two_sum_add(acc, g);
-  }
-}
-
 template <int G>
 __device__ __forceinline__ void group_comp_reduce(Comp &c) {
 #pragma unroll
@@ -245,200 +263,182 @@ __device__ __forceinline__ void group_comp_reduce(Comp &c) {
   }
 }
 
-// U strides of 32 edges of a row from `base` (warp-uniform); CHECK predicates
-// each slot on the row end (the last round of a row).
-template <bool WEIGHTED, int U, bool CHECK, typename Gather>
-__device__ __forceinline__ void prb_round(const PrbArgs &p, int32_t base, int32_t e, Gather &gather, Comp &acc) {
-  const int32_t k = base + (threadIdx.x & 31);
-  int32_t c[U];
-  float x[U];
-#pragma unroll
-  for (int j = 0; j < U; j++) c[j] = (!CHECK || k + 32 * j < e) ? prb_stream(p.idx + k + 32 * j) : 0;
-#pragma unroll
-  for (int j = 0; j < U; j++) x[j] = (!CHECK || k + 32 * j < e) ? gather(c[j]) : 0.f;
-#pragma unroll
-  for (int j = 0; j < U; j++)
-    if (!CHECK || k + 32 * j < e) prb_add<WEIGHTED>(acc, x[j], p.wts, k + 32 * j);
-}
-
-// One warp reduces edges [b, e) of a row in rounds of PRB_UNROLL strides of 32
-// edges (all loads of a round in flight together). ADAPT: full rounds run without
-// per-slot checks and the last round is sized to what is left (8, 4, 2 or 1
-// strides), so short rows do not pay for idle slots; otherwise each lane walks
-// its own edges in full predicated rounds (fewer code paths, which suits some
-// register-tight launch shapes).
-template <bool WEIGHTED, bool ADAPT, typename Gather>
-__device__ __forceinline__ Comp prb_warp_range(const PrbArgs &p, int32_t b, int32_t e, Gather &gather) {
+// Compensated sum of edges [b, e) by the L lanes of a group (sub: the lane's place
+// in it), 8 edges per lane and step: two 16-byte index loads (the lanes of a group
+// side by side) from the row's start rounded down to a vector, 8 gathers, then the
+// adds. Slots outside the row add +0, which a compensated sum does not notice; the
+// index and weight arrays are padded by 8 entries, so the last vector may run over
+// the row's (or the array's) end. Lanes of other groups may end earlier.
+template <int L, bool WEIGHTED, typename Gather>
+__device__ __forceinline__ Comp prb_group_range(const PrbArgs &p, int32_t b, int32_t e, int sub, Gather &gather) {
   Comp acc{0.f, 0.f};
-  if (ADAPT) {
-    int32_t base = b;
-    for (; base + 32 * PRB_UNROLL <= e; base += 32 * PRB_UNROLL)
-      prb_round<WEIGHTED, PRB_UNROLL, false>(p, base, e, gather, acc);
-    const int32_t rem = e - base;
-    if (rem > 128) prb_round<WEIGHTED, PRB_UNROLL, true>(p, base, e, gather, acc);
-    else if (rem > 64) prb_round<WEIGHTED, 4, true>(p, base, e, gather, acc);
-    else if (rem > 32) prb_round<WEIGHTED, 2, true>(p, base, e, gather, acc);
-    else if (rem > 0) prb_round<WEIGHTED, 1, true>(p, base, e, gather, acc);
-  } else {
-    // per-lane loop: a lane stops after its last edge
-    for (int32_t k = b + (threadIdx.x & 31); k < e; k += 32 * PRB_UNROLL) {
-      int32_t c[PRB_UNROLL];
-      float x[PRB_UNROLL];
+  for (int32_t k0 = (b & ~3) + 4 * sub; k0 < e; k0 += 8 * L) {
+    int32_t c[8];
+    float x[8];
+    float w[8];
+    const int32_t k1 = k0 + 4 * L;
+    const int4 i0 = prb_stream(reinterpret_cast<const int4 *>(p.idx + k0));
+    const int4 i1 = k1 < e ? prb_stream(reinterpret_cast<const int4 *>(p.idx + k1)) : make_int4(0, 0, 0, 0);
+    if (WEIGHTED) {
+      const float4 w0 = prb_stream(reinterpret_cast<const float4 *>(p.wts + k0));
+      const float4 w1 =
+          k1 < e ? prb_stream(reinterpret_cast<const float4 *>(p.wts + k1)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      w[0] = w0.x, w[1] = w0.y, w[2] = w0.z, w[3] = w0.w;
+      w[4] = w1.x, w[5] = w1.y, w[6] = w1.z, w[7] = w1.w;
+    }
+    c[0] = i0.x, c[1] = i0.y, c[2] = i0.z, c[3] = i0.w;
+    c[4] = i1.x, c[5] = i1.y, c[6] = i1.z, c[7] = i1.w;
 #pragma unroll
-      for (int j = 0; j < PRB_UNROLL; j++) c[j] = k + 32 * j < e ? prb_stream(p.idx + k + 32 * j) : 0;
+    for (int j = 0; j < 8; j++) {
+      const int32_t k = j < 4 ? k0 + j : k1 + j - 4;
+      x[j] = k >= b && k < e ? gather(c[j]) : 0.f;
+    }
 #pragma unroll
-      for (int j = 0; j < PRB_UNROLL; j++) x[j] = k + 32 * j < e ? gather(c[j]) : 0.f;
-#pragma unroll
-      for (int j = 0; j < PRB_UNROLL; j++)
-        if (k + 32 * j < e) prb_add<WEIGHTED>(acc, x[j], p.wts, k + 32 * j);
+    for (int j = 0; j < 8; j++) {
+      if (WEIGHTED) {
+        const int32_t k = j < 4 ? k0 + j : k1 + j - 4;
+        const float a = k >= b && k < e ? w[j] : 0.f;
+        const float pr = a * x[j];
+        two_sum_add(acc, pr);
+        acc.lo += __fmaf_rn(a, x[j], -pr);
+      } else {
+        two_sum_add(acc, x[j]);
+      }
     }
   }
-  group_comp_reduce<32>(acc);
+  if (L > 1) group_comp_reduce<L>(acc);
   return acc;
 }
 
-// 32 consecutive rows of bin `bin` (warp assignment `wa`), G lanes per row:
-// every lane first loads its slot's row and offsets; then G passes of 32/G rows
-// each. For light bins (G < 32, at most G edges per row) all G passes issue their
-// index loads and then their gathers back to back before any reduction, so a warp
-// waits for three memory round trips per assignment rather than three per pass.
-// The sum of slot l ends up in lane l, whose row is returned in *my_row (-1 past
-// the bin), so the row updates then run on all lanes at once.
-// prb_ranges32 is the same for 32 edge ranges [mb, me) given per lane (at most G
-// edges each for G < 32): the sum of lane l's range ends up in lane l.
-template <int G, bool WEIGHTED, bool ADAPT, typename Gather>
-__device__ __forceinline__ Comp prb_ranges32(const PrbArgs &p, int32_t mb, int32_t me, Gather &gather) {
-  constexpr int RPP = 32 / G;  // rows per pass
-  const int lane = threadIdx.x & 31;
-  const int gl = lane % G, grp = lane / G;
-  Comp mine{0.f, 0.f};
-  if (G == 32) {
-#pragma unroll 1
-    for (int q = 0; q < 32; q++) {
-      const int32_t b = __shfl_sync(0xffffffffu, mb, q), e = __shfl_sync(0xffffffffu, me, q);
-      const Comp acc = prb_warp_range<WEIGHTED, ADAPT>(p, b, e, gather);
-      if (lane == q) mine = acc;
-    }
-  } else {
-    // Passes run in batches of up to 8 so the in-flight loads fit the register budget.
-    constexpr int BATCH = G < PRB_BATCH ? G : PRB_BATCH;
+// Rows of up to 2 edges, one lane each, plain index loads.
+template <bool WEIGHTED, typename Gather>
+__device__ __forceinline__ Comp prb_short_range(const PrbArgs &p, int32_t b, int32_t e, Gather &gather) {
+  Comp acc{0.f, 0.f};
+  int32_t c[2];
+  float x[2], w[2];
 #pragma unroll
-    for (int q0 = 0; q0 < G; q0 += BATCH) {
-      int32_t k_of[BATCH];
-      int32_t c_of[BATCH];
-      float v_of[BATCH];
+  for (int j = 0; j < 2; j++) {
+    c[j] = b + j < e ? prb_stream(p.idx + b + j) : 0;
+    w[j] = WEIGHTED && b + j < e ? prb_stream(p.wts + b + j) : 0.f;
+  }
 #pragma unroll
-      for (int j = 0; j < BATCH; j++) {
-        const int src = (q0 + j) * RPP + grp;
-        const int32_t b = __shfl_sync(0xffffffffu, mb, src), e = __shfl_sync(0xffffffffu, me, src);
-        k_of[j] = b + gl < e ? b + gl : -1;
-      }
+  for (int j = 0; j < 2; j++) x[j] = b + j < e ? gather(c[j]) : 0.f;
 #pragma unroll
-      for (int j = 0; j < BATCH; j++) c_of[j] = k_of[j] >= 0 ? prb_stream(p.idx + k_of[j]) : 0;
-#pragma unroll
-      for (int j = 0; j < BATCH; j++) v_of[j] = k_of[j] >= 0 ? gather(c_of[j]) : 0.f;
-#pragma unroll
-      for (int j = 0; j < BATCH; j++) {
-        Comp acc{0.f, 0.f};
-        if (k_of[j] >= 0) prb_add<WEIGHTED>(acc, v_of[j], p.wts, k_of[j]);
-        group_comp_reduce<G>(acc);
-        const int src = (lane % RPP) * G;
-        const float h = __shfl_sync(0xffffffffu, acc.hi, src), l = __shfl_sync(0xffffffffu, acc.lo, src);
-        if (lane / RPP == q0 + j) mine = Comp{h, l};
-      }
+  for (int j = 0; j < 2; j++) {
+    if (WEIGHTED) {
+      const float pr = w[j] * x[j];
+      two_sum_add(acc, pr);
+      acc.lo += __fmaf_rn(w[j], x[j], -pr);
+    } else {
+      two_sum_add(acc, x[j]);
     }
   }
-  return mine;
+  return acc;
 }
 
-template <int G, bool WEIGHTED, bool ADAPT, typename Gather>
-__device__ __forceinline__ Comp prb_rows32(const PrbArgs &p, int bin, int64_t wa, Gather &gather, int32_t *my_row) {
-  const int lane = threadIdx.x & 31;
-  const int64_t slot = p.boff[bin] + wa * 32 + lane;
-  const int32_t mine_row = slot < p.boff[bin + 1] ? p.rows[slot] : -1;
-  const int32_t mb = mine_row >= 0 ? __ldg(p.off + mine_row) : 0;
-  const int32_t me = mine_row >= 0 ? __ldg(p.off + mine_row + 1) : 0;
-  *my_row = mine_row;
-  return prb_ranges32<G, WEIGHTED, ADAPT>(p, mb, me, gather);
-}
-
-// Walks every assignment of the plan with a persistent grid (fixed stride).
-// finish(row, Comp) consumes a row sum; finish_hub(h, row, Comp) consumes a hub's.
-template <bool WEIGHTED, bool ADAPT = true, typename Gather, typename Finish, typename FinishHub>
-__device__ __forceinline__ void prb_run(const PrbArgs &p, Gather &&gather, Finish &&finish, FinishHub &&finish_hub) {
+// Hands the plan's warp assignments to item(bin, wa), hub chunks first and the
+// lightest rows last (long items first shortens the tail), over a persistent grid.
+template <typename Item>
+__device__ __forceinline__ void prb_items(const PrbArgs &p, Item &&item) {
   const int64_t total = p.wstart[PRB_BINS];
-  const int lane = threadIdx.x & 31;
-  auto item = [&](int64_t wi) {
-    const int64_t w = PRB_HEAVY_FIRST ? total - 1 - wi : wi;
+  auto at = [&](int64_t wi) {
+    const int64_t w = total - 1 - wi;
     int bin = 0;
 #pragma unroll
     for (int q = 1; q < PRB_BINS; q++)
       if (w >= p.wstart[q]) bin = q;
-    const int64_t wa = w - p.wstart[bin];
-    if (bin < 6) {
-      int32_t row = -1;
-      Comp acc;
-      switch (bin) {
-        case 0: acc = prb_rows32<1, WEIGHTED, ADAPT>(p, 0, wa, gather, &row); break;
-        case 1: acc = prb_rows32<2, WEIGHTED, ADAPT>(p, 1, wa, gather, &row); break;
-        case 2: acc = prb_rows32<4, WEIGHTED, ADAPT>(p, 2, wa, gather, &row); break;
-        case 3: acc = prb_rows32<8, WEIGHTED, ADAPT>(p, 3, wa, gather, &row); break;
-        case 4: acc = prb_rows32<16, WEIGHTED, ADAPT>(p, 4, wa, gather, &row); break;
-        default: acc = prb_rows32<32, WEIGHTED, ADAPT>(p, 5, wa, gather, &row); break;
-      }
-      if (row >= 0) finish(row, acc);
-      return;
-    }
-    switch (bin) {
-      default: {
-        // Hub chunk task `wa`: find its hub by binary search over the chunk bases.
-        int64_t lo = 0, hi = p.nheavy;
-        while (hi - lo > 1) {
-          const int64_t mid = (lo + hi) >> 1;
-          if (p.hbase[mid] <= wa) lo = mid;
-          else hi = mid;
-        }
-        const int32_t row = p.hrows[lo];
-        const int32_t chunk = (int32_t)(wa - p.hbase[lo]);
-        const int32_t rb = __ldg(p.off + row);
-        const int32_t b = rb + chunk * PRB_CHUNK;
-        const int32_t e = min(b + PRB_CHUNK, __ldg(p.off + row + 1));
-        const Comp acc = prb_warp_range<WEIGHTED, ADAPT>(p, b, e, gather);
-        bool last = false;
-        if (lane == 0) {
-          p.hpart[wa] = acc;
-          __threadfence();
-          const int32_t nch = p.hbase[lo + 1] - p.hbase[lo];
-          last = atomicAdd(p.hcount + lo, 1) == nch - 1;
-          if (last) {
-            __threadfence();
-            Comp tot{0.f, 0.f};
-            const float2 *parts = reinterpret_cast<const float2 *>(p.hpart) + p.hbase[lo];
-            for (int32_t c = 0; c < nch; c++) {
-              const float2 v = __ldcg(parts + c);  // written by other SMs: read from L2
-              comp_add(tot, Comp{v.x, v.y});
-            }
-            p.hcount[lo] = 0;
-            finish_hub(lo, row, tot);
-          }
-        }
-        break;
-      }
-    }
+    item(bin, w - p.wstart[bin]);
   };
   if (p.grab) {
     for (;;) {
-      int64_t base = 0;
-      if (lane == 0) base = atomicAdd(p.grab, PRB_GRAB);
-      base = __shfl_sync(FULL, base, 0);
-      if (base >= total) break;
-      const int64_t end = min(base + (int64_t)PRB_GRAB, total);
-      for (int64_t wi = base; wi < end; wi++) item(wi);
+      int64_t wi = 0;
+      if (lane_id() == 0) wi = atomicAdd(p.grab, 1);
+      wi = __shfl_sync(FULL, wi, 0);
+      if (wi >= total) break;
+      at(wi);
     }
   } else {
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t wi = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wi < total; wi += nwarps) item(wi);
+    for (int64_t wi = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wi < total; wi += nwarps) at(wi);
   }
+}
+
+// Walks the plan's rows: body(L, row, b, e, sub, task) with L the lanes (an
+// integral constant) that share edges [b, e) of `row`, sub the lane's place among
+// them and task the chunk's number if they are a chunk of a hub (else -1). Every
+// lane of the warp calls it: a group past the bin's end has row -1 and no edges.
+template <typename Body>
+__device__ __forceinline__ void prb_walk(const PrbArgs &p, Body &&body) {
+  const int lane = threadIdx.x & 31;
+  prb_items(p, [&](int bin, int64_t wa) {
+    if (bin == PRB_HUB) {
+      // its hub by binary search over the chunk bases
+      int64_t lo = 0, hi = p.nheavy;
+      while (hi - lo > 1) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (p.hbase[mid] <= wa) lo = mid;
+        else hi = mid;
+      }
+      const int32_t row = p.hrows[lo];
+      const int32_t b = __ldg(p.off + row) + (int32_t)(wa - p.hbase[lo]) * PRB_CHUNK;
+      body(std::integral_constant<int, 32>(), row, b, min(b + PRB_CHUNK, __ldg(p.off + row + 1)), lane, wa, lo);
+      return;
+    }
+    const int lg = bin < PRB_QUAD ? 0 : bin == PRB_QUAD ? 2 : 5;  // log2 of the lanes per row
+    const int sub = lane & ((1 << lg) - 1);
+    const int nrow = bin == PRB_WARP ? prb_rows_per(PRB_WARP) : 1;
+    for (int q = 0; q < nrow; q++) {
+      const int64_t slot = p.boff[bin] + (bin == PRB_WARP ? wa * nrow + q : wa * (32 >> lg) + (lane >> lg));
+      const int32_t row = slot < p.boff[bin + 1] ? p.rows[slot] : -1;
+      const int32_t b = row >= 0 ? __ldg(p.off + row) : 0;
+      const int32_t e = row >= 0 ? __ldg(p.off + row + 1) : 0;
+      const int64_t whole = -1;
+      if (bin == PRB_WARP) body(std::integral_constant<int, 32>(), row, b, e, sub, whole, whole);
+      else if (bin == PRB_QUAD) body(std::integral_constant<int, 4>(), row, b, e, sub, whole, whole);
+      else if (bin > 1) body(std::integral_constant<int, 1>(), row, b, e, sub, whole, whole);
+      else body(std::integral_constant<int, 0>(), row, b, e, sub, whole, whole);  // at most 2 edges
+    }
+  });
+}
+
+// A lane's share (prb_walk's L and sub) of the compensated sum of edges [b, e).
+template <int L, bool WEIGHTED, typename Gather>
+__device__ __forceinline__ Comp prb_range(const PrbArgs &p, int32_t b, int32_t e, int sub, Gather &gather) {
+  if constexpr (L == 0) return prb_short_range<WEIGHTED>(p, b, e, gather);
+  else return prb_group_range<L, WEIGHTED>(p, b, e, sub, gather);
+}
+
+// A hub chunk's partial: stored, and the lane that stores the last one of hub h
+// gets the sum of all of them in chunk order (true). Lane 0 calls it.
+__device__ __forceinline__ bool prb_hub_done(const PrbArgs &p, int64_t task, int64_t h, const Comp &part, Comp &tot) {
+  p.hpart[task] = part;
+  __threadfence();
+  const int32_t nch = p.hbase[h + 1] - p.hbase[h];
+  if (atomicAdd(p.hcount + h, 1) != nch - 1) return false;
+  __threadfence();
+  tot = Comp{0.f, 0.f};
+  const float2 *parts = reinterpret_cast<const float2 *>(p.hpart) + p.hbase[h];
+  for (int32_t c = 0; c < nch; c++) {
+    const float2 v = __ldcg(parts + c);  // written by other SMs: read from L2
+    comp_add(tot, Comp{v.x, v.y});
+  }
+  p.hcount[h] = 0;
+  return true;
+}
+
+// Sums every row of the plan: finish(row, Comp) consumes a row sum,
+// finish_hub(h, row, Comp) a hub's.
+template <bool WEIGHTED, typename Gather, typename Finish, typename FinishHub>
+__device__ __forceinline__ void prb_run(const PrbArgs &p, Gather &&gather, Finish &&finish, FinishHub &&finish_hub) {
+  prb_walk(p, [&](auto lanes, int32_t row, int32_t b, int32_t e, int sub, int64_t task, int64_t h) {
+    const Comp acc = prb_range<decltype(lanes)::value, WEIGHTED>(p, b, e, sub, gather);
+    if (task >= 0) {
+      Comp tot;
+      if (sub == 0 && prb_hub_done(p, task, h, acc, tot)) finish_hub(h, row, tot);
+    } else if (row >= 0 && sub == 0) {
+      finish(row, acc);
+    }
+  });
 }
 
 }  // namespace mg
