@@ -6,10 +6,9 @@
 //   CSC  col_offsets[n+1], row_idx[m], perm[m] (CSC slot -> CSR edge id),
 //        cvals[m] (values already permuted, so in-edge kernels read them
 //        sequentially instead of through perm)
-// The CSC is built on the device by counting sort: per-column counts, an
-// exclusive scan, an atomic scatter, then a segmented sort of every column by
-// CSR edge id, which makes it identical to the reference's stable sort by column
-// (within a column, edges in CSR order) and therefore deterministic.
+// The CSC is built on the device by a stable radix sort of the edges by column,
+// which makes it identical to the reference's stable sort by column (within a
+// column, edges in CSR order) and therefore deterministic.
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -361,212 +360,201 @@ __global__ void fill_pad_kernel(int32_t *off, int64_t n, int32_t *edges, void *v
 }
 
 // ---------------------------------------------------------------------------
-// CSC build kernels.
-__global__ void count_cols_kernel(const int32_t *__restrict__ ci, int64_t m, int32_t *__restrict__ cnt) {
-  const int64_t m4 = m / 4;
-  const int4 *ci4 = reinterpret_cast<const int4 *>(ci);
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = tid; i < m4; i += stride) {
-    int4 c = __ldg(ci4 + i);
-    atomicAdd(&cnt[c.x], 1);
-    atomicAdd(&cnt[c.y], 1);
-    atomicAdd(&cnt[c.z], 1);
-    atomicAdd(&cnt[c.w], 1);
+// CSC build: least-significant-digit radix sort of (column, edge id), RS_BITS bits
+// a pass. A tile of RS_TILE edges is counted per digit, the counts are scanned
+// digit-major over the tiles, and the tile is ranked and written out.
+//
+// Memory traffic bounds it: 20 bytes per edge and pass. A counting sort by atomics
+// (count, scatter, sort every column) queues on the hot columns of a skewed graph:
+// R-MAT s20, 16.8 M edges, 0.34 ms for the counts, 3.2 ms for the scatter and 3.1
+// ms for sorting the columns.
+constexpr int RS_BITS = 8;
+constexpr int RS_NT = 256;
+constexpr int RS_WARPS = RS_NT / 32;
+constexpr int RS_VT = 16;
+constexpr int RS_TILE = RS_NT * RS_VT;
+
+// Lanes of the warp whose digit equals this lane's (all lanes call it).
+__device__ __forceinline__ unsigned rs_peers(unsigned d, int bits) {
+  unsigned m = FULL;
+  for (int b = 0; b < bits; b++) {
+    const unsigned v = __ballot_sync(FULL, (d >> b) & 1);
+    m &= (d >> b) & 1 ? v : ~v;
   }
-  for (int64_t i = m4 * 4 + tid; i < m; i += stride) atomicAdd(&cnt[ci[i]], 1);
+  return m;
 }
 
-// One warp per row: the warp walks the row's edges with coalesced loads and
-// drops (row, edge id) into the column buckets.
-__global__ void scatter_csc_kernel(const int32_t *__restrict__ ro, const int32_t *__restrict__ ci, int64_t n,
-                                   const int32_t *__restrict__ co, int32_t *__restrict__ cursor,
-                                   int32_t *__restrict__ ri, int32_t *__restrict__ perm) {
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int l = lane_id();
-  for (int64_t v = warp; v < n; v += nwarps) {
-    const int32_t b = ro[v], e = ro[v + 1];
-    for (int32_t k = b + l; k < e; k += 32) {
-      int32_t c = ci[k];
-      int32_t pos = co[c] + atomicAdd(&cursor[c], 1);
-      ri[pos] = (int32_t)v;
-      perm[pos] = k;
+// Digit counts of a tile: cnt[digit * ntiles + tile].
+__global__ void __launch_bounds__(RS_NT) rs_count_kernel(const int32_t *__restrict__ key, int64_t m, int shift,
+                                                         int bits, int32_t ntiles, int32_t *__restrict__ cnt) {
+  __shared__ int32_t s_cnt[1 << RS_BITS];
+  const unsigned mask = (1u << bits) - 1;
+  for (int i = threadIdx.x; i <= (int)mask; i += RS_NT) s_cnt[i] = 0;
+  __syncthreads();
+  const int64_t t0 = (int64_t)blockIdx.x * RS_TILE;
+  int32_t k[RS_VT];
+#pragma unroll
+  for (int r = 0; r < RS_VT; r++) {
+    const int64_t i = t0 + r * RS_NT + threadIdx.x;
+    k[r] = i < m ? __ldcs(key + i) : -1;
+  }
+#pragma unroll
+  for (int r = 0; r < RS_VT; r++) {
+    // lanes with the same digit add once: a skewed graph's hot column is in most warps
+    const unsigned d = k[r] < 0 ? (1u << bits) : ((unsigned)k[r] >> shift) & mask;
+    const unsigned peers = rs_peers(d, bits + 1);
+    if (k[r] >= 0 && (peers & lanemask_lt()) == 0) atomicAdd(s_cnt + d, __popc(peers));
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i <= (int)mask; i += RS_NT) cnt[(int64_t)i * ntiles + blockIdx.x] = s_cnt[i];
+}
+
+// Stable scatter of a tile: warp w ranks its RS_VT x 32 consecutive edges in order
+// (32 at a time, per-warp digit counters), the tile is put in digit order in shared
+// memory and leaves it in runs. val_in == nullptr: the payload is the edge id.
+__global__ void __launch_bounds__(RS_NT, 3) rs_scatter_kernel(const int32_t *__restrict__ key_in,
+                                                           const int32_t *__restrict__ val_in, int64_t m, int shift,
+                                                           int bits, int32_t ntiles,
+                                                           const int32_t *__restrict__ ofs,
+                                                           int32_t *__restrict__ key_out,
+                                                           int32_t *__restrict__ val_out) {
+  __shared__ int32_t s_key[RS_TILE], s_val[RS_TILE];
+  __shared__ uint16_t s_cnt[RS_WARPS][1 << RS_BITS];  // per warp: digit counts, then exclusive tile positions
+  __shared__ int32_t s_base[1 << RS_BITS];            // global position of a digit minus its tile position
+  __shared__ int32_t s_red[RS_WARPS + 1];
+  const unsigned mask = (1u << bits) - 1;
+  const int lane = lane_id(), w = warp_id();
+  for (int i = threadIdx.x; i < RS_WARPS << RS_BITS; i += RS_NT) (&s_cnt[0][0])[i] = 0;
+  __syncthreads();
+  const int64_t t0 = (int64_t)blockIdx.x * RS_TILE;
+  const int64_t w0 = t0 + w * (RS_VT * 32) + lane;
+  int32_t k[RS_VT], v[RS_VT];
+  uint16_t rank[RS_VT];
+#pragma unroll
+  for (int r = 0; r < RS_VT; r++) {
+    const int64_t i = w0 + r * 32;
+    k[r] = i < m ? __ldcs(key_in + i) : -1;
+    v[r] = i < m ? (val_in ? __ldcs(val_in + i) : (int32_t)i) : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < RS_VT; r++) {
+    const unsigned d = k[r] < 0 ? (1u << bits) : ((unsigned)k[r] >> shift) & mask;
+    const unsigned peers = rs_peers(d, bits + 1);
+    const int before = __popc(peers & lanemask_lt());
+    int32_t c = 0;
+    if (k[r] >= 0) c = s_cnt[w][d];
+    __syncwarp();
+    if (k[r] >= 0 && before == 0) s_cnt[w][d] = (uint16_t)(c + __popc(peers));
+    __syncwarp();
+    rank[r] = (uint16_t)(c + before);
+  }
+  __syncthreads();
+  // digit d (one per thread): the warps' counts become tile positions
+  int32_t tot = 0;
+  const int d0 = threadIdx.x;
+  if (d0 <= (int)mask)
+    for (int q = 0; q < RS_WARPS; q++) tot += s_cnt[q][d0];
+  int32_t all;
+  int32_t pos = block_exclusive_scan<RS_NT>(tot, s_red, &all);
+  if (d0 <= (int)mask) {
+    s_base[d0] = ofs[(int64_t)d0 * ntiles + blockIdx.x] - pos;
+    for (int q = 0; q < RS_WARPS; q++) {
+      const int32_t c = s_cnt[q][d0];
+      s_cnt[q][d0] = (uint16_t)pos;
+      pos += c;
     }
   }
-}
-
-// Sorting classes of column segments.
-constexpr int SEG_SMALL = 32;    // insertion sort by one thread
-constexpr int SEG_MEDIUM = 2048; // bitonic sort of the whole segment in shared memory
-constexpr int SORT_NT = 256;
-
-__global__ void classify_segments_kernel(const int32_t *__restrict__ co, int64_t n, int32_t *__restrict__ lists,
-                                         int32_t *__restrict__ lens, int32_t cap) {
-  int32_t dummy_overflow = 0;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-    int32_t len = co[c + 1] - co[c];
-    int cls = len <= 1 ? -1 : (len <= SEG_SMALL ? 0 : (len <= SEG_MEDIUM ? 1 : 2));
-    for (int k = 0; k < 3; k++) warp_append(cls == k, (int32_t)c, lists + (size_t)k * cap, &lens[k], cap, &dummy_overflow);
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < RS_VT; r++) {
+    if (k[r] < 0) continue;
+    const int32_t at = s_cnt[w][((unsigned)k[r] >> shift) & mask] + rank[r];
+    s_key[at] = k[r];
+    s_val[at] = v[r];
+  }
+  __syncthreads();
+  const int32_t n_here = (int32_t)min((int64_t)RS_TILE, m - t0);
+  for (int32_t i = threadIdx.x; i < n_here; i += RS_NT) {
+    const int32_t key = s_key[i];
+    const int32_t at = s_base[((unsigned)key >> shift) & mask] + i;
+    key_out[at] = key;
+    val_out[at] = s_val[i];
   }
 }
 
-__global__ void sort_small_kernel(const int32_t *__restrict__ co, const int32_t *__restrict__ list,
-                                  const int32_t *__restrict__ len, int32_t *__restrict__ key,
-                                  int32_t *__restrict__ val) {
-  const int32_t cnt = *len;
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    const int32_t c = list[i];
-    const int32_t b = co[c], e = co[c + 1];
-    for (int32_t x = b + 1; x < e; x++) {
-      int32_t k = key[x], v = val[x];
-      int32_t y = x - 1;
-      while (y >= b && key[y] > k) {
-        key[y + 1] = key[y];
-        val[y + 1] = val[y];
-        y--;
-      }
-      key[y + 1] = k;
-      val[y + 1] = v;
-    }
-  }
-}
-
-// Bitonic sort of `cnt` (<= SEG_MEDIUM) key/value pairs held in shared memory,
-// padded to the next power of two with INT_MAX keys.
-__device__ void smem_bitonic(int32_t *sk, int32_t *sv, int p2) {
-  for (int size = 2; size <= p2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < p2 / 2; t += blockDim.x) {
-        int lo = 2 * t - (t & (stride - 1));
-        int hi = lo + stride;
-        bool up = ((lo & size) == 0);
-        int32_t a = sk[lo], b = sk[hi];
-        if ((a > b) == up) {
-          sk[lo] = b;
-          sk[hi] = a;
-          int32_t tv = sv[lo];
-          sv[lo] = sv[hi];
-          sv[hi] = tv;
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-__global__ void __launch_bounds__(SORT_NT) sort_medium_kernel(const int32_t *__restrict__ co,
-                                                               const int32_t *__restrict__ list,
-                                                               const int32_t *__restrict__ len,
-                                                               int32_t *__restrict__ key, int32_t *__restrict__ val) {
-  __shared__ int32_t sk[SEG_MEDIUM], sv[SEG_MEDIUM];
-  const int32_t cnt = *len;
-  for (int32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
-    const int32_t c = list[i];
-    const int32_t b = co[c], L = co[c + 1] - b;
-    int p2 = 1;
-    while (p2 < L) p2 <<= 1;
-    for (int t = threadIdx.x; t < p2; t += SORT_NT) {
-      sk[t] = t < L ? key[b + t] : INT_MAX;
-      sv[t] = t < L ? val[b + t] : 0;
-    }
-    __syncthreads();
-    smem_bitonic(sk, sv, p2);
-    for (int t = threadIdx.x; t < L; t += SORT_NT) {
-      key[b + t] = sk[t];
-      val[b + t] = sv[t];
-    }
-    __syncthreads();
-  }
-}
-
-// Large segments: one CTA per segment sorts SEG_MEDIUM-sized runs in shared
-// memory, then merges runs pairwise through a scratch buffer (tk/tv, same
-// offsets as key/val). Each thread merges a fixed slice of the output found by
-// a merge-path search.
-__device__ int merge_path(const int32_t *a, int la, const int32_t *b, int lb, int diag) {
-  int lo = max(0, diag - lb), hi = min(diag, la);
+// First position in [lo, hi) of the ascending a whose value is >= x (hi if none).
+__device__ __forceinline__ int64_t lower_bound_i32(const int32_t *__restrict__ a, int64_t lo, int64_t hi, int32_t x) {
   while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (a[mid] <= b[diag - 1 - mid]) lo = mid + 1;
+    const int64_t mid = (lo + hi) >> 1;
+    if (__ldg(a + mid) < x) lo = mid + 1;
     else hi = mid;
   }
   return lo;
 }
 
-__global__ void __launch_bounds__(SORT_NT) sort_large_kernel(const int32_t *__restrict__ co,
-                                                              const int32_t *__restrict__ list,
-                                                              const int32_t *__restrict__ len, int32_t *key,
-                                                              int32_t *val, int32_t *tk, int32_t *tv) {
-  __shared__ int32_t sk[SEG_MEDIUM], sv[SEG_MEDIUM];
-  const int32_t cnt = *len;
-  for (int32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
-    const int32_t c = list[i];
-    const int32_t b = co[c], L = co[c + 1] - b;
-    for (int32_t r0 = 0; r0 < L; r0 += SEG_MEDIUM) {
-      int rl = min(SEG_MEDIUM, L - r0);
-      for (int t = threadIdx.x; t < SEG_MEDIUM; t += SORT_NT) {
-        sk[t] = t < rl ? key[b + r0 + t] : INT_MAX;
-        sv[t] = t < rl ? val[b + r0 + t] : 0;
-      }
-      __syncthreads();
-      smem_bitonic(sk, sv, SEG_MEDIUM);
-      for (int t = threadIdx.x; t < rl; t += SORT_NT) {
-        key[b + r0 + t] = sk[t];
-        val[b + r0 + t] = sv[t];
-      }
-      __syncthreads();
-    }
-    int32_t *srck = key + b, *srcv = val + b, *dstk = tk + b, *dstv = tv + b;
-    for (int32_t w = SEG_MEDIUM; w < L; w <<= 1) {
-      for (int32_t p0 = 0; p0 < L; p0 += 2 * w) {
-        const int32_t la = min(w, L - p0), lb = max(0, min(w, L - p0 - w));
-        const int32_t *ak = srck + p0, *bk = srck + p0 + la;
-        const int32_t *av = srcv + p0, *bv = srcv + p0 + la;
-        const int32_t tot = la + lb;
-        const int32_t per = (tot + SORT_NT - 1) / SORT_NT;
-        int32_t d0 = min(tot, (int32_t)threadIdx.x * per), d1 = min(tot, d0 + per);
-        int ia = merge_path(ak, la, bk, lb, d0);
-        int ib = d0 - ia;
-        for (int32_t d = d0; d < d1; d++) {
-          bool takea = ib >= lb || (ia < la && ak[ia] <= bk[ib]);
-          if (takea) {
-            dstk[p0 + d] = ak[ia];
-            dstv[p0 + d] = av[ia];
-            ia++;
-          } else {
-            dstk[p0 + d] = bk[ib];
-            dstv[p0 + d] = bv[ib];
-            ib++;
-          }
-        }
-      }
-      __syncthreads();
-      int32_t *t1 = srck, *t2 = srcv;
-      srck = dstk;
-      srcv = dstv;
-      dstk = t1;
-      dstv = t2;
-    }
-    if (srck != key + b) {
-      for (int32_t t = threadIdx.x; t < L; t += SORT_NT) {
-        key[b + t] = srck[t];
-        val[b + t] = srcv[t];
-      }
-    }
-    __syncthreads();
+// Column offsets from the sorted columns: a CTA brackets its 256 columns first.
+__global__ void __launch_bounds__(256) csc_offsets_kernel(const int32_t *__restrict__ key, int64_t m, int64_t n,
+                                                          int32_t *__restrict__ co) {
+  __shared__ int64_t s_lo, s_hi;
+  const int64_t c0 = (int64_t)blockIdx.x * 256, c = c0 + threadIdx.x;
+  if (threadIdx.x == 0) s_lo = lower_bound_i32(key, 0, m, (int32_t)c0);
+  if (threadIdx.x == 32) s_hi = c0 + 256 <= n ? lower_bound_i32(key, 0, m, (int32_t)(c0 + 255)) : m;
+  __syncthreads();
+  if (c <= n) co[c] = c == n ? (int32_t)m : (int32_t)lower_bound_i32(key, s_lo, s_hi, (int32_t)c);
+}
+
+// Row of every CSR edge beside its value, {row, value bits} (val == nullptr: the
+// row alone): a CTA brackets the rows of its 1024 edges, a thread then searches
+// between them. The pair is one random read per edge for csc_gather_kernel.
+constexpr int EP_VT = 4;
+template <bool PAIR>
+__global__ void __launch_bounds__(256) edge_rows_kernel(const int32_t *__restrict__ ro, int64_t n, int64_t m,
+                                                        const int32_t *__restrict__ val, int32_t *__restrict__ out) {
+  __shared__ int64_t s_row[2];
+  const int64_t k0 = (int64_t)blockIdx.x * 256 * EP_VT;
+  if ((threadIdx.x & 31) == 0 && threadIdx.x < 64) {
+    // last row that starts at or before the tile's first / last edge
+    const int64_t k = threadIdx.x == 0 ? k0 : min(k0 + 256 * EP_VT, m) - 1;
+    s_row[threadIdx.x >> 5] = lower_bound_i32(ro, 0, n + 1, (int32_t)k + 1) - 1;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < EP_VT; j++) {
+    const int64_t k = k0 + j * 256 + threadIdx.x;
+    if (k >= m) continue;
+    const int32_t row = (int32_t)(lower_bound_i32(ro, s_row[0], s_row[1] + 1, (int32_t)k + 1) - 1);
+    if (PAIR) reinterpret_cast<int2 *>(out)[k] = make_int2(row, val[k]);
+    else out[k] = row;
   }
 }
 
-template <typename T>
-__global__ void permute_values_kernel(const int32_t *__restrict__ perm, const T *__restrict__ src, int64_t m,
-                                      T *__restrict__ dst) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = src[perm[i]];
+// Row index and value of every CSC slot, through its edge id.
+template <bool PAIR>
+__global__ void __launch_bounds__(256) csc_gather_kernel(const int32_t *__restrict__ perm,
+                                                         const int32_t *__restrict__ rows, int64_t m,
+                                                         int32_t *__restrict__ ri, int32_t *__restrict__ cval) {
+  const int64_t stride = (int64_t)gridDim.x * 256;
+  for (int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x; i0 < m; i0 += 4 * stride) {
+    int32_t k[4];
+    int2 p[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) k[j] = i0 + j * stride < m ? __ldcs(perm + i0 + j * stride) : 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (PAIR) p[j] = __ldg(reinterpret_cast<const int2 *>(rows) + k[j]);
+      else p[j].x = __ldg(rows + k[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int64_t i = i0 + j * stride;
+      if (i >= m) continue;
+      ri[i] = p[j].x;
+      if (PAIR) cval[i] = p[j].y;
+    }
+  }
 }
 
 }  // namespace mg
-
-static int grid_for(const mg_graph *g, int per_sm = 8) { return g->num_sms * per_sm; }
 
 // Builds the CSC of g (co, ri, perm, cvals). Scratch is taken from ws_aux.
 static mg_status build_csc(mg_graph *g) {
@@ -581,36 +569,50 @@ static mg_status build_csc(mg_graph *g) {
   if (vbytes) MG_CUDA_TRY(mg_malloc_async(&g->cvals, vbytes * (m + MG_EDGE_PAD), s));
   mg::fill_pad_kernel<<<1, 32, 0, s>>>(g->co, n, g->ri, g->cvals, m);
   g->has_csc = true;
-  const int64_t ntiles = std::max<int64_t>(1, (n + SCAN_TILE - 1) / SCAN_TILE);
-  const size_t need = Carve::need({sizeof(int32_t) * (size_t)(n + 1), sizeof(int32_t) * (size_t)(n + 1),
-                                   sizeof(int64_t) * (size_t)ntiles, sizeof(int32_t) * 3 * (size_t)(n + 1),
-                                   sizeof(int32_t) * 4, sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1),
-                                   sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1)});
-  MG_TRY(ws_reserve(g, g->ws_aux, need));
+  if (m == 0) {
+    MG_CUDA_TRY(cudaMemsetAsync(g->co, 0, sizeof(int32_t) * (n + 1), s));
+    return MG_OK;
+  }
+  int bits = 1;
+  while (bits < 31 && ((int64_t)1 << bits) < n) bits++;
+  const int passes = (bits + RS_BITS - 1) / RS_BITS;
+  const int32_t tiles = (int32_t)((m + RS_TILE - 1) / RS_TILE);
+  const int64_t ncnt = (int64_t)tiles << RS_BITS;
+  const size_t em = sizeof(int32_t) * (size_t)m;
+  // keys ping-pong side by side (afterwards the {row, value} pairs), the payload's
+  // other buffer (one of the two is perm itself), tile counts and their offsets
+  MG_TRY(ws_reserve(g, g->ws_aux, Carve::need({2 * em + 256, em, sizeof(int32_t) * (size_t)ncnt,
+                                               sizeof(int32_t) * (size_t)(ncnt + 1),
+                                               sizeof(int64_t) * (size_t)(ncnt / SCAN_TILE + 2)})));
   Carve cv(g->ws_aux.ptr);
-  int32_t *cnt = cv.take<int32_t>(n + 1);
-  int32_t *cursor = cv.take<int32_t>(n + 1);
-  int64_t *tmp = cv.take<int64_t>(ntiles);
-  int32_t *lists = cv.take<int32_t>(3 * (size_t)(n + 1));
-  int32_t *lens = cv.take<int32_t>(4);
-  int32_t *tk = cv.take<int32_t>(std::max<int64_t>(m, 1));
-  int32_t *tv = cv.take<int32_t>(std::max<int64_t>(m, 1));
-  MG_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (n + 1), s));
-  MG_CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (n + 1), s));
-  MG_CUDA_TRY(cudaMemsetAsync(lens, 0, sizeof(int32_t) * 4, s));
-  const int grid = grid_for(g);
-  if (m > 0) count_cols_kernel<<<grid, 256, 0, s>>>(g->ci, m, cnt);
-  MG_TRY(device_exclusive_scan(cnt, g->co, n, tmp, s));
-  if (m > 0) {
-    scatter_csc_kernel<<<grid, 256, 0, s>>>(g->ro, g->ci, n, g->co, cursor, g->ri, g->perm);
-    classify_segments_kernel<<<grid, 256, 0, s>>>(g->co, n, lists, lens, (int32_t)(n + 1));
-    sort_small_kernel<<<grid, 256, 0, s>>>(g->co, lists, lens + 0, g->perm, g->ri);
-    sort_medium_kernel<<<grid, SORT_NT, 0, s>>>(g->co, lists + (n + 1), lens + 1, g->perm, g->ri);
-    sort_large_kernel<<<grid, SORT_NT, 0, s>>>(g->co, lists + 2 * (n + 1), lens + 2, g->perm, g->ri, tk, tv);
-    if (g->vtype == MG_DTYPE_I32)
-      permute_values_kernel<int32_t><<<grid, 256, 0, s>>>(g->perm, (const int32_t *)g->vals, m, (int32_t *)g->cvals);
-    else if (g->vtype == MG_DTYPE_F32)
-      permute_values_kernel<float><<<grid, 256, 0, s>>>(g->perm, (const float *)g->vals, m, (float *)g->cvals);
+  int32_t *keys = cv.take<int32_t>(2 * (size_t)m + 64);
+  int32_t *vtmp = cv.take<int32_t>(m);
+  int32_t *cnt = cv.take<int32_t>(ncnt);
+  int32_t *ofs = cv.take<int32_t>(ncnt + 1);
+  int64_t *tmp = cv.take<int64_t>(ncnt / SCAN_TILE + 2);
+  int32_t *kbuf[2] = {keys, keys + m};
+  const int32_t *kin = g->ci, *vin = nullptr;
+  int shift = 0;
+  for (int p = 0; p < passes; p++) {
+    const int b = (bits - shift + (passes - p) - 1) / (passes - p);  // digits of equal width
+    int32_t *ko = kbuf[p & 1], *vo = (passes - 1 - p) & 1 ? vtmp : g->perm;
+    rs_count_kernel<<<tiles, RS_NT, 0, s>>>(kin, m, shift, b, tiles, cnt);
+    MG_TRY(device_exclusive_scan(cnt, ofs, (int64_t)tiles << b, tmp, s));
+    rs_scatter_kernel<<<tiles, RS_NT, 0, s>>>(kin, vin, m, shift, b, tiles, ofs, ko, vo);
+    kin = ko;
+    vin = vo;
+    shift += b;
+  }
+  csc_offsets_kernel<<<(unsigned)(n / 256 + 1), 256, 0, s>>>(kin, m, n, g->co);
+  // the sorted keys are done with: the pairs take their place
+  const unsigned et = (unsigned)((m + 256 * EP_VT - 1) / (256 * EP_VT));
+  const int grid = g->num_sms * 8;
+  if (vbytes) {
+    edge_rows_kernel<true><<<et, 256, 0, s>>>(g->ro, n, m, (const int32_t *)g->vals, keys);
+    csc_gather_kernel<true><<<grid, 256, 0, s>>>(g->perm, keys, m, g->ri, (int32_t *)g->cvals);
+  } else {
+    edge_rows_kernel<false><<<et, 256, 0, s>>>(g->ro, n, m, nullptr, keys);
+    csc_gather_kernel<false><<<grid, 256, 0, s>>>(g->perm, keys, m, g->ri, nullptr);
   }
   MG_CUDA_TRY(cudaGetLastError());
   return MG_OK;
