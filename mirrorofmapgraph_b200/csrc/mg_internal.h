@@ -74,6 +74,12 @@ struct DevCtl {
   int32_t trace_len;  // per-level trace records written by this run (mg_graph_trace)
   uint32_t bar_count;
   uint32_t bar_gen;
+  // persistent near-far SSSP: per-step counters in a ring of three (near items
+  // appended, chunks, edges of the frontier, smallest waiting distance)
+  int32_t sq[3];
+  int32_t sc[3];
+  int32_t smin[3];
+  int64_t se[3];
 };
 
 // Padding of the device graph arrays. Offsets arrays hold n + 1 + MG_OFF_PAD

@@ -51,6 +51,8 @@ struct SsspArgs {
   DevCtl *ctl;
   cudaGraphConditionalHandle h;
   int32_t use_cond;
+  uint32_t bar_extra;            // test hook (mg_debug_barrier_skew)
+  unsigned long long bar_limit;  // barrier polls before MG_ERR_TIMEOUT
 };
 
 // Per-warp staging of next-frontier appends in shared memory: one global atomic
@@ -508,6 +510,192 @@ __global__ void __launch_bounds__(SSSP_NT) sssp_far_split_kernel(SsspArgs a) {
   if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
 }
 
+// All rounds of a near-far run in one cooperative launch. A high-diameter graph
+// takes hundreds of rounds of a few thousand vertices (4096^2 lattice: 437), where
+// a sequence of four launches per round cost 41 us a round, most of it in kernels
+// with nothing to do. Here a round is the relaxation and one grid barrier; rounds
+// with heavy vertices take a second barrier after their chunks, and a split of the
+// far pile takes two. One CTA of 1024 threads per SM: 148 arrivals per barrier.
+// Every block reads the same counters after a barrier and takes the same decisions.
+//
+// Counters rotate over three slots, one per step (a round or a split): a step adds
+// to its own slot and block 0 clears the next step's, which was last read two steps
+// ago, so at least one barrier lies between.
+constexpr int NF_NT = 1024;
+constexpr unsigned long long NF_WAIT = 1ull << 22;  // barrier polls (seconds at most) before giving up
+
+__global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
+  __shared__ int32_t s_stage[NF_NT / 32][SSSP_WS];
+  __shared__ int64_t s_sum[NF_NT / 32 + 1];
+  DevCtl *c = a.ctl;
+  if (vload(&c->done)) return;
+  const int lane = lane_id();
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  const int32_t nw = gridDim.x * (NF_NT / 32);
+  const int32_t gw = warp_id() * gridDim.x + blockIdx.x;  // neighbouring warps of work on different SMs
+  const int32_t hi = ~a.vmask;
+  const int32_t iter_cap = vload(&c->iter_cap);
+  int32_t nin = vload(&c->qlen[0]);
+  int sel = 0, fc = 0, step = 0, splits = 0;
+  int32_t lvl = 0;
+  int64_t thr = vload(&c->thr);
+  int64_t insp = 0, nexp = 0, upd = 0;
+  bool ok = true, done = false, over = false;
+  auto barrier = [&]() { return grid_barrier(&c->bar_count, &c->bar_gen, a.bar_limit, a.bar_extra); };
+  auto next_slot = [&]() {
+    const int slot = step % 3, z = (step + 1) % 3;
+    step++;
+    if (lead) {
+      c->sq[z] = 0;
+      c->sc[z] = 0;
+      c->se[z] = 0;
+      c->smin[z] = INT_MAX;
+    }
+    return slot;
+  };
+  while (!done) {
+    const int slot = next_slot();
+    const int32_t *qin = sel ? a.q1 : a.q0;
+    uint32_t *inq_cur = sel ? a.inq1 : a.inq0;
+    RelaxCtx x{a.dist, sel ? a.inq0 : a.inq1, a.ro, sel ? a.q0 : a.q1, &c->sq[slot], &c->overflow, a.qcap, a.vmask, 0,
+               a.delta, thr, a.infar, fc ? a.far1 : a.far0, &c->far_len[fc]};
+    WarpStage st{s_stage[warp_id()], 0};
+    const int32_t th = nin < nw * 32 ? a.heavy_small : a.heavy;
+    int64_t edges = 0;
+    for (int64_t base = (int64_t)gw * 32; base < nin; base += (int64_t)nw * 32) {
+      const int64_t i = base + lane;
+      const int32_t v = i < nin ? __ldcg(qin + i) : -1;
+      int32_t beg = 0, deg = 0, dv = 0, cb = 0, cdeg = 0;
+      if (v >= 0) {
+        inq_cur[v >> 5] = 0u;
+        nexp++;
+        beg = a.ro[v & a.vmask];
+        deg = a.ro[(v & a.vmask) + 1] - beg;
+        dv = vload(a.dist + v);
+        if (a.both) {
+          cb = a.co[v & a.vmask];
+          cdeg = a.co[(v & a.vmask) + 1] - cb;
+        }
+        edges += deg + cdeg;
+      }
+      deg = warp_chunks(a, &c->sc[slot], v, beg, deg, th, 0);
+      warp_walk(x, st, v, dv, beg, deg, a.ci, a.w, hi);
+      if (a.both) {
+        cdeg = warp_chunks(a, &c->sc[slot], v, cb, cdeg, th, INT_MIN);
+        warp_walk(x, st, v, dv, cb, cdeg, a.ri, a.cw, hi);
+      }
+    }
+    ws_flush(st, x.qout, x.qlen_out, x.qcap, x.overflow);
+    insp += edges;
+    edges = warp_sum(edges);
+    if (lane == 0 && edges) atomicAdd((unsigned long long *)&c->se[slot], (unsigned long long)edges);
+    if (!(ok = barrier())) break;
+    const int32_t nch = min(vload(&c->sc[slot]), a.chunk_cap);
+    if (nch > 0) {
+      for (int32_t ch = gw; ch < nch; ch += nw) {
+        const int2 e = __ldcg(a.chunks + ch);
+        if (e.x < 0) continue;
+        const bool rev = e.y < 0;
+        const int32_t k0 = e.y & INT_MAX;
+        const int32_t *off = rev ? a.co : a.ro;
+        const int32_t *adj = rev ? a.ri : a.ci;
+        const int32_t *wt = rev ? a.cw : a.w;
+        const int32_t end = min(k0 + SSSP_CH, off[(e.x & a.vmask) + 1]);
+        const int32_t dv = vload(a.dist + e.x);
+        for (int32_t b = k0; b < end; b += 32 * SSSP_U) {
+          int32_t u[SSSP_U], w[SSSP_U], d[SSSP_U];
+#pragma unroll
+          for (int r = 0; r < SSSP_U; r++) {
+            const int32_t k = b + r * 32 + lane;
+            const bool in = k < end;
+            u[r] = in ? ((e.x & hi) | adj[k]) : -1;
+            w[r] = in ? (wt ? wt[k] : 1) : 0;
+            d[r] = dv;
+          }
+          relax_group(x, st, u, w, d);
+        }
+      }
+      ws_flush(st, x.qout, x.qlen_out, x.qcap, x.overflow);
+      if (!(ok = barrier())) break;
+    }
+    upd += x.updates;
+    // Round end (sssp_level_end's rules).
+    if (lead) trace_level(c, lvl, MG_DIR_PUSH, nin, vload(&c->se[slot]), 0.0);
+    int32_t nf = vload(&c->sq[slot]);
+    const int32_t nfar = vload(&c->far_len[fc]);
+    over = vload(&c->overflow) != 0;
+    lvl++;
+    sel ^= 1;
+    bool split = nf == 0 && nfar > 0 && !over;
+    done = (nf == 0 && !split) || lvl >= iter_cap || over;
+    while (split && !done) {
+      const int sp = next_slot();
+      const int32_t len = min(vload(&c->far_len[fc]), a.qcap);
+      const int32_t *far = fc ? a.far1 : a.far0;
+      int32_t *keep_to = fc ? a.far0 : a.far1;
+      int32_t mn = INT_MAX;
+      for (int32_t i = gw * 32 + lane; i < len; i += nw * 32) {
+        const int32_t d = vload(a.dist + __ldcg(far + i));
+        if ((int64_t)d >= thr) mn = min(mn, d);
+      }
+      mn = __reduce_min_sync(FULL, mn);
+      if (lane == 0 && mn != INT_MAX) atomicMin(&c->smin[sp], mn);
+      if (!(ok = barrier())) break;
+      const int32_t fmin = vload(&c->smin[sp]);
+      const int64_t thr_new = (fmin == INT_MAX ? thr : max(thr, (int64_t)fmin)) + a.delta;
+      int32_t *qnear = sel ? a.q1 : a.q0;
+      uint32_t *inq_near = sel ? a.inq1 : a.inq0;
+      for (int64_t base = (int64_t)gw * 32; base < len; base += (int64_t)nw * 32) {
+        const int64_t i = base + lane;
+        bool to_near = false, keep = false;
+        int32_t u = 0;
+        if (i < len) {
+          u = __ldcg(far + i);
+          const int64_t d = vload(a.dist + u);
+          const uint32_t bit = 1u << (u & 31);
+          if (d < thr_new) {
+            atomicAnd(a.infar + (u >> 5), ~bit);
+            if (d >= thr) to_near = !(atomicOr(inq_near + (u >> 5), bit) & bit);
+          } else {
+            keep = true;
+          }
+        }
+        __syncwarp();
+        warp_append(to_near, u, qnear, &c->sq[sp], a.qcap, &c->overflow);
+        warp_append(keep, u, keep_to, &c->far_len[fc ^ 1], a.qcap, &c->overflow);
+      }
+      if (!(ok = barrier())) break;
+      nf = vload(&c->sq[sp]);
+      const int32_t nk = vload(&c->far_len[fc ^ 1]);
+      over = vload(&c->overflow) != 0;
+      thr = thr_new;
+      // the old pile's length: next added to two barriers from now
+      if (lead) c->far_len[fc] = 0;
+      fc ^= 1;
+      splits++;
+      done = (nf == 0 && nk == 0) || over;
+      split = nf == 0 && nk > 0;
+    }
+    if (!ok) break;
+    nin = nf;
+  }
+  const int64_t b0 = block_sum<NF_NT>(insp, s_sum);
+  const int64_t b1 = block_sum<NF_NT>(nexp, s_sum);
+  const int64_t b2 = block_sum<NF_NT>(upd, s_sum);
+  if (threadIdx.x == 0) {
+    if (b0) atomicAdd((unsigned long long *)&c->edges_inspected, (unsigned long long)b0);
+    if (b1) atomicAdd((unsigned long long *)&c->vertices_expanded, (unsigned long long)b1);
+    if (b2) atomicAdd((unsigned long long *)&c->vertices_updated, (unsigned long long)b2);
+    if (!ok) c->status = MG_ERR_TIMEOUT;
+  }
+  if (lead) {
+    c->level = lvl;
+    c->splits = splits;
+    if (over) c->status = MG_ERR_QUEUE_OVERFLOW;
+    c->done = 1;
+  }
+}
+
 __global__ void sssp_clear_kernel(int32_t *dist, uint32_t *b0, uint32_t *b1, uint32_t *b2, int64_t n) {
   const int64_t nw = (n + 31) >> 5;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -539,6 +727,7 @@ __global__ void sssp_seed_kernel(SsspArgs a, const int32_t *srcs, int32_t nsrc, 
     c->iter_cap = iter_cap;
     c->thr = a.delta > 0 ? (int64_t)a.delta : INT64_MAX;
     c->far_min = INT_MAX;
+    c->smin[0] = INT_MAX;
     c->done = c->overflow ? 1 : 0;
     if (c->overflow) c->status = MG_ERR_QUEUE_OVERFLOW;
   }
@@ -1026,6 +1215,8 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
   a.ctl = g->ctl;
   a.h = 0;
   a.use_cond = 0;
+  a.bar_extra = (uint32_t)debug_barrier_extra();
+  a.bar_limit = a.bar_extra ? debug_barrier_limit() : NF_WAIT;
   cudaStream_t s = g->stream;
   // Bellman-Ford rounds of every instance are bounded by its vertex count; the
   // near-far schedule adds rounds that find nothing new (a bucket's last round),
@@ -1061,8 +1252,22 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
       sssp_far_split_kernel<<<grid, SSSP_NT, 0, st>>>(b);
     }
   };
-  MG_TRY(run_loop(g, vmask == -1 ? SLOT_SSSP : SLOT_BSSSP, &sig, sizeof(sig), o.use_graph >= 0, body,
-                  (int64_t)iter_cap + 2));
+  // Near-far rounds in one cooperative launch where a CTA of it fits every SM; the
+  // per-round kernels serve plain rounds and the host-driven loop.
+  bool persist = false;
+  if (a.delta > 0 && o.use_graph >= 0) {
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sssp_persist_kernel, NF_NT, 0) == cudaSuccess && occ > 0) {
+      SsspArgs pa = a;
+      void *params[] = {&pa};
+      persist = cudaLaunchCooperativeKernel((const void *)sssp_persist_kernel, dim3(g->num_sms), dim3(NF_NT), params, 0,
+                                            s) == cudaSuccess;
+    }
+    cudaGetLastError();
+  }
+  if (!persist)
+    MG_TRY(run_loop(g, vmask == -1 ? SLOT_SSSP : SLOT_BSSSP, &sig, sizeof(sig), o.use_graph >= 0, body,
+                    (int64_t)iter_cap + 2));
   sssp_reach_kernel<<<g->num_sms * 4, 256, 0, s>>>(dist, nitems, vmask, g->ro, g->ctl);
   MG_CUDA_TRY(cudaGetLastError());
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
@@ -1078,8 +1283,14 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     stats->kernel_ms = ms;
     const int64_t per = a.delta > 0 ? 4 : 3;
-    stats->launches = 3 + (o.use_graph >= 0 ? (per + 1) * (int64_t)hc.body_iters : per * (int64_t)hc.level);
+    stats->launches = 3 + (persist             ? 1
+                           : o.use_graph >= 0 ? (per + 1) * (int64_t)hc.body_iters
+                                              : per * (int64_t)hc.level);
     stats->status_detail = a.delta > 0 ? a.delta : 0;
+  }
+  if (hc.status == MG_ERR_TIMEOUT) {
+    mg_set_error("mg_sssp: a grid barrier of the near-far rounds timed out");
+    return MG_ERR_TIMEOUT;
   }
   if (hc.status != 0) {
     mg_set_error("mg_sssp: device status %d (queue capacity %d)", hc.status, qcap);
