@@ -24,6 +24,8 @@
 // The direction switch (Beamer's heuristic: go bottom-up when the frontier's
 // out-edges exceed 1/14 of the unexplored edges, back when the frontier drops
 // below n/24) is evaluated on the device.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -80,6 +82,16 @@ inline void bfs_tuning(BfsArgs &a, const mg_tuning &t) {
   a.persist_edges = t.bfs_persist_edges;
   a.alpha = t.bfs_alpha;
   a.beta = t.bfs_beta;
+}
+
+// Whether the BFS thresholds are the defaults.
+inline bool bfs_tuning_default(const mg_tuning &t) {
+  const mg_tuning d = tuning_defaults();
+  return t.bfs_cta_th == d.bfs_cta_th && t.bfs_grid_th == d.bfs_grid_th && t.bfs_defer_warp == d.bfs_defer_warp &&
+         t.bfs_persist_max == d.bfs_persist_max && t.bfs_persist_edges == d.bfs_persist_edges &&
+         t.bfs_alpha == d.bfs_alpha && t.bfs_beta == d.bfs_beta && t.bfs_sparse_degree == d.bfs_sparse_degree &&
+         t.bfs_ctas_per_sm == d.bfs_ctas_per_sm && t.bfs_tail_max == d.bfs_tail_max &&
+         t.bfs_tail_edges == d.bfs_tail_edges;
 }
 
 __device__ void bfs_level_end(const BfsArgs &a) {
@@ -456,6 +468,224 @@ __global__ void bfs_seed_kernel(BfsArgs a, const int32_t *srcs, int32_t nsrc, in
   }
 }
 
+// A whole BFS of a small graph in one launch of one thread-block cluster: clear,
+// seeds, every level, counters. Levels are separated by the hardware cluster
+// barrier (well under a microsecond), where a grid barrier of every SM takes about
+// three and a launch per level more, and the level's lengths live in the first
+// CTA's shared memory. Each CTA keeps a copy of the visited bitmap, refreshed per
+// level, so most edges to vertices already reached end there; the others claim
+// their vertex with one atomic on the bitmap in L2. Latency bounds it: about eight
+// dependent memory round trips per level. Top-down only: the edges it could skip
+// bottom-up cost less than the extra passes at these sizes.
+//
+// The limits are where the cluster's 8 SMs stop beating the whole grid's per-level
+// kernels.
+constexpr int SB_NT = 1024;
+constexpr int SB_CLUSTER = 8;
+constexpr int64_t SB_MAX_N = 1 << 17;
+constexpr int64_t SB_MAX_M = 1 << 20;
+constexpr int SB_CH = 256;   // edges per chunk of a heavy vertex
+constexpr int SB_U = 4;      // edges a lane has in flight
+constexpr int SB_SRC = 8;    // sources passed by value
+
+struct SmallBfs {
+  int32_t src[SB_SRC];
+  const int32_t *dsrc;  // more sources than SB_SRC (else nullptr)
+  int32_t nsrc;
+  int32_t iter_cap;
+  int2 *chunks;  // {first edge | 1 << 31 for a CSC edge, end}
+};
+
+// Most chunks of a level: a vertex of at least SB_CH edges has under twice its
+// edges / SB_CH, in each direction.
+inline int32_t small_bfs_chunks(int64_t m) { return (int32_t)(4 * (m / SB_CH) + 64); }
+
+__global__ void __cluster_dims__(SB_CLUSTER, 1, 1) __launch_bounds__(SB_NT, 1)
+    bfs_small_kernel(BfsArgs a, SmallBfs sb) {
+  namespace cg = cooperative_groups;
+  __shared__ uint32_t s_vis[SB_MAX_N / 32];
+  __shared__ BlockQueue bq;
+  __shared__ int32_t s_len[3], s_chunk[3];
+  __shared__ unsigned long long s_mf[3], s_tot[2];
+  cg::cluster_group cl = cg::this_cluster();
+  DevCtl *c = a.ctl;
+  const int rank = (int)cl.block_rank(), tid = threadIdx.x, lane = lane_id();
+  const bool lead = rank == 0 && tid == 0;
+  const int32_t nthr = SB_CLUSTER * SB_NT, gt = tid * SB_CLUSTER + rank;
+  const int32_t nw = nthr / 32, gw = warp_id() * SB_CLUSTER + rank;
+  int32_t *len = cl.map_shared_rank(s_len, 0), *chunk = cl.map_shared_rank(s_chunk, 0);
+  unsigned long long *mfs = cl.map_shared_rank(s_mf, 0), *tot = cl.map_shared_rank(s_tot, 0);
+  const int32_t nwords = (int32_t)((a.n + 31) >> 5);
+  for (int32_t i = rank * SB_NT + tid; i < a.n; i += nthr) a.label[i] = -1;
+  for (int32_t i = rank * SB_NT + tid; i < nwords; i += nthr) a.vis[i] = 0u;
+  if (rank == 0) {
+    for (int i = tid; i < (int)(sizeof(DevCtl) / 4); i += SB_NT) reinterpret_cast<int32_t *>(c)[i] = 0;
+    if (tid < 3) {
+      s_len[tid] = 0;
+      s_chunk[tid] = 0;
+      s_mf[tid] = 0;
+    }
+    if (tid < 2) s_tot[tid] = 0;
+  }
+  bq_init(bq);
+  cl.sync();
+  if (rank == 0) {
+    for (int i = tid; i < sb.nsrc; i += SB_NT) {
+      const int32_t v = sb.dsrc ? sb.dsrc[i] : sb.src[i];
+      const uint32_t bit = 1u << (v & 31);
+      if (!(atomicOr(a.vis + (v >> 5), bit) & bit)) {
+        a.label[v] = 0;
+        const int pos = atomicAdd(&s_len[0], 1);
+        if (pos < a.qcap) a.q0[pos] = v;
+        else c->overflow = 1;
+      }
+    }
+  }
+  cl.sync();
+  int32_t nin = len[0];
+  int32_t lvl = 0, sel = 0;
+  bool over = vload(&c->overflow) != 0;
+  bool done = over || sb.iter_cap <= 0;
+  int64_t insp = 0, nexp = 0, vdeg = 0;
+  // claims the items u (-1: none) of a lane, issued together
+  auto claim = [&](const int32_t (&u)[SB_U], int32_t *qout, int32_t *qlen) {
+    uint32_t old[SB_U];
+#pragma unroll
+    for (int r = 0; r < SB_U; r++) {
+      const uint32_t bit = 1u << (u[r] & 31);
+      old[r] = FULL;
+      if (u[r] >= 0 && !(s_vis[u[r] >> 5] & bit)) {
+        old[r] = atomicOr(a.vis + (u[r] >> 5), bit);
+        atomicOr(s_vis + (u[r] >> 5), bit);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < SB_U; r++) {
+      const bool fresh = u[r] >= 0 && !((old[r] >> (u[r] & 31)) & 1u);
+      if (fresh) a.label[u[r]] = lvl + 1;
+      staged_append(&bq, fresh, u[r], qout, qlen, a.qcap, &c->overflow);
+    }
+  };
+  // the edges of the warp's vertices (a lane each), concatenated
+  auto walk = [&](int32_t beg, int32_t deg, const int32_t *__restrict__ adj, int32_t flag, int32_t *qout, int32_t *qlen,
+                  int32_t *clen) {
+    const int32_t nch = deg >= SB_CH ? (deg + SB_CH - 1) / SB_CH : 0;
+    if (nch) {
+      const int32_t base = atomicAdd(clen, nch);
+      for (int32_t j = 0; j < nch; j++)  // within the capacity: a level's vertices are distinct
+        sb.chunks[base + j] = make_int2((beg + j * SB_CH) | flag, min(beg + (j + 1) * SB_CH, beg + deg));
+      deg = 0;
+    }
+    __syncwarp();
+    const int32_t inc = warp_inclusive_scan(deg);
+    const int32_t total = __shfl_sync(FULL, inc, 31);
+    const int32_t ex = inc - deg, kb = beg - ex;
+    for (int32_t b0 = 0; b0 < total; b0 += 32 * SB_U) {
+      int32_t u[SB_U];
+#pragma unroll
+      for (int r = 0; r < SB_U; r++) {
+        const int32_t j = b0 + r * 32 + lane;
+        int l = 0;
+#pragma unroll
+        for (int sft = 16; sft > 0; sft >>= 1)
+          if (__shfl_sync(FULL, ex, l + sft) <= j) l += sft;
+        const int32_t k = __shfl_sync(FULL, kb, l) + j;
+        u[r] = j < total ? adj[k] : -1;
+      }
+      claim(u, qout, qlen);
+    }
+  };
+  while (!done) {
+    // counters in a ring of three: this level adds to `out`; nobody reads or adds to
+    // the next level's now
+    const int out = (lvl + 1) % 3, zero = (lvl + 2) % 3;
+    if (lead) {
+      s_len[zero] = 0;
+      s_chunk[zero] = 0;
+      s_mf[zero] = 0;
+    }
+    for (int32_t i = tid; i < nwords; i += SB_NT) s_vis[i] = __ldcg(a.vis + i);
+    __syncthreads();
+    const int32_t *qin = sel ? a.q1 : a.q0;
+    int32_t *qout = sel ? a.q0 : a.q1, *qlen = len + out, *clen = chunk + out;
+    // a small frontier is spread over all the warps
+    const int32_t per = max(1, min(32, (nin + nw - 1) / nw));
+    int64_t front = 0;
+    for (int32_t base = gw * per; base < nin; base += nw * per) {
+      const int32_t i = base + lane;
+      const int32_t v = lane < per && i < nin ? __ldcg(qin + i) : -1;
+      int32_t beg = 0, deg = 0, cb = 0, cdeg = 0;
+      if (v >= 0) {
+        beg = a.ro[v];
+        deg = a.ro[v + 1] - beg;
+        if (a.both) {
+          cb = a.co[v];
+          cdeg = a.co[v + 1] - cb;
+        }
+        front += deg;
+        insp += deg + cdeg;
+        nexp++;
+      }
+      walk(beg, deg, a.ci, 0, qout, qlen, clen);
+      if (a.both) walk(cb, cdeg, a.ri, INT_MIN, qout, qlen, clen);
+    }
+    front = warp_sum(front);
+    if (lane == 0 && front) atomicAdd(mfs + out, (unsigned long long)front);
+    cl.sync();
+    const int32_t nch = chunk[out];
+    if (nch > 0) {
+      for (int32_t ch = gw; ch < nch; ch += nw) {
+        const int2 e = __ldcg(sb.chunks + ch);
+        const int32_t k0 = e.x & INT_MAX;
+        const int32_t *adj = e.x < 0 ? a.ri : a.ci;
+        for (int32_t b = k0; b < e.y; b += 32 * SB_U) {
+          int32_t u[SB_U];
+#pragma unroll
+          for (int r = 0; r < SB_U; r++) u[r] = b + r * 32 + lane < e.y ? adj[b + r * 32 + lane] : -1;
+          claim(u, qout, qlen);
+        }
+      }
+    }
+    bq_flush(bq, qout, qlen, a.qcap, &c->overflow);
+    cl.sync();
+    // Level end, alike in every CTA.
+    const int64_t mf = (int64_t)mfs[out];
+    const int32_t nf = len[out];
+    over = vload(&c->overflow) != 0;
+    if (lead) {
+      trace_level(c, lvl, MG_DIR_PUSH, nin, mf, 0.0);
+      vdeg += mf;
+    }
+    lvl++;
+    sel ^= 1;
+    nin = nf;
+    done = nf == 0 || lvl >= sb.iter_cap || over;
+  }
+  // an iteration cap leaves a frontier that was reached but not expanded
+  const int32_t *qin = sel ? a.q1 : a.q0;
+  int64_t rest = 0;
+  for (int32_t i = gt; i < min(nin, a.qcap); i += nthr) {
+    const int32_t v = __ldcg(qin + i);
+    rest += a.ro[v + 1] - a.ro[v];
+  }
+  insp = warp_sum(insp);
+  nexp = warp_sum(nexp);
+  rest = warp_sum(rest + vdeg);
+  if (lane == 0) {
+    if (insp) atomicAdd(tot, (unsigned long long)insp);
+    if (nexp) atomicAdd(tot + 1, (unsigned long long)nexp);
+    if (rest) atomicAdd((unsigned long long *)&c->visited_deg, (unsigned long long)rest);
+  }
+  cl.sync();  // the last access to the first CTA's shared memory
+  if (lead) {
+    c->edges_inspected = (int64_t)s_tot[0];
+    c->vertices_expanded = (int64_t)s_tot[1];
+    c->level = lvl;
+    if (over) c->status = MG_ERR_QUEUE_OVERFLOW;
+    c->done = 1;
+  }
+}
+
 }  // namespace mg
 
 // Blocks of the persistent kernel: every SM's resident share (0 when the
@@ -505,7 +735,9 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
   const int64_t nwords = (n + 31) / 32;
   const size_t need = Carve::need({sizeof(int32_t) * (size_t)n, sizeof(uint32_t) * (size_t)nwords,
                                    sizeof(int32_t) * (size_t)qcap, sizeof(int32_t) * (size_t)qcap,
-                                   sizeof(int32_t) * (size_t)nsrc, sizeof(int32_t) * (size_t)BIG_CAP});
+                                   sizeof(int32_t) * (size_t)nsrc, sizeof(int32_t) * (size_t)BIG_CAP,
+                                   sizeof(int2) * (size_t)(n <= SB_MAX_N && g->m <= SB_MAX_M ? small_bfs_chunks(g->m)
+                                                                                             : 0)});
   MG_TRY(ws_reserve(g, g->ws_main, need));
   Carve cv(g->ws_main.ptr);
   int32_t *label_ws = cv.take<int32_t>(n);
@@ -547,56 +779,75 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
   a.bar_limit = a.bar_extra ? debug_barrier_limit() : PERSIST_WAIT;
 
   const int32_t iter_cap = o.iter_num > 0 ? (int32_t)std::min<int64_t>(o.iter_num, n + 1) : (int32_t)(n + 1);
-  MG_CUDA_TRY(cudaMemcpyAsync(dsrc, srcs, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, s));
-  MG_CUDA_TRY(cudaEventRecord(g->ev0, s));
-  MG_CUDA_TRY(cudaMemsetAsync(g->ctl, 0, sizeof(DevCtl), s));
-  bfs_clear_kernel<<<g->num_sms * 8, 256, 0, s>>>(label, vis, n);
-  bfs_seed_kernel<<<1, 1024, 0, s>>>(a, dsrc, nsrc, iter_cap, 0);
-  MG_CUDA_TRY(cudaGetLastError());
-  // Small push levels first, in one persistent cooperative launch (all blocks
-  // resident); a device that cannot co-schedule the grid skips it.
-  const int pgrid = persist_grid(g);
-  int64_t persist_launches = 0;
-  if (pgrid > 0 && o.direction != MG_DIR_PULL) {
-    BfsArgs pa = a;
-    void *params[] = {&pa};
-    if (cudaLaunchCooperativeKernel((const void *)bfs_persist_kernel, dim3(pgrid), dim3(BFS_NT), params, 0, s) ==
-        cudaSuccess)
-      persist_launches = 1;
-    cudaGetLastError();
-  }
-
-  const int grid = g->num_sms * g->tune.bfs_ctas_per_sm;
   const bool use_graph = o.use_graph >= 0;
-  struct Sig {
-    BfsArgs a;
-    int grid;
-    int32_t tail_max, tail_edges;
-  } sig;
-  std::memset(&sig, 0, sizeof(sig));
-  sig.a = a;
-  sig.grid = grid;
-  sig.tail_max = g->tune.bfs_tail_max;
-  sig.tail_edges = g->tune.bfs_tail_edges;
-  // Tail levels: one CTA runs the persistent kernel at the top of every iteration
-  // (its grid barrier is the CTA's own), so a run of tiny push levels (at most
-  // bfs_tail_max vertices and bfs_tail_edges out-edges) costs one launch instead of
-  // a launch sequence per level; on a larger frontier it returns at once and the
-  // per-level kernels go on from the same control block.
-  BfsArgs ta = a;
-  ta.persist_max = g->tune.bfs_tail_max;
-  ta.persist_edges = g->tune.bfs_tail_edges;
-  const bool tail = ta.persist_max > 0 && ta.persist_edges > 0 && o.direction != MG_DIR_PULL;
-  LoopBody body = [a, ta, tail, grid](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) {
-    BfsArgs b = a;
-    b.h = h;
-    b.use_cond = use_cond;
-    if (tail) bfs_persist_kernel<<<1, BFS_NT, 0, st>>>(ta);
-    bfs_push_kernel<<<grid, BFS_NT, 0, st>>>(b);
-    bfs_push_big_kernel<<<grid, BFS_NT, 0, st>>>(b);
-    bfs_pull_kernel<<<grid, BFS_NT, 0, st>>>(b);
-  };
-  MG_TRY(run_loop(g, SLOT_BFS, &sig, sizeof(sig), use_graph, body, n + 2));
+  // Small graphs in one cluster launch, unless the caller asked for bottom-up levels
+  // or the per-level kernels (host-driven loop, thresholds of its own for them), or a
+  // test skews the grid barriers.
+  const bool small = n <= SB_MAX_N && g->m <= SB_MAX_M && use_graph && o.direction != MG_DIR_PULL &&
+                     a.bar_extra == 0 && bfs_tuning_default(g->tune);
+  if (!small || nsrc > SB_SRC)
+    MG_CUDA_TRY(cudaMemcpyAsync(dsrc, srcs, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, s));
+  MG_CUDA_TRY(cudaEventRecord(g->ev0, s));
+  int64_t persist_launches = 0;
+  bool tail = false;
+  if (small) {
+    SmallBfs sb;
+    std::memset(&sb, 0, sizeof(sb));
+    for (int i = 0; i < std::min(nsrc, SB_SRC); i++) sb.src[i] = srcs[i];
+    sb.dsrc = nsrc > SB_SRC ? dsrc : nullptr;
+    sb.nsrc = nsrc;
+    sb.iter_cap = iter_cap;
+    sb.chunks = cv.take<int2>(small_bfs_chunks(g->m));
+    bfs_small_kernel<<<SB_CLUSTER, SB_NT, 0, s>>>(a, sb);
+    MG_CUDA_TRY(cudaGetLastError());
+  } else {
+    MG_CUDA_TRY(cudaMemsetAsync(g->ctl, 0, sizeof(DevCtl), s));
+    bfs_clear_kernel<<<g->num_sms * 8, 256, 0, s>>>(label, vis, n);
+    bfs_seed_kernel<<<1, 1024, 0, s>>>(a, dsrc, nsrc, iter_cap, 0);
+    MG_CUDA_TRY(cudaGetLastError());
+    // Small push levels first, in one persistent cooperative launch (all blocks
+    // resident); a device that cannot co-schedule the grid skips it.
+    const int pgrid = persist_grid(g);
+    if (pgrid > 0 && o.direction != MG_DIR_PULL) {
+      BfsArgs pa = a;
+      void *params[] = {&pa};
+      if (cudaLaunchCooperativeKernel((const void *)bfs_persist_kernel, dim3(pgrid), dim3(BFS_NT), params, 0, s) ==
+          cudaSuccess)
+        persist_launches = 1;
+      cudaGetLastError();
+    }
+
+    const int grid = g->num_sms * g->tune.bfs_ctas_per_sm;
+    struct Sig {
+      BfsArgs a;
+      int grid;
+      int32_t tail_max, tail_edges;
+    } sig;
+    std::memset(&sig, 0, sizeof(sig));
+    sig.a = a;
+    sig.grid = grid;
+    sig.tail_max = g->tune.bfs_tail_max;
+    sig.tail_edges = g->tune.bfs_tail_edges;
+    // Tail levels: one CTA runs the persistent kernel at the top of every iteration
+    // (its grid barrier is the CTA's own), so a run of tiny push levels (at most
+    // bfs_tail_max vertices and bfs_tail_edges out-edges) costs one launch instead of
+    // a launch sequence per level; on a larger frontier it returns at once and the
+    // per-level kernels go on from the same control block.
+    BfsArgs ta = a;
+    ta.persist_max = g->tune.bfs_tail_max;
+    ta.persist_edges = g->tune.bfs_tail_edges;
+    tail = ta.persist_max > 0 && ta.persist_edges > 0 && o.direction != MG_DIR_PULL;
+    LoopBody body = [a, ta, tail, grid](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) {
+      BfsArgs b = a;
+      b.h = h;
+      b.use_cond = use_cond;
+      if (tail) bfs_persist_kernel<<<1, BFS_NT, 0, st>>>(ta);
+      bfs_push_kernel<<<grid, BFS_NT, 0, st>>>(b);
+      bfs_push_big_kernel<<<grid, BFS_NT, 0, st>>>(b);
+      bfs_pull_kernel<<<grid, BFS_NT, 0, st>>>(b);
+    };
+    MG_TRY(run_loop(g, SLOT_BFS, &sig, sizeof(sig), use_graph, body, n + 2));
+  }
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
   if (!o.device_output) MG_TRY(copy_out(g, depth, label, sizeof(int32_t) * n, 0));
   MG_TRY(fetch_ctl(g));
@@ -613,7 +864,7 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
     stats->kernel_ms = ms;
     stats->status_detail = hc.levels_pull;
     const int64_t per = 3 + (tail ? 1 : 0);
-    stats->launches = 2 + persist_launches + (use_graph ? (per + 1) * (int64_t)hc.body_iters : per * g->host_iters);
+    stats->launches = small ? 1 : 2 + persist_launches + (use_graph ? (per + 1) * (int64_t)hc.body_iters : per * g->host_iters);
   }
   if (hc.status == MG_ERR_TIMEOUT) {
     mg_set_error("mg_bfs: a grid barrier of the persistent levels timed out");

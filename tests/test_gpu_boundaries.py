@@ -1,0 +1,195 @@
+"""Kernels at the sizes where their tiles, bins and limits end, against the oracle:
+the degree bins of the PageRank gather and of its adjoint, the radix sort behind the
+CSC, the sampled forest of the components, the reference-compatible sweep in its
+three forms, the near-far rounds in one launch and the cluster BFS of small graphs."""
+import numpy as np
+import pytest
+
+import oracle
+import mirrorofmapgraph_b200 as mg
+
+pytestmark = pytest.mark.gpu
+
+L1_TOL = 1e-6  # FP32 compensated sums against the FP64 oracle, same iterations
+
+
+def _csr(n, src, dst, w=None):
+    order = np.argsort(src, kind="stable")
+    ro = np.searchsorted(src[order], np.arange(n + 1)).astype(np.int32)
+    return ro, dst[order].astype(np.int32), None if w is None else w[order]
+
+
+def _device_array(ptr, n, dtype):
+    import torch
+
+    class View:
+        __cuda_array_interface__ = {"data": (ptr, False), "shape": (n,), "typestr": np.dtype(dtype).str, "version": 2}
+    return torch.as_tensor(View(), device="cuda").cpu().numpy()
+
+
+def _in_degrees(degs, seed):
+    """A digraph whose vertex i has degs[i] in-edges from random vertices."""
+    rng = np.random.default_rng(seed)
+    n = max(len(degs), 64)
+    dst = np.repeat(np.arange(len(degs)), degs)
+    src = rng.integers(0, n, dst.size)
+    p = rng.permutation(dst.size)
+    return (n,) + _csr(n, src[p], dst[p], rng.lognormal(0, 1, dst.size).astype(np.float32))
+
+
+# every bin's first and last degree, one or several rows of each
+BIN_DEGREES = [0, 1, 2, 3, 4, 5, 8, 9, 12, 13, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65, 255, 256, 257, 2047, 2048, 4097]
+
+
+@pytest.mark.parametrize("rep", [1, 9, 33])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_gather_bins(rep, weighted):
+    n, ro, ci, w = _in_degrees(BIN_DEGREES * rep, rep)
+    with mg.Graph(ro, ci, w) as g:
+        for gather in ("binned", "cached"):
+            x, st = g.pagerank(mode="normalized", weighted=weighted, max_iter=12, tol=1e-30, gather=gather)
+            xr, _, _ = oracle.pr_normalized(ro, ci, w if weighted else None, 0.85, 0.0, 12)
+            assert np.abs(x - xr).sum() <= L1_TOL
+    # the adjoint gathers over the rows: the same degrees on the out-side
+    co, ri, _ = mg.csr_to_csc(mg.HostCsr(ro, ci))
+    wt = np.random.default_rng(1).lognormal(0, 1, ci.size).astype(np.float32)
+    dl = np.random.default_rng(2).standard_normal(n).astype(np.float32)
+    with mg.Graph(co, ri, wt) as g:
+        x, _ = g.pagerank(mode="normalized", weighted=weighted, max_iter=300, tol=1e-9)
+        gw, gt, _ = g.pagerank_backward(x, dl, weighted=weighted, tol=1e-7, max_iter=300)
+        rw, rt, _, _ = oracle.pr_adjoint(co, ri, wt if weighted else None, x.astype(np.float64), dl, 0.85, 1e-12, 1000)
+        assert np.linalg.norm(gw - rw) <= 1e-5 * np.linalg.norm(rw)
+        assert np.linalg.norm(gt - rt) <= 1e-5 * np.linalg.norm(rt)
+
+
+def test_edge_gradients_unaligned_output():
+    import torch
+    n, ro, ci, w = _in_degrees(BIN_DEGREES, 5)
+    dl = torch.randn(n, device="cuda")
+    with mg.Graph(torch.from_numpy(ro).cuda(), torch.from_numpy(ci).cuda(), torch.from_numpy(w).cuda()) as g:
+        x = g.pagerank(mode="normalized", weighted=True, out=torch.empty(n, device="cuda"))[0]
+        a = g.pagerank_backward(x, dl, weighted=True, out_weights=torch.empty(ci.size, device="cuda"),
+                                out_teleport=torch.empty(n, device="cuda"))[0]
+        buf = torch.full((ci.size + 2,), 7.0, device="cuda")
+        b = g.pagerank_backward(x, dl, weighted=True, out_weights=buf[1:-1],
+                                out_teleport=torch.empty(n, device="cuda"))[0]
+        # two solves agree to an ulp or so (their FP64 sums follow the work schedule)
+        assert torch.allclose(a, b, rtol=1e-5, atol=1e-7 * float(a.abs().max()))
+        assert buf[0] == 7.0 and buf[-1] == 7.0
+
+
+@pytest.mark.parametrize("n,m", [(1, 0), (1, 5), (2, 1), (3, 31), (255, 4095), (256, 4096), (257, 4097), (65536, 9000),
+                                 (65537, 70001), (300000, 5)])
+@pytest.mark.parametrize("vals", [None, np.int32, np.float32])
+@pytest.mark.parametrize("hot", [False, True])
+def test_csc_build(n, m, vals, hot):
+    rng = np.random.default_rng(n + m)
+    src, dst = rng.integers(0, n, m), rng.integers(0, n, m)
+    if hot:  # half of the edges into one column, from one row
+        dst[: m // 2] = n - 1
+        src[m // 3:] = n // 2
+    w = None if vals is None else rng.integers(1, 1000, m).astype(vals)
+    ro, ci, w = _csr(n, src, dst, w)
+    co, ri, perm = mg.csr_to_csc(mg.HostCsr(ro, ci))
+    with mg.Graph(ro, ci, w) as g:
+        d = g.device_arrays()
+        np.testing.assert_array_equal(_device_array(d["col_offsets"], n + 1, np.int32), co)
+        if m:
+            np.testing.assert_array_equal(_device_array(d["row_idx"], m, np.int32), ri)
+            np.testing.assert_array_equal(_device_array(d["csc_perm"], m, np.int32), perm)
+        if m and vals is not None:  # in-edge values: the undirected run reads them
+            if vals is np.int32:
+                np.testing.assert_array_equal(g.sssp([n // 2], directed=0)[0],
+                                              oracle.sssp(ro, ci, w, [n // 2], directed=0))
+            else:
+                x, _ = g.pagerank(mode="normalized", weighted=True, max_iter=5, tol=1e-30)
+                assert np.abs(x - oracle.pr_normalized(ro, ci, w, 0.85, 0.0, 5)[0]).sum() <= L1_TOL
+
+
+@pytest.mark.parametrize("shape", ["lattice", "path", "star", "pairs", "er1", "rmat", "isolated"])
+@pytest.mark.parametrize("sym", [False, True])
+def test_cc_forest(shape, sym):
+    rng = np.random.default_rng(3)
+    n = 5000
+    if shape == "lattice":
+        h = mg.gen_lattice(61, 83, 0.0, 1)
+        n, ro, ci = h.n, h.row_offsets, h.col_idx
+    elif shape == "rmat":
+        h = mg.gen_rmat(13, 3, 4, symmetrize=True)
+        n, ro, ci = h.n, h.row_offsets, h.col_idx
+    else:
+        src, dst = {"path": (np.arange(n - 1, 0, -1), np.arange(n - 2, -1, -1)),
+                    "star": (np.full(n - 1, n - 1), np.arange(n - 1)),
+                    "pairs": (np.arange(0, n, 2), np.arange(1, n, 2)),
+                    "er1": (rng.integers(0, n, n), rng.integers(0, n, n)),
+                    "isolated": (np.array([n - 1]), np.array([n - 1]))}[shape]
+        if sym:
+            src, dst = np.concatenate([src, dst]), np.concatenate([dst, src])
+        ro, ci, _ = _csr(n, src, dst)
+    with mg.Graph(ro, ci, symmetric=sym or shape in ("lattice", "rmat")) as g:
+        for rounds in (0, 1, 3):
+            g.set_tuning(cc_rounds=rounds)
+            np.testing.assert_array_equal(g.cc()[0], oracle.cc(ro, ci))
+
+
+@pytest.mark.parametrize("directed", [0, 1])
+@pytest.mark.parametrize("sym", [False, True])
+def test_refcompat_sweep(directed, sym):
+    n, ro, ci, _ = _in_degrees(BIN_DEGREES * 3, 8)
+    if sym:
+        src = np.repeat(np.arange(n), np.diff(ro))
+        ro, ci, _ = _csr(n, np.concatenate([src, ci]), np.concatenate([ci, src]))
+    with mg.Graph(ro, ci, symmetric=sym) as g:
+        for cap in (0, 1, 3):
+            x, st = g.pagerank(mode="refcompat", directed=directed, max_iter=cap)
+            xr, it = oracle.pr_refcompat(ro, ci, directed, cap or 2**31 - 1)
+            assert st["iterations"] == it
+            assert np.abs(x - xr).max() <= 1e-5 * max(1.0, np.abs(xr).max())
+
+
+@pytest.mark.parametrize("kind", ["lattice", "hubs", "path", "one"])
+@pytest.mark.parametrize("directed", [0, 1])
+def test_near_far_rounds(kind, directed):
+    if kind == "lattice":
+        h = mg.gen_lattice(90, 70, 0.01, 2, weights="int", p0=1, p1=1000)
+    elif kind == "hubs":  # mean degree 6, some vertices of thousands of edges: chunks
+        h = mg.gen_rmat(15, 3, 6, symmetrize=True, weights="int", p0=1, p1=50)
+    elif kind == "path":
+        n = 700
+        ro, ci, w = _csr(n, np.arange(n - 1), np.arange(1, n), np.arange(1, n, dtype=np.int32))
+        h = mg.HostCsr(ro, ci, w)
+    else:
+        h = mg.HostCsr(np.array([0, 1], dtype=np.int32), np.array([0], dtype=np.int32), np.array([3], dtype=np.int32))
+    with mg.Graph(h.row_offsets, h.col_idx, h.weights_i32) as g:
+        ref = oracle.sssp(h.row_offsets, h.col_idx, h.weights_i32, [0], directed=directed)
+        for delta in (0, 1, 37, 1 << 28):
+            d, st = g.sssp([0], directed=directed, delta=delta)
+            np.testing.assert_array_equal(d, ref)
+            assert st["edges_traversed"] == int(np.diff(h.row_offsets)[ref != 2**31 - 1].sum())
+        rows = g.sssp_batch([0, 0], directed=directed, delta=5)[0]
+        np.testing.assert_array_equal(rows[1], ref)
+
+
+@pytest.mark.parametrize("n,m", [(1, 0), (1, 3), (31, 60), (32, 64), (33, 40), (8193, 40000), (131072, 300000),
+                                 (131073, 300000), (500, 1 << 20), (500, (1 << 20) + 1)])
+@pytest.mark.parametrize("directed", [0, 1])
+def test_small_bfs(n, m, directed):
+    rng = np.random.default_rng(n + m)
+    src, dst = rng.integers(0, n, m), rng.integers(0, n, m)
+    src[: m // 3] = n // 2  # a hub: chunks
+    ro, ci, _ = _csr(n, src, dst)
+    deg = np.diff(ro)
+    with mg.Graph(ro, ci) as g:
+        for srcs in ([n // 2], [0, n - 1, 0], [int(v) for v in rng.integers(0, n, 11)]):
+            ref = oracle.bfs(ro, ci, srcs, directed=directed)
+            d, st = g.bfs(srcs, directed=directed)
+            np.testing.assert_array_equal(d, ref)
+            assert st["iterations"] == ref.max() + 1
+            assert st["edges_traversed"] == int(deg[ref >= 0].sum())
+            d, st = g.bfs(srcs, directed=directed, iter_num=1)
+            np.testing.assert_array_equal(d, np.where(ref <= 1, ref, -1))
+            assert st["edges_traversed"] == int(deg[(ref >= 0) & (ref <= 1)].sum())
+        if n >= 33:
+            with pytest.raises(mg.MapGraphError):
+                g.bfs(list(range(33)), queue_sizing=2 / n)
+            np.testing.assert_array_equal(g.bfs([0])[0], oracle.bfs(ro, ci, [0]))
