@@ -228,6 +228,13 @@ static mg::PrbArgs prb_args_of(const mg_graph *g, const mg::BinPlan &bp, bool cs
   return p;
 }
 
+mg_status graph_bin_plan(mg_graph *g, bool csr, mg::PrbArgs *out) {
+  mg::BinPlan *bp = nullptr;
+  MG_TRY(get_bin_plan(g, csr, &bp));
+  *out = prb_args_of(g, *bp, csr, nullptr);
+  return MG_OK;
+}
+
 namespace mg {
 
 // Per-row inputs of the row update.
@@ -427,7 +434,7 @@ __global__ void __launch_bounds__(PRB_NT, PRB_MIN_BLOCKS) solve_binned_kernel(So
     p.hcontrib[2 * h + 1] = hu.red2;
     __threadfence();
   };
-  prb_run<WEIGHTED>(p, [&](int32_t col) { return __ldg(gold + col); }, up, hub);
+  prb_run<WEIGHTED>(p, [&](int32_t col) { return col >= 0 ? __ldg(gold + col) : 0.f; }, up, hub);
   const double r = block_sum<PRB_NT>(up.resid, s_red);
   const double d = block_sum<PRB_NT>(up.red2, s_red);
   if (threadIdx.x == 0) {
@@ -474,6 +481,7 @@ __global__ void __launch_bounds__(PRB_HUB_NT, PRB_HUB_MINB) solve_binned_hub_ker
   for (int32_t i = threadIdx.x; i < nh4; i += PRB_HUB_NT)
     reinterpret_cast<float4 *>(s_hub)[i] = __ldcg(reinterpret_cast<const float4 *>(ghold) + i);
   for (int32_t i = 4 * nh4 + threadIdx.x; i < a.nhub; i += PRB_HUB_NT) s_hub[i] = __ldcg(ghold + i);
+  if (threadIdx.x == 0) s_hub[a.nhub] = 0.f;  // no column
   __syncthreads();
   const double scal = vload(&c->dprev[1]);
   RowUpdate up{&a, vold, vnew, gnew, scal};
@@ -486,7 +494,8 @@ __global__ void __launch_bounds__(PRB_HUB_NT, PRB_HUB_MINB) solve_binned_hub_ker
     p.hcontrib[2 * h + 1] = hu.red2;
     __threadfence();
   };
-  prb_run<WEIGHTED>(p, [&](int32_t col) { return col < 0 ? s_hub[col & 0x7fffffff] : __ldg(gold + col); }, up, hub);
+  prb_run<WEIGHTED>(
+      p, [&](int32_t col) { return col < 0 ? s_hub[min(col & 0x7fffffff, a.nhub)] : __ldg(gold + col); }, up, hub);
   const double r = block_sum<PRB_HUB_NT>(up.resid, s_red);
   const double d = block_sum<PRB_HUB_NT>(up.red2, s_red);
   if (threadIdx.x == 0) {
@@ -519,6 +528,7 @@ __global__ void __launch_bounds__(SEG_NT, 1) solve_segment_kernel(SolveArgs a, P
   if (threadIdx.x == 0) {
     mbar_init(&s_bar, 1);
     fence_barrier_init();
+    s_buf[sg.S] = 0.f;  // where padding reads; the block copies end before it
   }
   __syncthreads();
   auto fin = [&](const int2 &e, const Comp &acc) {
@@ -554,7 +564,9 @@ __global__ void __launch_bounds__(SEG_NT, 1) solve_rows_kernel(SolveArgs a, PrbA
   for (int32_t i = threadIdx.x; i < nh4; i += SEG_NT)
     reinterpret_cast<float4 *>(s_hub)[i] = __ldcg(reinterpret_cast<const float4 *>(ghold) + i);
   for (int32_t i = 4 * nh4 + threadIdx.x; i < a.nhub; i += SEG_NT) s_hub[i] = __ldcg(ghold + i);
+  if (threadIdx.x == 0) s_hub[a.nhub] = 0.f;  // no column (cached_gather)
   __syncthreads();
+  const uint32_t cache = cache_addr(s_hub), zero = 4u * (uint32_t)a.nhub;
   const double scal = vload(&c->dprev[1]);
   double resid = 0.0, red2 = 0.0;
   // Row update at position `pos` (row r): x' = alpha (acc + d t) + (1 - alpha) t,
@@ -599,7 +611,7 @@ __global__ void __launch_bounds__(SEG_NT, 1) solve_rows_kernel(SolveArgs a, PrbA
     const int32_t r = sg.rrow[pos];
     if (r >= 0) update(pos, r, Comp{0.f, 0.f});
   }
-  auto gather = [&](int32_t col) { return col < 0 ? s_hub[col & 0x7fffffff] : __ldg(gold + col); };
+  auto gather = [&](int32_t col) { return cached_gather(cache, zero, gold, col); };
   // Short groups (depth <= SEG_SHORT; rows of a few edges, most of the groups that
   // hold an edge): a fixed share per warp, two groups at a time with their loads
   // issued together, no counter and no header round trip in between.
@@ -705,7 +717,7 @@ struct RowSumStore {
 // Row sums s_u of the weighted CSR through the binned gather (unit gathered values).
 __global__ void __launch_bounds__(PRB_NT) rowsum_binned_kernel(PrbArgs p, float *s) {
   RowSumStore st{s};
-  prb_run<true>(p, [](int32_t) { return 1.0f; }, st, [&](int64_t, int32_t row, Comp v) { s[row] = v.hi + v.lo; });
+  prb_run<true>(p, [](int32_t c) { return c >= 0 ? 1.0f : 0.0f; }, st, [&](int64_t, int32_t row, Comp v) { s[row] = v.hi + v.lo; });
 }
 
 __global__ void __launch_bounds__(PRG_NT) solve_fixup_kernel(SolveArgs a) {
@@ -1263,8 +1275,9 @@ static mg_status solve_setup(mg_graph *g, bool adjoint, bool weighted, const flo
   sp.use_tma = use_tma;
   sp.use_hub = use_hub && !use_seg;
   sp.use_seg = use_seg;
-  sp.hub_bytes = use_hub ? (int32_t)(sizeof(float) * hubs->K) : 0;
-  sp.seg_bytes = use_seg ? (int32_t)(sizeof(float) * seg->S) : 0;
+  // the column cache and a column block, each with a zero behind it
+  sp.hub_bytes = use_hub ? (int32_t)(sizeof(float) * hubs->K + 16) : 0;
+  sp.seg_bytes = use_seg ? (int32_t)(sizeof(float) * seg->S + 16) : 0;
   sp.weighted = weighted;
   sp.gather = nullptr;
   if (use_tma) sp.gather = gather_variant(weighted, nr, &occ);
@@ -1494,7 +1507,7 @@ __global__ void __launch_bounds__(PRB_NT, PRR_MIN_BLOCKS) prr_sweep_kernel(RefAr
   int64_t insp = 0, nchg = 0, more = 0;
   bool any = false;
   auto gather = [&](int32_t u) {
-    const float t = __ldg(told + u);
+    const float t = u >= 0 ? __ldg(told + u) : 0.f;
     any |= __float_as_int(t) < 0;
     return fabsf(t);
   };
@@ -2153,12 +2166,12 @@ struct AdjRowStore {
 
 template <bool WEIGHTED>
 __global__ void __launch_bounds__(PRB_NT) adj_rows_kernel(PrbArgs p, const float *lam, AdjRowStore st) {
-  prb_run<WEIGHTED>(p, [&](int32_t c) { return __ldg(lam + c); }, st,
+  prb_run<WEIGHTED>(p, [&](int32_t c) { return c >= 0 ? __ldg(lam + c) : 0.f; }, st,
                     [&](int64_t, int32_t row, Comp v) { st(row, v); });
 }
 
 // dL/da_uv = coef[u] * (lambda_v - pl[u]) for every CSR edge, over the rows of the
-// bin plan: a lane takes 8 edges of its row at a time (16-byte index loads and, on
+// bin plan: a lane takes 8 edges of its row at a time (a 32-byte index load and, on
 // an aligned gradient array, 16-byte stores). The random lambda reads bound it; in
 // tiles of 256 consecutive vertices the few tiles with the hubs ran alone at the
 // end (R-MAT s22 directed, 67 M edges: 5.4 ms).
@@ -2170,23 +2183,17 @@ __global__ void __launch_bounds__(PRB_NT) adj_edge_grad_kernel(PrbArgs p, const 
   prb_walk(p, [&](auto lanes, int32_t row, int32_t b, int32_t e, int sub, int64_t, int64_t) {
     constexpr int L = decltype(lanes)::value > 0 ? decltype(lanes)::value : 1;
     const double cf = row >= 0 ? coef[row] : 0.0, mean = row >= 0 ? pl[row] : 0.0;
-    for (int32_t k0 = (b & ~3) + 4 * sub; k0 < e; k0 += 8 * L) {
-      const int32_t k1 = k0 + 4 * L;
-      int4 c[2];
-      c[0] = prb_stream(reinterpret_cast<const int4 *>(p.idx + k0));
-      c[1] = k1 < e ? prb_stream(reinterpret_cast<const int4 *>(p.idx + k1)) : make_int4(0, 0, 0, 0);
+    for (int32_t k0 = (b & ~7) + 8 * sub; k0 < e; k0 += 8 * L) {
+      int32_t c[8];
+      prb_load8(p.idx + k0, c);
       float x[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int32_t k = j < 4 ? k0 + j : k1 + j - 4;
-        const int4 &q = c[j >> 2];
-        x[j] = k >= b && k < e ? __ldg(lam + ((j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w)) : 0.f;
-      }
+      for (int j = 0; j < 8; j++) x[j] = k0 + j >= b && k0 + j < e ? __ldg(lam + c[j]) : 0.f;
 #pragma unroll
       for (int j = 0; j < 8; j++) x[j] = (float)(cf * ((double)x[j] - mean));
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const int32_t k = h ? k1 : k0;
+        const int32_t k = k0 + 4 * h;
         if (vec && k >= b && k + 3 < e) {
           __stcs(reinterpret_cast<float4 *>(grad + k), make_float4(x[4 * h], x[4 * h + 1], x[4 * h + 2], x[4 * h + 3]));
         } else {

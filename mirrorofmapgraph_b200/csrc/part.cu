@@ -276,7 +276,7 @@ struct PartPrRow {
 __global__ void __launch_bounds__(PRB_NT, PRB_MIN_BLOCKS) part_pr_kernel(PrbArgs p, const float *y, float *slice,
                                                                          double alpha, double tn, PartCtl *ctl) {
   const PartPrRow up{slice, alpha, tn, __ldcg(&ctl->dang)};
-  prb_run<false>(p, [&](int32_t col) { return __ldg(y + col); }, up,
+  prb_run<false>(p, [&](int32_t col) { return col >= 0 ? __ldg(y + col) : 0.f; }, up,
                  [&](int64_t, int32_t row, Comp v) { up(row, v); });
   if (last_block(&ctl->blocks_done) && threadIdx.x == 0) {
     *p.grab = 0;

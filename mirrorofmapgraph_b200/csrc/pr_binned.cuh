@@ -6,8 +6,8 @@
 //   bin 0       no edges: only the row update;
 //   bin 1       1 or 2 edges: one lane per row, plain loads;
 //   bins 2..9   up to 64 edges: one lane per row, classes narrow enough that the
-//               32 rows of a warp end together. A lane reads its row's indices as
-//               16-byte vectors and gathers 8 values before its first add, so a
+//               32 rows of a warp end together. A lane reads its row's indices a
+//               sector at a time and gathers 8 values before its first add, so a
 //               warp keeps up to 256 gathers in flight, with no shuffles;
 //   bin 10      65..256 edges: 4 lanes per row, 8 rows per warp;
 //   bin 11      up to PRB_HEAVY: one warp per row, 256 edges per step;
@@ -91,6 +91,11 @@ struct BinPlan {
 mg_status bin_plan_build(cudaStream_t s, const int32_t *off, int64_t n, mg::BinPlan &bp,
                          int32_t heavy = mg::PRB_HEAVY);
 void bin_plan_release(cudaStream_t s, mg::BinPlan &bp);
+namespace mg {
+struct PrbArgs;
+}
+// Arguments of the graph's cached plan of its CSC (or CSR) rows, without weights.
+mg_status graph_bin_plan(mg_graph *g, bool csr, mg::PrbArgs *out);
 
 namespace mg {
 
@@ -263,44 +268,73 @@ __device__ __forceinline__ void group_comp_reduce(Comp &c) {
   }
 }
 
+// 32 bytes of an index or weight stream (256-bit load, sm_100): read once, so not
+// kept in L1.
+__device__ __forceinline__ void prb_load8(const int32_t *p, int32_t (&c)[8]) {
+  asm("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7])
+      : "l"(p));
+}
+__device__ __forceinline__ void prb_load8(const float *p, float (&c)[8]) {
+  asm("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]), "=f"(c[4]), "=f"(c[5]), "=f"(c[6]), "=f"(c[7])
+      : "l"(p));
+}
+
+// Shared-memory address of a column cache that is complete: taken behind the barrier
+// that ends its filling, so that no gather through it moves ahead of that.
+__device__ __forceinline__ uint32_t cache_addr(const float *s) {
+  uint32_t a = smem_u32(s);
+  asm volatile("" : "+r"(a)::"memory");
+  return a;
+}
+
+// Value of column entry c with a shared-memory column cache: c < 0 is a cached
+// column's slot | 0x80000000, or -1 for no column, which reads the zero behind the
+// cache (`zero`: its byte offset from `cache`, a shared-memory address). One
+// predicated load either way, no branch.
+__device__ __forceinline__ float cached_gather(uint32_t cache, uint32_t zero, const float *__restrict__ g, int32_t c) {
+  float x;
+  asm("{\n\t.reg .pred h;\n\t.reg .u32 s;\n\t.reg .s64 a;\n\tsetp.lt.s32 h, %1, 0;\n\t"
+      "shl.b32 s, %1, 2;\n\tmin.u32 s, s, %3;\n\tadd.u32 s, s, %2;\n\tmad.wide.s32 a, %1, 4, %4;\n\t"
+      "@h ld.shared.f32 %0, [s];\n\t@!h ld.global.nc.f32 %0, [a];\n\t}"
+      : "=f"(x)
+      : "r"(c), "r"(cache), "r"(zero), "l"(g));
+  return x;
+}
+
 // Compensated sum of edges [b, e) by the L lanes of a group (sub: the lane's place
-// in it), 8 edges per lane and step: two 16-byte index loads (the lanes of a group
-// side by side) from the row's start rounded down to a vector, 8 gathers, then the
-// adds. Slots outside the row add +0, which a compensated sum does not notice; the
-// index and weight arrays are padded by 8 entries, so the last vector may run over
-// the row's (or the array's) end. Lanes of other groups may end earlier.
+// in it), 8 edges per lane and step: one 32-byte index load (the lanes of a group
+// side by side) from the row's start rounded down to a sector, 8 gathers, then the
+// adds. Slots outside the row gather column -1, which is 0, and +0 leaves a
+// compensated sum as it is. Index and weight arrays are padded by 8 entries, so the
+// last sector may run over the row's (or the array's) end. Lanes of other groups
+// may end earlier.
+//
+// A warp's load of 32 rows' sectors costs the L1 32 tag lookups, one per clock, like
+// a load of 32 random columns, and lookups bound this kernel: 32-byte loads make it
+// an eighth of a lookup per index against a quarter with 16-byte loads (weighted
+// R-MAT s22 iteration 380 us with those, 338 with these).
 template <int L, bool WEIGHTED, typename Gather>
 __device__ __forceinline__ Comp prb_group_range(const PrbArgs &p, int32_t b, int32_t e, int sub, Gather &gather) {
   Comp acc{0.f, 0.f};
-  for (int32_t k0 = (b & ~3) + 4 * sub; k0 < e; k0 += 8 * L) {
+  for (int32_t k0 = (b & ~7) + 8 * sub; k0 < e; k0 += 8 * L) {
     int32_t c[8];
-    float x[8];
-    float w[8];
-    const int32_t k1 = k0 + 4 * L;
-    const int4 i0 = prb_stream(reinterpret_cast<const int4 *>(p.idx + k0));
-    const int4 i1 = k1 < e ? prb_stream(reinterpret_cast<const int4 *>(p.idx + k1)) : make_int4(0, 0, 0, 0);
-    if (WEIGHTED) {
-      const float4 w0 = prb_stream(reinterpret_cast<const float4 *>(p.wts + k0));
-      const float4 w1 =
-          k1 < e ? prb_stream(reinterpret_cast<const float4 *>(p.wts + k1)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      w[0] = w0.x, w[1] = w0.y, w[2] = w0.z, w[3] = w0.w;
-      w[4] = w1.x, w[5] = w1.y, w[6] = w1.z, w[7] = w1.w;
-    }
-    c[0] = i0.x, c[1] = i0.y, c[2] = i0.z, c[3] = i0.w;
-    c[4] = i1.x, c[5] = i1.y, c[6] = i1.z, c[7] = i1.w;
+    float x[8], w[8];
+    prb_load8(p.idx + k0, c);
+    if (WEIGHTED) prb_load8(p.wts + k0, w);
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      const int32_t k = j < 4 ? k0 + j : k1 + j - 4;
-      x[j] = k >= b && k < e ? gather(c[j]) : 0.f;
+      const bool in = k0 + j >= b && k0 + j < e;
+      x[j] = gather(in ? c[j] : -1);
+      if (WEIGHTED) w[j] = in ? w[j] : 0.f;
     }
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       if (WEIGHTED) {
-        const int32_t k = j < 4 ? k0 + j : k1 + j - 4;
-        const float a = k >= b && k < e ? w[j] : 0.f;
-        const float pr = a * x[j];
+        const float pr = w[j] * x[j];
         two_sum_add(acc, pr);
-        acc.lo += __fmaf_rn(a, x[j], -pr);
+        acc.lo += __fmaf_rn(w[j], x[j], -pr);
       } else {
         two_sum_add(acc, x[j]);
       }
@@ -318,11 +352,11 @@ __device__ __forceinline__ Comp prb_short_range(const PrbArgs &p, int32_t b, int
   float x[2], w[2];
 #pragma unroll
   for (int j = 0; j < 2; j++) {
-    c[j] = b + j < e ? prb_stream(p.idx + b + j) : 0;
+    c[j] = b + j < e ? prb_stream(p.idx + b + j) : -1;
     w[j] = WEIGHTED && b + j < e ? prb_stream(p.wts + b + j) : 0.f;
   }
 #pragma unroll
-  for (int j = 0; j < 2; j++) x[j] = b + j < e ? gather(c[j]) : 0.f;
+  for (int j = 0; j < 2; j++) x[j] = gather(c[j]);
 #pragma unroll
   for (int j = 0; j < 2; j++) {
     if (WEIGHTED) {
@@ -426,7 +460,7 @@ __device__ __forceinline__ bool prb_hub_done(const PrbArgs &p, int64_t task, int
   return true;
 }
 
-// Sums every row of the plan: finish(row, Comp) consumes a row sum,
+// Sums every row of the plan, gather(-1) being 0: finish(row, Comp) consumes a row sum,
 // finish_hub(h, row, Comp) a hub's.
 template <bool WEIGHTED, typename Gather, typename Finish, typename FinishHub>
 __device__ __forceinline__ void prb_run(const PrbArgs &p, Gather &&gather, Finish &&finish, FinishHub &&finish_hub) {

@@ -312,7 +312,9 @@ __global__ void seg_pos_slot_kernel(const int32_t *__restrict__ prow, int64_t np
 
 // One lane's row of a sliced-ELL group (a phase-1 fragment or a phase-2 row):
 // `depth` steps from q (qw), index loads one round of U steps ahead of the
-// gathers; -1 entries are padding.
+// gathers; -1 entries are padding, for which gather returns 0 (and whose weight is
+// 0): adding +0 leaves a compensated sum as it is, and a step without a branch is
+// a third of the instructions.
 template <bool WEIGHTED, int U, typename Gather>
 __device__ __forceinline__ Comp sell_walk(const int32_t *q, const float *qw, int32_t depth, Gather &gather) {
   Comp acc{0.f, 0.f};
@@ -334,10 +336,9 @@ __device__ __forceinline__ Comp sell_walk(const int32_t *q, const float *qw, int
     }
     float v[U];
 #pragma unroll
-    for (int j = 0; j < U; j++) v[j] = c[j] != -1 ? gather(c[j]) : 0.f;
+    for (int j = 0; j < U; j++) v[j] = gather(c[j]);
 #pragma unroll
     for (int j = 0; j < U; j++) {
-      if (c[j] == -1) continue;
       if (WEIGHTED) {
         const float p = w[j] * v[j];
         two_sum_add(acc, p);
@@ -358,7 +359,8 @@ __device__ __forceinline__ Comp sell_walk(const int32_t *q, const float *qw, int
 // One lane's hub fragment (phase 1): `depth` (even) steps of 16-bit block offsets,
 // two per 32-bit word at q + 32 p (seg_pk), weights (weighted graphs) one per step
 // at qw + 32 i; index words loaded one round of U steps ahead of the gathers, the
-// sum taken in step order like sell_walk's. 0xFFFF entries are padding.
+// sum taken in step order like sell_walk's. 0xFFFF entries are padding: gather
+// returns 0 for them.
 template <bool WEIGHTED, int U, typename Gather>
 __device__ __forceinline__ Comp sell_walk16(const uint32_t *q, const float *qw, int32_t depth, Gather &gather) {
   static_assert(U % 2 == 0, "two steps per index word");
@@ -385,12 +387,10 @@ __device__ __forceinline__ Comp sell_walk16(const uint32_t *q, const float *qw, 
     float v[U];
 #pragma unroll
     for (int j = 0; j < U; j++) {
-      const uint32_t off = (c[j >> 1] >> (16 * (j & 1))) & 0xffffu;
-      v[j] = off != 0xffffu ? gather((int32_t)off) : 0.f;
+      v[j] = gather((c[j >> 1] >> (16 * (j & 1))) & 0xffffu);
     }
 #pragma unroll
     for (int j = 0; j < U; j++) {
-      if (((c[j >> 1] >> (16 * (j & 1))) & 0xffffu) == 0xffffu) continue;
       if (WEIGHTED) {
         const float pr = w[j] * v[j];
         two_sum_add(acc, pr);
@@ -426,30 +426,22 @@ __device__ __forceinline__ void sell_short2(const int32_t *qa, const float *qwa,
   }
 #pragma unroll
   for (int j = 0; j < SEG_SHORT; j++) {
-    va[j] = ca[j] != -1 ? gather(ca[j]) : 0.f;
-    vb[j] = cb[j] != -1 ? gather(cb[j]) : 0.f;
+    va[j] = gather(ca[j]);
+    vb[j] = gather(cb[j]);
   }
   acc_a = Comp{0.f, 0.f};
   acc_b = Comp{0.f, 0.f};
 #pragma unroll
   for (int j = 0; j < SEG_SHORT; j++) {
-    if (ca[j] != -1) {
-      if (WEIGHTED) {
-        const float p = wa[j] * va[j];
-        two_sum_add(acc_a, p);
-        acc_a.lo += __fmaf_rn(wa[j], va[j], -p);
-      } else {
-        two_sum_add(acc_a, va[j]);
-      }
-    }
-    if (cb[j] != -1) {
-      if (WEIGHTED) {
-        const float p = wb[j] * vb[j];
-        two_sum_add(acc_b, p);
-        acc_b.lo += __fmaf_rn(wb[j], vb[j], -p);
-      } else {
-        two_sum_add(acc_b, vb[j]);
-      }
+    if (WEIGHTED) {
+      const float pa = wa[j] * va[j], pb = wb[j] * vb[j];
+      two_sum_add(acc_a, pa);
+      acc_a.lo += __fmaf_rn(wa[j], va[j], -pa);
+      two_sum_add(acc_b, pb);
+      acc_b.lo += __fmaf_rn(wb[j], vb[j], -pb);
+    } else {
+      two_sum_add(acc_a, va[j]);
+      two_sum_add(acc_b, vb[j]);
     }
   }
 }
@@ -505,8 +497,9 @@ __device__ __forceinline__ void seg_phase(const SegArgs &sg, const float *gold, 
       phase ^= 1;
     }
     const float *gblk = gold + c_lo;
-    auto from_smem = [&](int32_t off) { return sbuf[off]; };
-    auto from_global = [&](int32_t off) { return __ldg(gblk + off); };
+    // sbuf[S] is 0 (set by the kernel): where a padding offset reads
+    auto from_smem = [&](uint32_t off) { return sbuf[min(off, (uint32_t)sg.S)]; };
+    auto from_global = [&](uint32_t off) { return off != 0xffffu ? __ldg(gblk + off) : 0.f; };
     for (;;) {
       int32_t gi = 0;
       if (lane == 0) gi = atomicAdd(next, 1);
