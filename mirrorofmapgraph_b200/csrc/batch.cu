@@ -29,13 +29,14 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "expand.cuh"
+#define MG_PRB_NO_PLAN_KERNELS
+#include "pr_binned.cuh"
 
 namespace mg {
 
 constexpr int MS_NT = 256;
 constexpr int MS_CTA_TH = 512;
 constexpr int MS_WIDTH = 64;        // sources per bit-parallel group
-constexpr int MS_PULL_SERIAL = 8;   // in-edges a lane scans alone before the warp helps
 constexpr int64_t MS_ALPHA = 14;    // bottom-up when the union frontier's out-edges exceed m / MS_ALPHA
 
 struct MsArgs {
@@ -49,6 +50,7 @@ struct MsArgs {
   int64_t n, m_total;
   uint64_t full;   // mask of the group's sources
   int32_t mode, can_pull, both;
+  int32_t *grab;   // work counters of the bottom-up passes (reset at the level's end)
   DevCtl *ctl;
   cudaGraphConditionalHandle h;
   int32_t use_cond;
@@ -66,6 +68,8 @@ __device__ void ms_level_end(const MsArgs &a) {
   c->mf_next = 0;
   c->blocks_done = 0;
   c->big_len = 0;
+  a.grab[0] = 0;
+  a.grab[1] = 0;
   const bool over = vload(&c->overflow) != 0;
   const bool done = nf == 0 || lvl >= c->iter_cap || over;
   int dir = 0;
@@ -159,12 +163,16 @@ __global__ void __launch_bounds__(MS_NT) ms_push_big_kernel(MsArgs a) {
   });
 }
 
-// Commits a top-down level: new bits = accumulated & ~seen; rewrites every
-// vertex's next-frontier mask and clears the accumulators it read.
+// Commits a level: new bits = accumulated & ~seen; rewrites every vertex's
+// next-frontier mask and clears the accumulators it read. In vertex order, so the
+// stores of a depth row are coalesced whichever way the level ran.
 __global__ void __launch_bounds__(MS_NT) ms_finish_kernel(MsArgs a) {
   __shared__ int64_t s_sum[MS_NT / 32 + 1];
-  if (ms_skip(a, 0)) return;
   DevCtl *c = a.ctl;
+  if (vload(&c->done)) {
+    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    return;
+  }
   const int cur = vload(&c->cur);
   const int32_t d = vload(&c->level) + 1;
   uint64_t *fnext = cur ? a.f0 : a.f1;
@@ -202,157 +210,64 @@ __global__ void __launch_bounds__(MS_NT) ms_finish_kernel(MsArgs a) {
   if (last_block(&c->blocks_done) && threadIdx.x == 0) ms_level_end(a);
 }
 
-// OR of the frontier masks over edges [beg, end) of one vertex per lane: each
-// lane first scans up to MS_PULL_SERIAL edges alone; vertices with more edges
-// still missing sources are then scanned by the whole warp, one at a time,
-// 32 edges per step, until every missing source has arrived.
-__device__ __forceinline__ uint64_t ms_gather(const int32_t *__restrict__ off, const int32_t *__restrict__ idx,
-                                              const uint64_t *__restrict__ fcur, bool need, int64_t v, uint64_t miss,
-                                              uint64_t acc, int64_t &insp) {
-  const int lane = lane_id();
-  int32_t beg = 0, end = 0;
-  if (need && (acc & miss) != miss) {
-    beg = off[v];
-    end = off[v + 1];
-  }
-  const int32_t lim = min(end, beg + MS_PULL_SERIAL);
-  for (int32_t e = beg; e < lim; e++) {
-    insp++;
-    acc |= __ldg(fcur + idx[e]);
-    if ((acc & miss) == miss) break;
-  }
-  unsigned pend = __ballot_sync(FULL, need && (acc & miss) != miss && lim < end);
-  while (pend) {
-    const int l = __ffs(pend) - 1;
-    pend &= pend - 1;
-    const int32_t b = __shfl_sync(FULL, lim, l), en = __shfl_sync(FULL, end, l);
-    const uint64_t m = __shfl_sync(FULL, miss, l);
-    uint64_t got = __shfl_sync(FULL, acc, l);
-    for (int32_t e0 = b; e0 < en; e0 += 32) {
-      const int32_t e = e0 + lane;
-      uint64_t x = 0;
-      if (e < en) {
-        x = __ldg(fcur + idx[e]);
-        insp++;
-      }
-      const unsigned lo = __reduce_or_sync(FULL, (unsigned)x), hi = __reduce_or_sync(FULL, (unsigned)(x >> 32));
-      got |= ((uint64_t)hi << 32) | lo;
-      if ((got & m) == m) break;
-    }
-    if (lane == l) acc = got;
-  }
-  return acc;
-}
-
-// Bottom-up level: every vertex still missing sources gathers its in-neighbours'
-// frontier masks; commits the new bits and rewrites the next-frontier masks.
-__global__ void __launch_bounds__(MS_NT) ms_pull_kernel(MsArgs a) {
+// Bottom-up pass: every vertex still missing sources ORs its in-neighbours'
+// frontier masks into its accumulator and stops once all of them have arrived.
+// Vertices come in the degree bins of the gather plan `p` (a lane each up to 64
+// in-edges, 8 index loads and 8 masks in flight per step; 4 lanes to 256; then a
+// warp; hubs in chunks, which add to the accumulator by atomics). In vertex order,
+// with a lane per vertex that calls its warp once it runs long, a few warps walked
+// neighbouring hubs one after another, two dependent loads per 32 edges: R-MAT s20,
+// 64 sources, 1.48 ms for the first bottom-up level, 0.12 ms with the bins. The
+// random mask reads bound it.
+// `second`: the out-edges' pass of an undirected run, on top of the first.
+__global__ void __launch_bounds__(MS_NT) ms_pull_kernel(MsArgs a, PrbArgs p, int second) {
   __shared__ int64_t s_sum[MS_NT / 32 + 1];
   if (ms_skip(a, 1)) return;
   DevCtl *c = a.ctl;
-  const int cur = vload(&c->cur);
-  const int32_t d = vload(&c->level) + 1;
-  const uint64_t *fcur = cur ? a.f1 : a.f0;
-  uint64_t *fnext = cur ? a.f0 : a.f1;
-  int32_t *qout = cur ? a.q0 : a.q1;
-  int32_t *qlen_out = &c->qlen[cur ^ 1];
-  int64_t mf = 0, vdeg = 0, insp = 0, nexp = 0;
-  const BigList big{a.big_v, &c->big_len};
-  const int64_t stride = (int64_t)gridDim.x * MS_NT;
-  for (int64_t base = (int64_t)blockIdx.x * MS_NT; base < a.n; base += stride) {
-    const int64_t v = base + threadIdx.x;
-    const bool in = v < a.n;
-    const uint64_t s = in ? a.seen[v] : a.full;
-    const uint64_t miss = a.full & ~s;
-    bool need = miss != 0;
-    nexp += need;
-    // In-degrees of GRID_TH and more go to the grid-strided bin (ms_pull_big_kernel).
-    if (need && !a.both && a.co[v + 1] - a.co[v] >= GRID_TH && defer_big(big, (int32_t)v, GRID_TH)) need = false;
-    uint64_t acc = ms_gather(a.co, a.ri, fcur, need, v, miss, 0, insp);
-    if (a.both) acc = ms_gather(a.ro, a.ci, fcur, need, v, miss, acc, insp);
-    const uint64_t nw = acc & miss;
-    if (in) {
-      if (nw) {
-        a.seen[v] = s | nw;
-        const int64_t deg = a.ro[v + 1] - a.ro[v];
-        mf += deg;
-        vdeg += deg * __popcll(nw);
-      }
-      fnext[v] = nw;
+  const uint64_t *__restrict__ fcur = vload(&c->cur) ? a.f1 : a.f0;
+  unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc);
+  int64_t insp = 0, nexp = 0;
+  prb_walk(p, [&](auto lanes, int32_t row, int32_t b, int32_t e, int sub, int64_t task, int64_t) {
+    constexpr int L = decltype(lanes)::value > 0 ? decltype(lanes)::value : 1;
+    uint64_t miss = 0;
+    if (row >= 0) {
+      miss = a.full & ~a.seen[row];
+      // bits an earlier chunk or pass has brought already
+      if (miss && (task >= 0 || second)) miss &= ~__ldcg(a.acc + row);
     }
-    ms_write_depths(a.depth, a.n, v, nw, d);
-    warp_append(nw != 0, (int32_t)v, qout, qlen_out, a.qcap, &c->overflow);
-  }
-  const int64_t bmf = block_sum<MS_NT>(mf, s_sum);
-  const int64_t bvd = block_sum<MS_NT>(vdeg, s_sum);
+    if (sub == 0 && miss && task < 0 && !second) nexp++;
+    if (!miss) e = b;
+    uint64_t got = 0;
+    for (int32_t k0 = (b & ~7) + 8 * sub; L == 32 ? k0 - 8 * sub < e : k0 < e; k0 += 8 * L) {
+      int32_t u[8];
+      uint64_t x[8];
+      if (k0 < e) prb_load8(p.idx + k0, u);
+#pragma unroll
+      for (int j = 0; j < 8; j++) x[j] = k0 + j >= b && k0 + j < e ? __ldg(fcur + u[j]) : 0ull;
+      insp += max(0, min(e, k0 + 8) - max(b, k0));
+#pragma unroll
+      for (int j = 0; j < 8; j++) got |= x[j];
+      if constexpr (L == 32) {
+        const unsigned lo = __reduce_or_sync(FULL, (unsigned)got), hi = __reduce_or_sync(FULL, (unsigned)(got >> 32));
+        got = ((uint64_t)hi << 32) | lo;
+      }
+      if ((got & miss) == miss) break;
+    }
+    if constexpr (L == 4) {
+      got |= __shfl_xor_sync(FULL, got, 1);
+      got |= __shfl_xor_sync(FULL, got, 2);
+    }
+    got &= miss;
+    if (sub == 0 && got) {
+      if (task >= 0) atomicOr(acc + row, (unsigned long long)got);
+      else a.acc[row] = second ? a.acc[row] | got : got;
+    }
+  });
   const int64_t bins = block_sum<MS_NT>(insp, s_sum);
   const int64_t bexp = block_sum<MS_NT>(nexp, s_sum);
   if (threadIdx.x == 0) {
-    if (bmf) atomicAdd((unsigned long long *)&c->mf_next, (unsigned long long)bmf);
-    if (bvd) atomicAdd((unsigned long long *)&c->visited_deg, (unsigned long long)bvd);
     if (bins) atomicAdd((unsigned long long *)&c->edges_inspected, (unsigned long long)bins);
     if (bexp) atomicAdd((unsigned long long *)&c->vertices_expanded, (unsigned long long)bexp);
-  }
-}
-
-// Grid-strided bin of a bottom-up level: every CTA ORs the frontier masks of an
-// equal slice of the deferred hubs' in-edges into their accumulators; the last
-// CTA commits the hubs' new bits and closes the level.
-__global__ void __launch_bounds__(MS_NT) ms_pull_big_kernel(MsArgs a) {
-  __shared__ BigSmem<MS_NT> sm;
-  __shared__ int64_t s_sum[MS_NT / 32 + 1];
-  if (ms_skip(a, 1)) return;
-  DevCtl *c = a.ctl;
-  const int cur = vload(&c->cur);
-  const uint64_t *fcur = cur ? a.f1 : a.f0;
-  const uint64_t *seen = a.seen;
-  unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc);
-  const int32_t *ri = a.ri;
-  const uint64_t full = a.full;
-  int64_t insp = 0;
-  expand_big<MS_NT>(sm, a.co, BigList{a.big_v, &c->big_len}, [&](int32_t v, int32_t k) {
-    insp++;
-    const uint64_t x = __ldg(fcur + ri[k]) & full & ~__ldg(seen + v);
-    if (x && (x & ~__ldcg(reinterpret_cast<const uint64_t *>(acc) + v))) atomicOr(acc + v, (unsigned long long)x);
-  });
-  const int64_t bins = block_sum<MS_NT>(insp, s_sum);
-  if (threadIdx.x == 0 && bins) atomicAdd((unsigned long long *)&c->edges_inspected, (unsigned long long)bins);
-  if (!last_block(&c->blocks_done)) return;
-  const int32_t d = vload(&c->level) + 1;
-  uint64_t *fnext = cur ? a.f0 : a.f1;
-  int32_t *qout = cur ? a.q0 : a.q1;
-  int32_t *qlen_out = &c->qlen[cur ^ 1];
-  const int32_t nb = min(vload(&c->big_len), BIG_CAP);
-  int64_t mf = 0, vdeg = 0;
-  for (int32_t i = threadIdx.x; i < nb; i += MS_NT) {
-    const int32_t v = a.big_v[i];
-    const uint64_t ac = __ldcg(a.acc + v);
-    a.acc[v] = 0;
-    const uint64_t s = a.seen[v];
-    uint64_t nw = ac & full & ~s;
-    fnext[v] = nw;
-    if (nw) {
-      a.seen[v] = s | nw;
-      const int64_t deg = a.ro[v + 1] - a.ro[v];
-      mf += deg;
-      vdeg += deg * __popcll(nw);
-      while (nw) {
-        const int j = __ffsll((long long)nw) - 1;
-        nw &= nw - 1;
-        a.depth[(int64_t)j * a.n + v] = d;
-      }
-      const int32_t pos = atomicAdd(qlen_out, 1);
-      if (pos < a.qcap) qout[pos] = v;
-      else c->overflow = 1;
-    }
-  }
-  const int64_t bmf = block_sum<MS_NT>(mf, s_sum);
-  const int64_t bvd = block_sum<MS_NT>(vdeg, s_sum);
-  if (threadIdx.x == 0) {
-    c->mf_next = vload(&c->mf_next) + bmf;
-    c->visited_deg = vload(&c->visited_deg) + bvd;
-    __threadfence();
-    ms_level_end(a);
   }
 }
 
@@ -424,7 +339,8 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
   const size_t need = Carve::need({sizeof(uint64_t) * (size_t)n, sizeof(uint64_t) * (size_t)n,
                                    sizeof(uint64_t) * (size_t)n, sizeof(uint64_t) * (size_t)n,
                                    sizeof(int32_t) * (size_t)n, sizeof(int32_t) * (size_t)n,
-                                   sizeof(int32_t) * (size_t)BIG_CAP, sizeof(int32_t) * (size_t)nsrc});
+                                   sizeof(int32_t) * (size_t)BIG_CAP, sizeof(int32_t) * (size_t)nsrc,
+                                   sizeof(int32_t) * 2});
   MG_TRY(ws_reserve(g, g->ws_main, need));
   Carve cv(g->ws_main.ptr);
   MsArgs a;
@@ -437,6 +353,7 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
   a.q1 = cv.take<int32_t>(n);
   a.big_v = cv.take<int32_t>(BIG_CAP);
   int32_t *dsrc = cv.take<int32_t>(nsrc);
+  a.grab = cv.take<int32_t>(2);
   a.qcap = (int32_t)n;
   a.ro = g->ro;
   a.ci = g->ci;
@@ -447,11 +364,25 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
   a.mode = o.direction;
   a.can_pull = g->has_csc || symmetric;
   a.both = undirected ? 1 : 0;
+  // bottom-up levels walk the gather plan of the in-edges (then of the out-edges)
+  const bool pull = a.can_pull && o.direction != MG_DIR_PUSH;
+  PrbArgs pin, pout;
+  std::memset(&pin, 0, sizeof(pin));
+  std::memset(&pout, 0, sizeof(pout));
+  if (pull) {
+    MG_TRY(graph_bin_plan(g, !g->has_csc, &pin));
+    pin.grab = a.grab;
+    if (undirected) {
+      MG_TRY(graph_bin_plan(g, true, &pout));
+      pout.grab = a.grab + 1;
+    }
+  }
   a.ctl = g->ctl;
   cudaStream_t s = g->stream;
   const int32_t iter_cap = o.iter_num > 0 ? (int32_t)std::min<int64_t>(o.iter_num, n + 1) : (int32_t)(n + 1);
   const int32_t dir0 = (o.direction == MG_DIR_PULL && a.can_pull) ? 1 : 0;
   MG_CUDA_TRY(cudaMemcpyAsync(dsrc, srcs, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, s));
+  MG_CUDA_TRY(cudaMemsetAsync(a.grab, 0, sizeof(int32_t) * 2, s));
   const int grid = g->num_sms * 4;
   const bool use_graph = o.use_graph >= 0;
   int64_t iters = 0, vdeg = 0, insp = 0, launches = 0, pulls = 0;
@@ -467,20 +398,23 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
     MG_CUDA_TRY(cudaGetLastError());
     struct Sig {
       MsArgs a;
+      PrbArgs pin, pout;
       int grid;
     } sig;
     std::memset(&sig, 0, sizeof(sig));
     sig.a = a;
+    sig.pin = pin;
+    sig.pout = pout;
     sig.grid = grid;
-    LoopBody body = [a, grid](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) {
+    LoopBody body = [a, pin, pout, pull, grid](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) {
       MsArgs b = a;
       b.h = h;
       b.use_cond = use_cond;
       ms_push_kernel<<<grid, MS_NT, 0, st>>>(b);
       ms_push_big_kernel<<<grid, MS_NT, 0, st>>>(b);
+      if (pull) ms_pull_kernel<<<grid, MS_NT, 0, st>>>(b, pin, 0);
+      if (pull && b.both) ms_pull_kernel<<<grid, MS_NT, 0, st>>>(b, pout, 1);
       ms_finish_kernel<<<grid, MS_NT, 0, st>>>(b);
-      ms_pull_kernel<<<grid, MS_NT, 0, st>>>(b);
-      ms_pull_big_kernel<<<grid, MS_NT, 0, st>>>(b);
     };
     MG_TRY(run_loop(g, SLOT_MSBFS, &sig, sizeof(sig), use_graph, body, n + 2));
     MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
@@ -497,7 +431,8 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
     vdeg += hc.visited_deg;
     insp += hc.edges_inspected;
     pulls += hc.levels_pull;
-    launches += 2 + (use_graph ? 6 * (int64_t)hc.body_iters : 5 * (int64_t)hc.level);
+    const int64_t per = 3 + (pull ? 1 + a.both : 0);
+    launches += 2 + (use_graph ? (per + 1) * (int64_t)hc.body_iters : per * (int64_t)hc.level);
   }
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
