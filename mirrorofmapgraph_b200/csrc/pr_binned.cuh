@@ -45,19 +45,25 @@ __host__ __device__ constexpr int prb_rows_per(int bin) { return bin < PRB_QUAD 
 #ifndef PRB_MIN_BLOCKS
 #define PRB_MIN_BLOCKS 5
 #endif
-// Index (and weight) streams are read once per iteration: loads marked
-// evict-first (ld.global.cs) keep them from displacing the gathered vector in
-// L1 and L2. PRB_STREAM_LOADS=0 uses plain read-only loads instead.
+// Index (and weight) streams are read once per iteration: they do not displace the
+// gathered vector in L1.
 #ifndef PRB_STREAM_LOADS
 #define PRB_STREAM_LOADS 1
 #endif
-template <typename T>
-__device__ __forceinline__ T prb_stream(const T *p) {
+__device__ __forceinline__ int32_t prb_stream(const int32_t *p) {
 #if PRB_STREAM_LOADS
-  return __ldcs(p);
+  int32_t v;
+  asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
 #else
-  return __ldg(p);
+  return __ldcs(p);
 #endif
+}
+__device__ __forceinline__ uint32_t prb_stream(const uint32_t *p) {
+  return (uint32_t)prb_stream(reinterpret_cast<const int32_t *>(p));
+}
+__device__ __forceinline__ float prb_stream(const float *p) {
+  return __int_as_float(prb_stream(reinterpret_cast<const int32_t *>(p)));
 }
 #ifndef PRB_HEAVY_EDGES
 #define PRB_HEAVY_EDGES 2048
