@@ -206,7 +206,9 @@ __device__ void ppr_iteration_end(const PprArgs &a, int cur, double *s_max) {
 }
 
 // One iteration for every column of the group. Warp items: hub chunks first (the
-// longest items start first), then the non-hub rows; each warp takes the next
+// longest items start first), then the non-hub rows from the plan's longest class to
+// its rows without edges (lightest first left the longest rows alone at the end:
+// R-MAT s20, 256 vectors, 5.15 ms an iteration against 5.00); each warp takes the next
 // item from a shared counter, so faster SMs take more.
 template <int VPL, bool WEIGHTED>
 __global__ void __launch_bounds__(PPR_NT) ppr_iter_kernel(PprArgs a) {
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__(PPR_NT) ppr_iter_kernel(PprArgs a) {
 #pragma unroll
     for (int j = 0; j < VPL; j++) acc[j] = Comp{0.f, 0.f};
     if (it >= a.nchunks) {
-      const int32_t row = a.rows[it - a.nchunks];
+      const int32_t row = a.rows[a.nlight - 1 - (it - a.nchunks)];  // longest rows first
       ppr_gather<VPL, WEIGHTED>(a, go, __ldg(a.off + row), __ldg(a.off + row + 1), acc);
       ppr_update<VPL>(a, row, acc, xo, xn, gn, dj, rs, ds);
       return;
