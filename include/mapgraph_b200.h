@@ -78,8 +78,10 @@ typedef struct mg_opts {
   double queue_sizing;   /* frontier capacity = queue_sizing * n (reference "max_queue_sizing");
                             <= 0 means n, which cannot overflow */
   int32_t threshold;     /* reference "threshold": accepted for compatibility; strategy is chosen on the device */
-  int32_t use_graph;     /* 1 (default when 0): run the iteration loop as a CUDA graph with a device-side while node;
-                            -1: host-driven loop (one frontier-size read per iteration) */
+  int32_t use_graph;     /* 1: run the iteration loop as a CUDA graph with a device-side while node; 0 (default): the
+                            same for traversals, while PageRank iterations are queued ahead of the device, which
+                            reports each end to pinned host memory; -1: host-driven loop (one frontier-size read
+                            per iteration) */
   int32_t delta;         /* SSSP only (int32 weights, iter_num unbounded): > 0 runs the near-far schedule with
                             this bucket width; 0 (default) chooses near-far with 8 x the mean weight on sparse
                             graphs (mean out-degree <= 8) and plain frontier Bellman-Ford otherwise; < 0 always

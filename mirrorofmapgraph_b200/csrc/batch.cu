@@ -81,13 +81,13 @@ __device__ void ms_level_end(const MsArgs &a) {
   if (over) c->status = MG_ERR_QUEUE_OVERFLOW;
   __threadfence();
   c->done = done ? 1 : 0;
-  if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+  loop_signal(a.ctl, a.h, a.use_cond, done);
 }
 
 __device__ __forceinline__ bool ms_skip(const MsArgs &a, int want_dir) {
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return true;
   }
   return vload(&c->dir) != want_dir;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(MS_NT) ms_finish_kernel(MsArgs a) {
   __shared__ int64_t s_sum[MS_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
@@ -384,7 +384,6 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
   MG_CUDA_TRY(cudaMemcpyAsync(dsrc, srcs, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, s));
   MG_CUDA_TRY(cudaMemsetAsync(a.grab, 0, sizeof(int32_t) * 2, s));
   const int grid = g->num_sms * 4;
-  const bool use_graph = o.use_graph >= 0;
   int64_t iters = 0, vdeg = 0, insp = 0, launches = 0, pulls = 0;
   float ms_total = 0.f;
   for (int32_t g0 = 0; g0 < nsrc; g0 += MS_WIDTH) {
@@ -416,7 +415,7 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
       if (pull && b.both) ms_pull_kernel<<<grid, MS_NT, 0, st>>>(b, pout, 1);
       ms_finish_kernel<<<grid, MS_NT, 0, st>>>(b);
     };
-    MG_TRY(run_loop(g, SLOT_MSBFS, &sig, sizeof(sig), use_graph, body, n + 2));
+    MG_TRY(run_loop(g, SLOT_MSBFS, &sig, sizeof(sig), o.use_graph, body, n + 2));
     MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
     MG_TRY(fetch_ctl(g));
     const DevCtl &hc = *g->ctl_host;
@@ -432,7 +431,7 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
     insp += hc.edges_inspected;
     pulls += hc.levels_pull;
     const int64_t per = 3 + (pull ? 1 + a.both : 0);
-    launches += 2 + (use_graph ? (per + 1) * (int64_t)hc.body_iters : per * (int64_t)hc.level);
+    launches += 2 + loop_launches(g, per);
   }
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));

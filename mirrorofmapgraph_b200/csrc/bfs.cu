@@ -846,7 +846,7 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
       bfs_push_big_kernel<<<grid, BFS_NT, 0, st>>>(b);
       bfs_pull_kernel<<<grid, BFS_NT, 0, st>>>(b);
     };
-    MG_TRY(run_loop(g, SLOT_BFS, &sig, sizeof(sig), use_graph, body, n + 2));
+    MG_TRY(run_loop(g, SLOT_BFS, &sig, sizeof(sig), o.use_graph, body, n + 2));
   }
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
   if (!o.device_output) MG_TRY(copy_out(g, depth, label, sizeof(int32_t) * n, 0));
@@ -864,7 +864,7 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
     stats->kernel_ms = ms;
     stats->status_detail = hc.levels_pull;
     const int64_t per = 3 + (tail ? 1 : 0);
-    stats->launches = small ? 1 : 2 + persist_launches + (use_graph ? (per + 1) * (int64_t)hc.body_iters : per * g->host_iters);
+    stats->launches = small ? 1 : 2 + persist_launches + loop_launches(g, per);
   }
   if (hc.status == MG_ERR_TIMEOUT) {
     mg_set_error("mg_bfs: a grid barrier of the persistent levels timed out");
@@ -1029,7 +1029,7 @@ extern "C" mg_status mg_bfs_noalloc(mg_graph *g, const int32_t *srcs, int32_t ns
     bfs_push_big_kernel<<<grid, BFS_NT, 0, st>>>(a);
     bfs_pull_kernel<<<grid, BFS_NT, 0, st>>>(a);
   };
-  MG_TRY(run_loop(g, SLOT_BFS, nullptr, 0, false, body, n + 2));
+  MG_TRY(run_loop(g, SLOT_BFS, nullptr, 0, -1, body, n + 2));
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
   MG_TRY(fetch_ctl(g));
   const DevCtl &hc = *g->ctl_host;

@@ -782,6 +782,10 @@ static mg_status create_impl(const int32_t *row_offsets, const int32_t *col_idx,
     mg_set_error("mg_graph_create: pinned host allocation failed");
     return fail(MG_ERR_OOM);
   }
+  {
+    unsigned long long *box = const_cast<unsigned long long *>(graph_mailbox(g));
+    CREATE_TRY(cudaMemcpyAsync(loop_mailbox(g->ctl), &box, sizeof(box), cudaMemcpyHostToDevice, s));
+  }
   CREATE_TRY(cudaEventCreate(&g->ev0));
   CREATE_TRY(cudaEventCreate(&g->ev1));
   // Validate on the device.

@@ -80,6 +80,8 @@ struct DevCtl {
   int32_t sc[3];
   int32_t smin[3];
   int64_t se[3];
+  uint32_t reports;  // iterations reported to the host (engine.cuh, launches ahead)
+  uint32_t pad;
 };
 
 // Padding of the device graph arrays. Offsets arrays hold n + 1 + MG_OFF_PAD
@@ -149,7 +151,7 @@ struct mg_graph {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   void *cache = nullptr;       // cached executable loop graphs (engine.cu)
   mg_tuning tune = tuning_defaults();  // traversal thresholds and launch shapes (mg_graph_set_tuning)
-  int64_t host_iters = 0;              // body calls of the last host-driven loop (run_loop)
+  int64_t host_iters = 0;              // body calls of the last loop the host launched (0: a graph; run_loop)
 };
 
 // Every device allocation of the library goes through here: cudaMallocAsync on
@@ -189,6 +191,18 @@ __device__ inline void trace_level(DevCtl *c, int32_t level, int32_t dir, int64_
   r.time_ns = t;
   trace_of(c)[level] = r;
   if (level + 1 > c->trace_len) c->trace_len = level + 1;
+}
+
+// The word of pinned host memory that the device reports a run's progress in
+// (engine.cuh): behind the pinned mirror of the control block, its address behind
+// the control block, past the spare bytes that the checks use.
+constexpr size_t MG_MAIL_OFF = sizeof(DevCtl) + 32;
+static_assert(MG_MAIL_OFF % 8 == 0, "the mailbox address is an aligned word");
+__host__ __device__ inline unsigned long long **loop_mailbox(DevCtl *c) {
+  return reinterpret_cast<unsigned long long **>(reinterpret_cast<char *>(c) + MG_MAIL_OFF);
+}
+inline volatile unsigned long long *graph_mailbox(mg_graph *g) {
+  return reinterpret_cast<volatile unsigned long long *>(reinterpret_cast<char *>(g->ctl_host) + MG_MAIL_OFF);
 }
 
 // Grows a workspace to at least `bytes` (contents are not preserved).

@@ -337,7 +337,7 @@ struct RowUpdate {
 
 __device__ __forceinline__ bool solve_skip(const SolveArgs &a) {
   if (vload(&a.ctl->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return true;
   }
   return false;
@@ -411,7 +411,7 @@ __device__ void solve_iteration_end(const SolveArgs &a, int cur, const double *h
     const bool done = r < thr || lvl >= a.max_iter || c->status != 0;
     __threadfence();
     c->done = done ? 1 : 0;
-    if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+    loop_signal(a.ctl, a.h, a.use_cond, done);
   }
 }
 
@@ -1456,7 +1456,7 @@ static mg_status solve_run(mg_graph *g, SolvePlan &sp, int use_graph, int slot) 
       solve_binned_kernel<false><<<g1, PRB_NT, 0, st>>>(b, p);
     }
   };
-  MG_TRY(run_loop(g, slot, &sig, sizeof(sig), use_graph >= 0, body, (int64_t)a.max_iter + 2));
+  MG_TRY(run_loop(g, slot, &sig, sizeof(sig), use_graph, body, (int64_t)a.max_iter + 2, true));
   return MG_OK;
 }
 
@@ -1496,7 +1496,7 @@ __global__ void __launch_bounds__(PRB_NT, PRR_MIN_BLOCKS) prr_sweep_kernel(RefAr
   __shared__ int64_t s_sum[PRB_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const PrbArgs &p = PASS == 2 ? a.second : a.first;
@@ -1597,7 +1597,7 @@ __global__ void __launch_bounds__(PRB_NT, PRR_MIN_BLOCKS) prr_sweep_kernel(RefAr
     const bool done = none || lvl >= c->iter_cap;
     __threadfence();
     c->done = done ? 1 : 0;
-    if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+    loop_signal(a.ctl, a.h, a.use_cond, done);
   }
 }
 
@@ -1683,7 +1683,7 @@ static mg_status pagerank_refcompat(mg_graph *g, float *ranks, const mg_pr_opts 
       prr_sweep_kernel<0><<<grid, PRB_NT, 0, st>>>(b);
     }
   };
-  MG_TRY(run_loop(g, SLOT_PR_REF, &sig, sizeof(sig), o.use_graph >= 0, body, (int64_t)cap + 2));
+  MG_TRY(run_loop(g, SLOT_PR_REF, &sig, sizeof(sig), o.use_graph, body, (int64_t)cap + 2, true));
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
   if (!o.device_output) MG_TRY(copy_out(g, ranks, a.x, sizeof(float) * n, 0));
   MG_TRY(fetch_ctl(g));
@@ -1698,7 +1698,7 @@ static mg_status pagerank_refcompat(mg_graph *g, float *ranks, const mg_pr_opts 
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     stats->kernel_ms = ms;
     const int64_t per_it = split ? 2 : 1;
-    stats->launches = 1 + (o.use_graph >= 0 ? (per_it + 1) * (int64_t)hc.body_iters : per_it * (int64_t)hc.level);
+    stats->launches = 1 + loop_launches(g, per_it);
   }
   if (hc.status != 0) {
     mg_set_error("mg_pagerank: device status %d", hc.status);
@@ -1844,7 +1844,7 @@ static mg_status pagerank_normalized(mg_graph *g, const float *tele_dev, float *
     stats->status_detail = (sp.use_hub || sp.use_seg) ? sp.a.nhub : 0;
     stats->variant = variant;
     stats->launches = 4 + ((sp.use_hub || sp.use_seg) ? 1 : 0) +
-                      (o.use_graph >= 0 ? (per_it + 1) * (int64_t)hc.body_iters : per_it * (int64_t)hc.level);
+                      loop_launches(g, per_it);
   }
   return MG_OK;
 }
@@ -2025,7 +2025,7 @@ static mg_status pagerank_ppr(mg_graph *g, const float *tele_dev, int32_t nvec, 
         default: ppr_launch_iter<8, true>(b, st); break;
       }
     };
-    MG_TRY(run_loop(g, SLOT_PPR, &sig, sizeof(sig), o.use_graph >= 0, body, (int64_t)a.max_iter + 2));
+    MG_TRY(run_loop(g, SLOT_PPR, &sig, sizeof(sig), o.use_graph, body, (int64_t)a.max_iter + 2, true));
     MG_TRY(fetch_ctl(g));
     const DevCtl &hc = *g->ctl_host;
     const float *res = hc.cur ? a.x1 : a.x0;
@@ -2052,7 +2052,7 @@ static mg_status pagerank_ppr(mg_graph *g, const float *tele_dev, int32_t nvec, 
     // and x read, x, g written and t read per vertex
     total.bytes_compulsory += hc.level * (4 * (n + 1) + (weighted ? 8 : 4) * g->m + (int64_t)4 * W * g->m +
                                           (int64_t)16 * W * n);
-    total.launches += 5 + (o.use_graph >= 0 ? 2 * (int64_t)hc.body_iters : (int64_t)hc.level);
+    total.launches += 5 + loop_launches(g, 1);
   }
   if (stats) *stats = total;
   return MG_OK;
@@ -2341,7 +2341,7 @@ extern "C" mg_status mg_pagerank_backward(mg_graph *g, const float *teleport, co
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     stats->kernel_ms = ms;
-    stats->launches = 4 + launches + (o.use_graph >= 0 ? 2 * (int64_t)hc.body_iters : (int64_t)hc.level);
+    stats->launches = 4 + launches + loop_launches(g, 1);
   }
   if (hc.status != 0) {
     mg_set_error("mg_pagerank_backward: device status %d", hc.status);

@@ -201,7 +201,7 @@ __device__ void ppr_iteration_end(const PprArgs &a, int cur, double *s_max) {
     const bool done = s_max[0] < a.tol || lvl >= a.max_iter || c->status != 0;
     __threadfence();
     c->done = done ? 1 : 0;
-    if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+    loop_signal(a.ctl, a.h, a.use_cond, done);
   }
 }
 
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(PPR_NT) ppr_iter_kernel(PprArgs a) {
   __shared__ int s_last;
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);

@@ -1266,7 +1266,7 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
     cudaGetLastError();
   }
   if (!persist)
-    MG_TRY(run_loop(g, vmask == -1 ? SLOT_SSSP : SLOT_BSSSP, &sig, sizeof(sig), o.use_graph >= 0, body,
+    MG_TRY(run_loop(g, vmask == -1 ? SLOT_SSSP : SLOT_BSSSP, &sig, sizeof(sig), o.use_graph, body,
                     (int64_t)iter_cap + 2));
   sssp_reach_kernel<<<g->num_sms * 4, 256, 0, s>>>(dist, nitems, vmask, g->ro, g->ctl);
   MG_CUDA_TRY(cudaGetLastError());
@@ -1283,9 +1283,7 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     stats->kernel_ms = ms;
     const int64_t per = a.delta > 0 ? 4 : 3;
-    stats->launches = 3 + (persist             ? 1
-                           : o.use_graph >= 0 ? (per + 1) * (int64_t)hc.body_iters
-                                              : per * (int64_t)hc.level);
+    stats->launches = 3 + (persist ? 1 : loop_launches(g, per));
     stats->status_detail = a.delta > 0 ? a.delta : 0;
   }
   if (hc.status == MG_ERR_TIMEOUT) {
@@ -1406,7 +1404,7 @@ static mg_status msssp_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
     mss_chunk_kernel<<<grid, SSSP_NT, 0, st>>>(b);
     mss_compact_kernel<<<cgrid, SSSP_NT, 0, st>>>(b, rows);
   };
-  MG_TRY(run_loop(g, SLOT_MSSSP, &sig, sizeof(sig), o.use_graph >= 0, body, n + 3));
+  MG_TRY(run_loop(g, SLOT_MSSSP, &sig, sizeof(sig), o.use_graph, body, n + 3));
   mss_unpack_kernel<<<g->num_sms * 2, 1024, 0, s>>>(a, dist, nsrc, groups);
   MG_CUDA_TRY(cudaGetLastError());
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
@@ -1424,7 +1422,7 @@ static mg_status msssp_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     stats->kernel_ms = ms;
-    stats->launches = 3 + (o.use_graph >= 0 ? 4 * (int64_t)hc.body_iters : 3 * (int64_t)hc.level);
+    stats->launches = 3 + loop_launches(g, 3);
   }
   if (hc.status != 0) {
     mg_set_error("mg_sssp_batch: device status %d", hc.status);

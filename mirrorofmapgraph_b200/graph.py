@@ -53,6 +53,11 @@ def _len(x) -> int:
     return int(x.numel()) if _is_torch(x) else int(np.asarray(x).size)
 
 
+def _loop_mode(use_graph) -> int:
+    """mg_opts.use_graph of True (the program's default), "graph" (a CUDA graph per run) or False (host-driven)."""
+    return -1 if not use_graph else 1 if use_graph == "graph" else 0
+
+
 def _opts(directed=1, iter_num=0, direction="auto", device_output=False, queue_sizing=0.0, threshold=0,
           use_graph=True, delta=0) -> L.MgOpts:
     o = L.MgOpts()
@@ -62,7 +67,7 @@ def _opts(directed=1, iter_num=0, direction="auto", device_output=False, queue_s
     o.device_output = int(device_output)
     o.queue_sizing = float(queue_sizing)
     o.threshold = int(threshold)
-    o.use_graph = 0 if use_graph else -1
+    o.use_graph = _loop_mode(use_graph)
     o.delta = int(delta)
     return o
 
@@ -330,7 +335,7 @@ class Graph:
         o.tol = 0.0 if tol is None else float(tol)
         o.compensated = 1 if compensated else -1
         o.device_output = int(device_output)
-        o.use_graph = 0 if use_graph else -1
+        o.use_graph = _loop_mode(use_graph)
         return o
 
     def pagerank(self, teleport=None, nvec: int = 1, out=None, **kw):

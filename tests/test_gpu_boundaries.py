@@ -193,3 +193,23 @@ def test_small_bfs(n, m, directed):
             with pytest.raises(mg.MapGraphError):
                 g.bfs(list(range(33)), queue_sizing=2 / n)
             np.testing.assert_array_equal(g.bfs([0])[0], oracle.bfs(ro, ci, [0]))
+
+
+def test_loop_modes_agree():
+    """Launches ahead of the device (the default), the CUDA-graph loop and the host-driven one."""
+    h = mg.gen_rmat(17, 16, 9, symmetrize=True, weights="int", p0=1, p1=255)
+    modes = (True, "graph", False)
+    with mg.Graph(h.row_offsets, h.col_idx, h.weights_i32, symmetric=True) as g:
+        runs = [(g.bfs([5], use_graph=m), g.sssp([5], use_graph=m), g.sssp([5], delta=20, use_graph=m),
+                 g.bfs_batch([5, 9, 70000], use_graph=m), g.sssp_batch([5, 9], use_graph=m),
+                 g.bfs([5], iter_num=2, use_graph=m)) for m in modes]
+        for other in runs[1:]:
+            for (a, sa), (b, sb) in zip(runs[0], other):
+                np.testing.assert_array_equal(a, b)
+                assert sa["edges_traversed"] == sb["edges_traversed"]
+        for kw in (dict(mode="refcompat"), dict(mode="normalized"), dict(mode="normalized", gather="segmented"),
+                   dict(mode="normalized", gather="tma"), dict(mode="normalized", max_iter=1)):
+            res = [g.pagerank(use_graph=m, **kw) for m in modes]
+            assert len({r[1]["iterations"] for r in res}) == 1
+            for r in res[1:]:
+                assert np.abs(r[0] - res[0][0]).sum() <= 1e-9 * max(1.0, float(np.abs(res[0][0]).sum()))
