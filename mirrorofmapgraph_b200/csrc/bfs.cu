@@ -19,7 +19,10 @@
 //  pull (bottom-up) every unvisited vertex scans its in-edges for a parent whose
 //                   depth equals the current level and stops at the first hit.
 //                   A warp owns 32 consecutive vertices, i.e. one bitmap word,
-//                   so visited words are updated without atomics.
+//                   so visited words are updated without atomics. An in-neighbour
+//                   of an unvisited vertex that is visited at all was reached in
+//                   the last level, so the test is one bit of the bitmap as the
+//                   level found it (the level writes a second one).
 //
 // The direction switch (Beamer's heuristic: go bottom-up when the frontier's
 // out-edges exceed 1/14 of the unexplored edges, back when the frontier drops
@@ -36,12 +39,15 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "expand.cuh"
+#define MG_PRB_NO_PLAN_KERNELS
+#include "pr_binned.cuh"
 
 namespace mg {
 
 constexpr int BFS_NT = 256;
 constexpr int BFS_CTA_TH = 512;   // out-degree at or above which a CTA expands the vertex
-constexpr int PULL_SERIAL = 8;    // in-edges a lane scans alone before the warp helps
+constexpr int PULL_SERIAL = 8;    // in-edges a lane scans alone before others help
+constexpr int PULL_QUAD = 256;    // in-edges four lanes scan before the whole warp does
 // Beamer's direction rule (mg_tuning.bfs_alpha / bfs_beta, defaults 14 and 24):
 // pull when the frontier's out-edges exceed the unvisited vertices' out-edges /
 // alpha, back to push when the frontier holds fewer than n / beta vertices. AUTO
@@ -51,7 +57,7 @@ struct BfsArgs {
   const int32_t *ro, *ci;  // out-edges (CSR)
   const int32_t *co, *ri;  // in-edges (CSC; the CSR itself for symmetric graphs)
   int32_t *label;
-  uint32_t *vis;
+  uint32_t *vis, *vis2;  // visited bitmaps, current by DevCtl::vsel (vis2 nullptr: only vis, updated in place)
   int32_t *q0, *q1;
   int32_t qcap;
   int32_t mode;      // MG_DIR_*
@@ -103,6 +109,7 @@ __device__ void bfs_level_end(const BfsArgs &a) {
   const int lvl = vload(&c->level) + 1;
   trace_level(c, lvl - 1, vload(&c->dir) == 1 ? MG_DIR_PULL : MG_DIR_PUSH, vload(&c->qlen[cur]),
               vload(&c->mf_front), 0.0);
+  if (vload(&c->dir) == 1 && a.vis2) c->vsel ^= 1;  // the level wrote the other bitmap
   c->visited_deg = vdeg;
   c->mf_front = mf;
   c->level = lvl;
@@ -137,7 +144,7 @@ __device__ void bfs_level_end(const BfsArgs &a) {
   if (over) c->status = MG_ERR_QUEUE_OVERFLOW;
   __threadfence();
   c->done = done ? 1 : 0;
-  if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+  loop_signal(a.ctl, a.h, a.use_cond, done);
 }
 
 // Early exit shared by both kernels: when the run is already over, make sure
@@ -145,11 +152,13 @@ __device__ void bfs_level_end(const BfsArgs &a) {
 __device__ __forceinline__ bool bfs_skip(const BfsArgs &a, int want_dir) {
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return true;
   }
   return vload(&c->dir) != want_dir;
 }
+
+__device__ __forceinline__ uint32_t *bfs_vis(const BfsArgs &a) { return vload(&a.ctl->vsel) ? a.vis2 : a.vis; }
 
 // Per-thread state of a push level (plain copies, so nothing is read through
 // the kernel-parameter block).
@@ -190,7 +199,8 @@ __global__ void __launch_bounds__(BFS_NT) bfs_push_kernel(BfsArgs a) {
   const int cur = vload(&c->cur);
   const int32_t nin = vload(&c->qlen[cur]);
   const int32_t *qin = cur ? a.q1 : a.q0;
-  PushCtx x{a.label, a.vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, vload(&c->level), 0};
+  uint32_t *vis = bfs_vis(a);
+  PushCtx x{a.label, vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, vload(&c->level), 0};
   bq_init(bq);
   x.bq = &bq;
   int64_t insp = 0, nexp = 0;
@@ -246,6 +256,7 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
   const int32_t iter_cap = vload(&c->iter_cap);
   if (vload(&c->done) || vload(&c->dir) != 0 || nin > a.persist_max || mf > a.persist_edges) return;
   bq_init(bq);
+  uint32_t *vis = bfs_vis(a);
   for (;;) {
     // Per-level counters rotate over three slots: this level appends to `out`;
     // `zero` is the slot the next level appends to (nobody touches it now).
@@ -256,7 +267,7 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
       c->pb[zero] = 0;
     }
     const int32_t *qin = sel ? a.q1 : a.q0;
-    PushCtx x{a.label, a.vis, a.ro, sel ? a.q0 : a.q1, &c->pq[out], &c->overflow, a.qcap, lvl, 0};
+    PushCtx x{a.label, vis, a.ro, sel ? a.q0 : a.q1, &c->pq[out], &c->overflow, a.qcap, lvl, 0};
     x.bq = &bq;
     const BigList big{a.big_v, &c->pb[out], defer_threshold<BFS_NT>(nin, a.cta_th, a.grid_th, a.defer_warp)};
     const int32_t *ci = a.ci, *ri = a.ri;
@@ -348,7 +359,8 @@ __global__ void __launch_bounds__(BFS_NT) bfs_push_big_kernel(BfsArgs a) {
   if (bfs_skip(a, 0)) return;
   DevCtl *c = a.ctl;
   const int cur = vload(&c->cur);
-  PushCtx x{a.label, a.vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, vload(&c->level), 0};
+  uint32_t *vis = bfs_vis(a);
+  PushCtx x{a.label, vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, vload(&c->level), 0};
   bq_init(bq);
   x.bq = &bq;
   const int32_t *ci = a.ci;
@@ -359,65 +371,125 @@ __global__ void __launch_bounds__(BFS_NT) bfs_push_big_kernel(BfsArgs a) {
   if (last_block(&c->blocks_done) && threadIdx.x == 0) bfs_level_end(a);
 }
 
-__global__ void __launch_bounds__(BFS_NT) bfs_pull_kernel(BfsArgs a) {
+// Latency bounds it: few edges are read (R-MAT s22, three levels: 11 M), each at the
+// end of a chain of dependent loads. So the next word's bits and offsets are loaded
+// while this one is scanned; a lane tests a sector of indices at a time, 8 bits in
+// flight; vertices still without a parent after that are taken eight at a time by
+// four lanes each, 32 edges per step (a warp per vertex took up to 32 turns for a word
+// of vertices of middling degree, a lane per vertex up to the longest row); and
+// discoveries are staged per warp (one queue atomic per word queued 130,000 of them on
+// one address). Largest level of R-MAT s22: 191 us one edge and one depth load at a
+// time, 136 us now.
+// BITS: the test reads the bitmap the level found (else the depth, and the one bitmap
+// is updated in place).
+template <bool BITS>
+__global__ void __launch_bounds__(BFS_NT, 6) bfs_pull_kernel(BfsArgs a) {
   __shared__ int64_t s_sum[BFS_NT / 32 + 1];
+  __shared__ int32_t s_stage[BFS_NT / 32][WS_CAP];
   if (bfs_skip(a, 1)) return;
   DevCtl *c = a.ctl;
   const int cur = vload(&c->cur);
   const int32_t level = vload(&c->level);
+  const uint32_t *vis = bfs_vis(a);
+  uint32_t *vout = BITS ? (vload(&c->vsel) ? a.vis : a.vis2) : a.vis;
   int32_t *qout = cur ? a.q0 : a.q1;
   int32_t *qlen_out = &c->qlen[cur ^ 1];
+  WarpStage st{s_stage[warp_id()], 0};
   const int lane = lane_id();
-  const int64_t nwords = (a.n + 31) >> 5;
-  const int64_t wstride = ((int64_t)gridDim.x * BFS_NT) >> 5;
+  const int32_t nwords = (int32_t)((a.n + 31) >> 5), wstride = (int32_t)(gridDim.x * (BFS_NT / 32));
+  const bool same = a.ro == a.co;  // the in-degree is the out-degree
   int64_t mf = 0, insp = 0, nexp = 0;
-  for (int64_t w = ((int64_t)blockIdx.x * BFS_NT + threadIdx.x) >> 5; w < nwords; w += wstride) {
-    const uint32_t vw = a.vis[w];
-    if (vw == FULL) continue;
-    const int64_t v = (w << 5) + lane;
-    const bool need = v < a.n && !((vw >> lane) & 1u);
-    bool found = false;
-    int32_t beg = 0, end = 0;
-    if (need) {
+  // any parent among the sector at e of edges [b, end): all eight loads are issued
+  // before the first is tested
+  auto sector = [&](int32_t e, int32_t b, int32_t end) {
+    int32_t u[8];
+    uint32_t x[8];
+    prb_load8(a.ri + e, u);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const bool in = e + j >= b && e + j < end;
+      if (BITS) x[j] = in ? __ldg(vis + (u[j] >> 5)) : 0u;
+      else x[j] = in ? (uint32_t)a.label[u[j]] : ~0u;
+    }
+    bool f = false;
+#pragma unroll
+    for (int j = 0; j < 8; j++) f |= BITS ? ((x[j] >> (u[j] & 31)) & 1u) != 0 : x[j] == (uint32_t)level;
+    insp += min(e + 8, end) - max(e, b);
+    return f;
+  };
+  // a word's bits and its vertices' offsets, loaded one word ahead
+  auto fetch = [&](int32_t w, uint32_t &vw, int32_t &beg, int32_t &end) {
+    vw = FULL;
+    beg = end = 0;
+    if (w >= nwords) return;
+    vw = vis[w];
+    const int64_t v = ((int64_t)w << 5) + lane;
+    if (v < a.n) {
       beg = a.co[v];
       end = a.co[v + 1];
-      nexp++;
     }
-    const int32_t lim = min(end, beg + PULL_SERIAL);
-    for (int32_t e = beg; e < lim; e++) {
-      insp++;
-      if (a.label[a.ri[e]] == level) {
-        found = true;
-        break;
+  };
+  int32_t w = blockIdx.x * (BFS_NT / 32) + warp_id();
+  uint32_t vw, vw1;
+  int32_t beg, end, beg1, end1;
+  fetch(w, vw, beg, end);
+  for (; w < nwords; w += wstride, vw = vw1, beg = beg1, end = end1) {
+    fetch(w + wstride, vw1, beg1, end1);
+    if (vw == FULL) {
+      if (BITS && lane == 0) vout[w] = FULL;
+      continue;
+    }
+    const int64_t v = ((int64_t)w << 5) + lane;
+    const bool need = v < a.n && !((vw >> lane) & 1u);
+    bool found = false;
+    nexp += need;
+    const int32_t lim = min(end, (beg & ~7) + PULL_SERIAL);
+    if (need && beg < end) found = sector(beg & ~7, beg, lim);
+    unsigned pend = __ballot_sync(FULL, need && !found && lim < end);
+    unsigned far = 0;  // lanes whose vertex is left for the whole warp
+    while (pend) {
+      // quad q takes the q-th waiting vertex
+      unsigned m = pend;
+      for (int q = lane >> 2; q > 0; q--) m &= m - 1;
+      const int l = m ? __ffs(m) - 1 : 0;
+      const int32_t b = __shfl_sync(FULL, lim, l), en0 = __shfl_sync(FULL, end, l);
+      const int32_t en = m ? min(en0, b + PULL_QUAD) : b;
+      const unsigned mine = 0xfu << (lane & ~3);
+      bool f = false;
+      for (int32_t e = (b & ~7) + 8 * (lane & 3); __any_sync(FULL, !f && e - 8 * (lane & 3) < en); e += 32) {
+        if (!f && e < en && e + 8 > b) f = sector(e, b, en);
+        f = (__ballot_sync(FULL, f) & mine) != 0;
+      }
+      // back to the vertices' lanes
+      for (int q = 0; q < 8 && pend; q++) {
+        const int t = __ffs(pend) - 1;
+        pend &= pend - 1;
+        const bool fq = __shfl_sync(FULL, f, 4 * q);
+        const bool more = __shfl_sync(FULL, en0 > en, 4 * q);
+        if (lane == t) found = fq;
+        if (!fq && more) far |= 1u << t;
       }
     }
-    unsigned pend = __ballot_sync(FULL, need && !found && lim < end);
-    while (pend) {
-      const int l = __ffs(pend) - 1;
-      pend &= pend - 1;
-      const int32_t b = __shfl_sync(FULL, lim, l), en = __shfl_sync(FULL, end, l);
+    while (far) {
+      const int l = __ffs(far) - 1;
+      far &= far - 1;
+      const int32_t b = __shfl_sync(FULL, lim, l) + PULL_QUAD, en = __shfl_sync(FULL, end, l);
       bool f = false;
-      for (int32_t e0 = b; e0 < en; e0 += 32) {
-        const int32_t e = e0 + lane;
-        const bool hit = e < en && a.label[a.ri[e]] == level;
-        insp += e < en;
-        if (__any_sync(FULL, hit)) {
-          f = true;
-          break;
-        }
+      for (int32_t e0 = b & ~7; e0 < en && !f; e0 += 256) {
+        const int32_t e = e0 + 8 * lane;
+        f = __any_sync(FULL, e < en && e + 8 > b && sector(e, b, en));
       }
       if (lane == l) found = f;
     }
     const unsigned fm = __ballot_sync(FULL, found);
-    if (fm) {
-      if (lane == 0) a.vis[w] = vw | fm;
-      if (found) {
-        a.label[v] = level + 1;
-        mf += a.ro[v + 1] - a.ro[v];
-      }
-      warp_append(found, (int32_t)v, qout, qlen_out, a.qcap, &c->overflow);
+    if (lane == 0 && (fm || BITS)) vout[w] = vw | fm;
+    if (found) {
+      a.label[v] = level + 1;
+      mf += same ? end - beg : a.ro[v + 1] - a.ro[v];
     }
+    ws_push(st, found, (int32_t)v, qout, qlen_out, a.qcap, &c->overflow);
   }
+  ws_flush(st, qout, qlen_out, a.qcap, &c->overflow);
   const int64_t bmf = block_sum<BFS_NT>(mf, s_sum);
   const int64_t bins = block_sum<BFS_NT>(insp, s_sum);
   const int64_t bexp = block_sum<BFS_NT>(nexp, s_sum);
@@ -479,7 +551,8 @@ __global__ void bfs_seed_kernel(BfsArgs a, const int32_t *srcs, int32_t nsrc, in
 // bottom-up cost less than the extra passes at these sizes.
 //
 // The limits are where the cluster's 8 SMs stop beating the whole grid's per-level
-// kernels.
+// kernels: 1 M edges, R-MAT 194 us against 226, uniform 150 against 218 (32 K edges:
+// 85 and 204, 68 and 179).
 constexpr int SB_NT = 1024;
 constexpr int SB_CLUSTER = 8;
 constexpr int64_t SB_MAX_N = 1 << 17;
@@ -734,14 +807,14 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
   const int32_t qcap = (int32_t)qcap64;
   const int64_t nwords = (n + 31) / 32;
   const size_t need = Carve::need({sizeof(int32_t) * (size_t)n, sizeof(uint32_t) * (size_t)nwords,
-                                   sizeof(int32_t) * (size_t)qcap, sizeof(int32_t) * (size_t)qcap,
+                                   sizeof(uint32_t) * (size_t)nwords, sizeof(int32_t) * (size_t)qcap, sizeof(int32_t) * (size_t)qcap,
                                    sizeof(int32_t) * (size_t)nsrc, sizeof(int32_t) * (size_t)BIG_CAP,
                                    sizeof(int2) * (size_t)(n <= SB_MAX_N && g->m <= SB_MAX_M ? small_bfs_chunks(g->m)
                                                                                              : 0)});
   MG_TRY(ws_reserve(g, g->ws_main, need));
   Carve cv(g->ws_main.ptr);
   int32_t *label_ws = cv.take<int32_t>(n);
-  uint32_t *vis = cv.take<uint32_t>(nwords);
+  uint32_t *vis = cv.take<uint32_t>(nwords), *vis2 = cv.take<uint32_t>(nwords);
   int32_t *q0 = cv.take<int32_t>(qcap);
   int32_t *q1 = cv.take<int32_t>(qcap);
   int32_t *dsrc = cv.take<int32_t>(nsrc);
@@ -758,6 +831,7 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
   a.ri = g->has_csc ? g->ri : g->ci;
   a.label = label;
   a.vis = vis;
+  a.vis2 = vis2;
   a.q0 = q0;
   a.q1 = q1;
   a.qcap = qcap;
@@ -844,7 +918,7 @@ extern "C" mg_status mg_bfs(mg_graph *g, const int32_t *srcs, int32_t nsrc, int3
       if (tail) bfs_persist_kernel<<<1, BFS_NT, 0, st>>>(ta);
       bfs_push_kernel<<<grid, BFS_NT, 0, st>>>(b);
       bfs_push_big_kernel<<<grid, BFS_NT, 0, st>>>(b);
-      bfs_pull_kernel<<<grid, BFS_NT, 0, st>>>(b);
+      bfs_pull_kernel<true><<<grid + grid / 2, BFS_NT, 0, st>>>(b);  // less state per warp than the push kernels
     };
     MG_TRY(run_loop(g, SLOT_BFS, &sig, sizeof(sig), o.use_graph, body, n + 2));
   }
@@ -1027,7 +1101,7 @@ extern "C" mg_status mg_bfs_noalloc(mg_graph *g, const int32_t *srcs, int32_t ns
   LoopBody body = [a, grid](cudaStream_t st, cudaGraphConditionalHandle, int) {
     bfs_push_kernel<<<grid, BFS_NT, 0, st>>>(a);
     bfs_push_big_kernel<<<grid, BFS_NT, 0, st>>>(a);
-    bfs_pull_kernel<<<grid, BFS_NT, 0, st>>>(a);
+    bfs_pull_kernel<false><<<grid, BFS_NT, 0, st>>>(a);
   };
   MG_TRY(run_loop(g, SLOT_BFS, nullptr, 0, -1, body, n + 2));
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));

@@ -65,6 +65,7 @@ struct DevCtl {
   int32_t far_min;
   int32_t splits;
   int64_t mf_front;          // out-edges of the current frontier (BFS)
+  int32_t vsel;              // BFS: which of the two visited bitmaps is current
   // persistent kernels: per-level counters in a ring of three (frontier out-edges,
   // frontier sizes), and the grid barrier (arrivals, generation)
   int64_t pm[3];

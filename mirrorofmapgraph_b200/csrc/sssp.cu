@@ -28,7 +28,6 @@ namespace mg {
 constexpr int SSSP_NT = 256;
 constexpr int SSSP_CH = 256;  // edges per chunk of a heavy frontier vertex
 constexpr int SSSP_U = 4;     // edge slots of 32 a warp holds in flight
-constexpr int SSSP_WS = 128;  // next-frontier stage per warp (shared memory)
 
 struct SsspArgs {
   const int32_t *ro, *ci, *w;   // CSR with weights (w == nullptr: unit weights)
@@ -54,42 +53,6 @@ struct SsspArgs {
   uint32_t bar_extra;            // test hook (mg_debug_barrier_skew)
   unsigned long long bar_limit;  // barrier polls before MG_ERR_TIMEOUT
 };
-
-// Per-warp staging of next-frontier appends in shared memory: one global atomic
-// per SSSP_WS items instead of one per warp-wide append (a round of R-MAT s22 adds
-// two million vertices to one queue).
-struct WarpStage {
-  int32_t *buf;
-  int32_t n;  // entries held (the same in every lane)
-};
-
-// Every lane of the warp calls it.
-__device__ __forceinline__ void ws_flush(WarpStage &st, int32_t *queue, int32_t *len, int32_t cap,
-                                         int32_t *overflow) {
-  __syncwarp();
-  if (st.n == 0) return;
-  int32_t base = 0;
-  if (lane_id() == 0) base = atomicAdd(len, st.n);
-  base = __shfl_sync(FULL, base, 0);
-  for (int32_t i = lane_id(); i < st.n; i += 32) {
-    const int32_t pos = base + i;
-    if (pos < cap) queue[pos] = st.buf[i];
-    else *overflow = 1;
-  }
-  __syncwarp();
-  st.n = 0;
-}
-
-// Appends item where pred; every lane of the warp calls it.
-__device__ __forceinline__ void ws_push(WarpStage &st, bool pred, int32_t item, int32_t *queue, int32_t *len,
-                                        int32_t cap, int32_t *overflow) {
-  const unsigned pm = __ballot_sync(FULL, pred);
-  if (pm == 0) return;
-  const int32_t cnt = __popc(pm);
-  if (st.n + cnt > SSSP_WS) ws_flush(st, queue, len, cap, overflow);
-  if (pred) st.buf[st.n + __popc(pm & lanemask_lt())] = item;
-  st.n += cnt;
-}
 
 struct RelaxCtx {
   int32_t *dist;
@@ -274,7 +237,7 @@ __device__ __forceinline__ void sssp_counters(DevCtl *c, int64_t *s_sum, int64_t
 // Relaxation round, pass 1: each warp takes 32 frontier items, cuts the heavy ones
 // into chunks for pass 2 and walks the edges of the others itself.
 __global__ void __launch_bounds__(SSSP_NT, 4) sssp_relax_kernel(SsspArgs a) {
-  __shared__ int32_t s_stage[SSSP_NT / 32][SSSP_WS];
+  __shared__ int32_t s_stage[SSSP_NT / 32][WS_CAP];
   __shared__ int64_t s_sum[SSSP_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
@@ -328,7 +291,7 @@ __global__ void __launch_bounds__(SSSP_NT, 4) sssp_relax_kernel(SsspArgs a) {
 // Pass 2: every warp of the grid relaxes chunks of the heavy vertices' edges; the
 // last CTA closes the round.
 __global__ void __launch_bounds__(SSSP_NT, 4) sssp_chunk_kernel(SsspArgs a) {
-  __shared__ int32_t s_stage[SSSP_NT / 32][SSSP_WS];
+  __shared__ int32_t s_stage[SSSP_NT / 32][WS_CAP];
   __shared__ int64_t s_sum[SSSP_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
@@ -525,7 +488,7 @@ constexpr int NF_NT = 1024;
 constexpr unsigned long long NF_WAIT = 1ull << 22;  // barrier polls (seconds at most) before giving up
 
 __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
-  __shared__ int32_t s_stage[NF_NT / 32][SSSP_WS];
+  __shared__ int32_t s_stage[NF_NT / 32][WS_CAP];
   __shared__ int64_t s_sum[NF_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) return;
