@@ -112,12 +112,29 @@ __device__ __forceinline__ void relax_group(RelaxCtx &x, WarpStage &st, const in
     ob[r] = 0xffffffffu;  // no claim: reads as "already queued"
     if (win) ob[r] = atomicOr((nearq[r] ? x.inq_next : x.infar) + (u[r] >> 5), 1u << (u[r] & 31));
   }
+  unsigned far[SSSP_U];
+  int32_t nfar = 0;
 #pragma unroll
   for (int r = 0; r < SSSP_U; r++) {
     if (tr[r] && nd[r] < old[r]) x.updates++;
     const bool fresh = u[r] >= 0 && !(ob[r] & (1u << (u[r] & 31)));
     ws_push(st, fresh && nearq[r], u[r], x.qout, x.qlen_out, x.qcap, x.overflow);
-    warp_append(fresh && !nearq[r], u[r], x.far_out, x.far_len_out, x.qcap, x.overflow);
+    far[r] = __ballot_sync(FULL, fresh && !nearq[r]);
+    nfar += __popc(far[r]);
+  }
+  if (nfar == 0) return;
+  // one round trip for the far appends of all SSSP_U edges
+  int32_t at = 0;
+  if (lane_id() == 0) at = atomicAdd(x.far_len_out, nfar);
+  at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+  for (int r = 0; r < SSSP_U; r++) {
+    if ((far[r] >> lane_id()) & 1u) {
+      const int32_t pos = at + __popc(far[r] & lanemask_lt());
+      if (pos < x.qcap) x.far_out[pos] = u[r];
+      else *x.overflow = 1;
+    }
+    at += __popc(far[r]);
   }
 }
 
@@ -479,7 +496,9 @@ __global__ void __launch_bounds__(SSSP_NT) sssp_far_split_kernel(SsspArgs a) {
 // with nothing to do. Here a round is the relaxation and one grid barrier; rounds
 // with heavy vertices take a second barrier after their chunks, and a split of the
 // far pile takes two. One CTA of 1024 threads per SM: 148 arrivals per barrier.
-// Every block reads the same counters after a barrier and takes the same decisions.
+// Every block sees the same counters after a barrier and takes the same decisions;
+// one thread per block reads them, with the barrier's last poll behind it, since
+// every warp of the grid reading one L2 sector queues for microseconds.
 //
 // Counters rotate over three slots, one per step (a round or a split): a step adds
 // to its own slot and block 0 clears the next step's, which was last read two steps
@@ -490,6 +509,9 @@ constexpr unsigned long long NF_WAIT = 1ull << 22;  // barrier polls (seconds at
 __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
   __shared__ int32_t s_stage[NF_NT / 32][WS_CAP];
   __shared__ int64_t s_sum[NF_NT / 32 + 1];
+  __shared__ struct {
+    int32_t sq, sc, smin, far[2], over, ok;
+  } s_c;
   DevCtl *c = a.ctl;
   if (vload(&c->done)) return;
   const int lane = lane_id();
@@ -504,7 +526,33 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
   int64_t thr = vload(&c->thr);
   int64_t insp = 0, nexp = 0, upd = 0;
   bool ok = true, done = false, over = false;
-  auto barrier = [&]() { return grid_barrier(&c->bar_count, &c->bar_gen, a.bar_limit, a.bar_extra); };
+  unsigned arrivals = 0;  // what bar_count reaches at the current barrier (it only grows)
+  auto barrier = [&](int slot) {
+    __syncthreads();
+    arrivals += gridDim.x + a.bar_extra;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(&c->bar_count, 1u);
+      unsigned long long it = 0;
+      int in = 1;
+      while ((int)(vload(&c->bar_count) - arrivals) < 0) {
+        if (++it > a.bar_limit) {
+          in = 0;
+          break;
+        }
+      }
+      __threadfence();
+      s_c.sq = vload(&c->sq[slot]);
+      s_c.sc = vload(&c->sc[slot]);
+      s_c.smin = vload(&c->smin[slot]);
+      s_c.far[0] = vload(&c->far_len[0]);
+      s_c.far[1] = vload(&c->far_len[1]);
+      s_c.over = vload(&c->overflow);
+      s_c.ok = in;
+    }
+    __syncthreads();
+    return s_c.ok != 0;
+  };
   auto next_slot = [&]() {
     const int slot = step % 3, z = (step + 1) % 3;
     step++;
@@ -552,8 +600,8 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
     insp += edges;
     edges = warp_sum(edges);
     if (lane == 0 && edges) atomicAdd((unsigned long long *)&c->se[slot], (unsigned long long)edges);
-    if (!(ok = barrier())) break;
-    const int32_t nch = min(vload(&c->sc[slot]), a.chunk_cap);
+    if (!(ok = barrier(slot))) break;
+    const int32_t nch = min(s_c.sc, a.chunk_cap);
     if (nch > 0) {
       for (int32_t ch = gw; ch < nch; ch += nw) {
         const int2 e = __ldcg(a.chunks + ch);
@@ -579,21 +627,21 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
         }
       }
       ws_flush(st, x.qout, x.qlen_out, x.qcap, x.overflow);
-      if (!(ok = barrier())) break;
+      if (!(ok = barrier(slot))) break;
     }
     upd += x.updates;
     // Round end (sssp_level_end's rules).
     if (lead) trace_level(c, lvl, MG_DIR_PUSH, nin, vload(&c->se[slot]), 0.0);
-    int32_t nf = vload(&c->sq[slot]);
-    const int32_t nfar = vload(&c->far_len[fc]);
-    over = vload(&c->overflow) != 0;
+    int32_t nf = s_c.sq;
+    const int32_t nfar = s_c.far[fc];
+    over = s_c.over != 0;
     lvl++;
     sel ^= 1;
     bool split = nf == 0 && nfar > 0 && !over;
     done = (nf == 0 && !split) || lvl >= iter_cap || over;
     while (split && !done) {
       const int sp = next_slot();
-      const int32_t len = min(vload(&c->far_len[fc]), a.qcap);
+      const int32_t len = min(s_c.far[fc], a.qcap);
       const int32_t *far = fc ? a.far1 : a.far0;
       int32_t *keep_to = fc ? a.far0 : a.far1;
       int32_t mn = INT_MAX;
@@ -603,8 +651,8 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
       }
       mn = __reduce_min_sync(FULL, mn);
       if (lane == 0 && mn != INT_MAX) atomicMin(&c->smin[sp], mn);
-      if (!(ok = barrier())) break;
-      const int32_t fmin = vload(&c->smin[sp]);
+      if (!(ok = barrier(sp))) break;
+      const int32_t fmin = s_c.smin;
       const int64_t thr_new = (fmin == INT_MAX ? thr : max(thr, (int64_t)fmin)) + a.delta;
       int32_t *qnear = sel ? a.q1 : a.q0;
       uint32_t *inq_near = sel ? a.inq1 : a.inq0;
@@ -627,10 +675,10 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
         warp_append(to_near, u, qnear, &c->sq[sp], a.qcap, &c->overflow);
         warp_append(keep, u, keep_to, &c->far_len[fc ^ 1], a.qcap, &c->overflow);
       }
-      if (!(ok = barrier())) break;
-      nf = vload(&c->sq[sp]);
-      const int32_t nk = vload(&c->far_len[fc ^ 1]);
-      over = vload(&c->overflow) != 0;
+      if (!(ok = barrier(sp))) break;
+      nf = s_c.sq;
+      const int32_t nk = s_c.far[fc ^ 1];
+      over = s_c.over != 0;
       thr = thr_new;
       // the old pile's length: next added to two barriers from now
       if (lead) c->far_len[fc] = 0;
