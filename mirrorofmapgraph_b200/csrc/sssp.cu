@@ -27,7 +27,8 @@ namespace mg {
 
 constexpr int SSSP_NT = 256;
 constexpr int SSSP_CH = 256;  // edges per chunk of a heavy frontier vertex
-constexpr int SSSP_U = 4;     // edge slots of 32 a warp holds in flight
+constexpr int SSSP_U = 4;     // edge slots of 32 a warp holds in flight (near-far rounds)
+constexpr int SSSP_P = 8;     // the same for plain rounds
 
 struct SsspArgs {
   const int32_t *ro, *ci, *w;   // CSR with weights (w == nullptr: unit weights)
@@ -45,6 +46,7 @@ struct SsspArgs {
   int32_t vmask;   // item -> vertex mask: -1 for one instance; batched runs keep the
                    // instance number in the bits above it (item = instance << s | v)
   int32_t delta;   // near-far bucket width (0: plain frontier Bellman-Ford)
+  int32_t plain;   // 1: plain rounds in the one-launch kernel: every improvement is near
   int32_t *far0, *far1;  // far piles (ping-pong)
   uint32_t *infar;       // bit per item: in the current far pile
   DevCtl *ctl;
@@ -69,72 +71,91 @@ struct RelaxCtx {
   int32_t *far_out, *far_len_out;
 };
 
-// Relaxes SSSP_U edges per lane: edge r goes to item u[r] (-1: none) with weight
-// w[r] from a vertex at distance dv[r]. The loads, the atomicMins and the bitmap
-// claims of the SSSP_U edges are each issued together, so a lane waits for one
-// memory round trip per step rather than per edge. Every lane of the warp calls it.
-__device__ __forceinline__ void relax_group(RelaxCtx &x, WarpStage &st, const int32_t (&u)[SSSP_U],
-                                            const int32_t (&w)[SSSP_U], const int32_t (&dv)[SSSP_U]) {
-  int32_t cd[SSSP_U], nd[SSSP_U], old[SSSP_U];
-  bool tr[SSSP_U];
+// Near-far: lowers the heads of the edges tr[r] to nd[r], claims those that did
+// improve and appends them to the near frontier or the far pile.
+template <int U>
+__device__ __forceinline__ void relax_far(RelaxCtx &x, WarpStage &st, const int32_t (&u)[U], const uint32_t (&nd)[U],
+                                          const bool (&tr)[U]) {
+  int32_t old[U];
 #pragma unroll
-  for (int r = 0; r < SSSP_U; r++) cd[r] = u[r] >= 0 ? __ldcg(x.dist + u[r]) : INT_MIN;
+  for (int r = 0; r < U; r++) old[r] = tr[r] ? atomicMin(x.dist + u[r], (int32_t)nd[r]) : INT_MIN;
+  uint32_t ob[U];
+  bool nearq[U];
 #pragma unroll
-  for (int r = 0; r < SSSP_U; r++) {
-    const int64_t s = (int64_t)dv[r] + (int64_t)w[r];
-    tr[r] = u[r] >= 0 && s < (int64_t)cd[r];
-    nd[r] = (int32_t)min(s, (int64_t)INT_MAX);
-  }
-  if (x.delta <= 0) {
-    // Plain rounds: an edge that improves on the distance read before the
-    // atomicMin marks its head in the next-frontier bitmap, and neither atomic's
-    // old value is waited for (the frontier is compacted from the bitmap after the
-    // round). A mark from an improvement that a concurrent smaller one overtook
-    // only expands that vertex once more.
-#pragma unroll
-    for (int r = 0; r < SSSP_U; r++) {
-      if (tr[r]) {
-        red_min(x.dist + u[r], nd[r]);
-        red_or(x.inq_next + (u[r] >> 5), 1u << (u[r] & 31));
-        x.updates++;
-      }
-    }
-    return;
-  }
-#pragma unroll
-  for (int r = 0; r < SSSP_U; r++) old[r] = tr[r] ? atomicMin(x.dist + u[r], nd[r]) : INT_MIN;
-  uint32_t ob[SSSP_U];
-  bool nearq[SSSP_U];
-#pragma unroll
-  for (int r = 0; r < SSSP_U; r++) {
-    const bool win = tr[r] && nd[r] < old[r];
+  for (int r = 0; r < U; r++) {
+    const bool win = tr[r] && (int32_t)nd[r] < old[r];
     nearq[r] = (int64_t)nd[r] < x.thr;
     ob[r] = 0xffffffffu;  // no claim: reads as "already queued"
     if (win) ob[r] = atomicOr((nearq[r] ? x.inq_next : x.infar) + (u[r] >> 5), 1u << (u[r] & 31));
   }
-  unsigned far[SSSP_U];
+  unsigned far[U];
   int32_t nfar = 0;
 #pragma unroll
-  for (int r = 0; r < SSSP_U; r++) {
-    if (tr[r] && nd[r] < old[r]) x.updates++;
+  for (int r = 0; r < U; r++) {
+    if (tr[r] && (int32_t)nd[r] < old[r]) x.updates++;
     const bool fresh = u[r] >= 0 && !(ob[r] & (1u << (u[r] & 31)));
     ws_push(st, fresh && nearq[r], u[r], x.qout, x.qlen_out, x.qcap, x.overflow);
     far[r] = __ballot_sync(FULL, fresh && !nearq[r]);
     nfar += __popc(far[r]);
   }
   if (nfar == 0) return;
-  // one round trip for the far appends of all SSSP_U edges
+  // one round trip for the far appends of all U edges
   int32_t at = 0;
   if (lane_id() == 0) at = atomicAdd(x.far_len_out, nfar);
   at = __shfl_sync(FULL, at, 0);
 #pragma unroll
-  for (int r = 0; r < SSSP_U; r++) {
+  for (int r = 0; r < U; r++) {
     if ((far[r] >> lane_id()) & 1u) {
       const int32_t pos = at + __popc(far[r] & lanemask_lt());
       if (pos < x.qcap) x.far_out[pos] = u[r];
       else *x.overflow = 1;
     }
     at += __popc(far[r]);
+  }
+}
+
+// Relaxes U edges per lane: edge r goes to item u[r] (-1: none) with weight w[r]
+// from a vertex at distance dv[r]. The loads, the atomicMins and the bitmap claims of
+// the U edges are each issued together, so a lane waits for one memory round trip per
+// step rather than per edge. FAR: near-far rounds. Every lane of the warp calls it.
+template <int U, bool FAR>
+__device__ __forceinline__ void relax_group(RelaxCtx &x, WarpStage &st, const int32_t (&u)[U], const int32_t (&w)[U],
+                                            const int32_t (&dv)[U]) {
+  uint32_t cd[U], nd[U];
+  bool tr[U];
+#pragma unroll
+  for (int r = 0; r < U; r++) cd[r] = u[r] >= 0 ? (uint32_t)(FAR ? __ldcg(x.dist + u[r]) : __ldca(x.dist + u[r])) : 0u;
+#pragma unroll
+  for (int r = 0; r < U; r++) {
+    nd[r] = (uint32_t)dv[r] + (uint32_t)w[r];  // below 2^32; an improvement is below INT_MAX
+    tr[r] = nd[r] < cd[r];
+  }
+  if constexpr (!FAR) {
+    // The first look goes through L1, which holds the hubs' distances: the traffic of
+    // random sectors from the L2 bounds the large rounds (160 sectors a nanosecond, as
+    // in every gather here). A distance in L1 may be an older, larger one, so an edge
+    // that passes looks again in the L2.
+#pragma unroll
+    for (int r = 0; r < U; r++) cd[r] = tr[r] ? (uint32_t)__ldcg(x.dist + u[r]) : 0u;
+#pragma unroll
+    for (int r = 0; r < U; r++) tr[r] = nd[r] < cd[r];
+  }
+  if constexpr (!FAR) {
+    // Plain rounds: an edge that improves on the distance read before the
+    // atomicMin marks its head in the next-frontier bitmap, and neither atomic's
+    // old value is waited for (the frontier is compacted from the bitmap after the
+    // round). A mark from an improvement that a concurrent smaller one overtook
+    // only expands that vertex once more.
+#pragma unroll
+    for (int r = 0; r < U; r++) {
+      if (tr[r]) {
+        red_min(x.dist + u[r], (int32_t)nd[r]);
+        red_or(x.inq_next + (u[r] >> 5), 1u << (u[r] & 31));
+        x.updates++;
+      }
+    }
+  } else {
+    relax_far<U>(x, st, u, nd, tr);
   }
 }
 
@@ -146,9 +167,9 @@ __device__ __forceinline__ RelaxCtx relax_ctx(const SsspArgs &a, DevCtl *c, int 
 }
 
 // The edges of the warp's 32 vertices (lane l brings vertex item v, its distance
-// dv, its first edge beg and deg edges), concatenated and walked 32 x SSSP_U at a
-// time: edge slot j belongs to the last lane whose exclusive degree prefix is <= j
+// dv, its first edge beg and deg edges), concatenated and walked 32 x U at a time: edge slot j belongs to the last lane whose exclusive degree prefix is <= j
 // (binary search over the lanes' prefixes by shuffles).
+template <int U, bool FAR>
 __device__ __forceinline__ void warp_walk(RelaxCtx &x, WarpStage &st, int32_t v, int32_t dv, int32_t beg,
                                           int32_t deg, const int32_t *__restrict__ adj,
                                           const int32_t *__restrict__ wt, int32_t hi) {
@@ -157,10 +178,10 @@ __device__ __forceinline__ void warp_walk(RelaxCtx &x, WarpStage &st, int32_t v,
   const int32_t tot = __shfl_sync(FULL, inc, 31);
   const int32_t ex = inc - deg;
   const int32_t kb = beg - ex;  // edge index of slot j of this lane's vertex: kb + j
-  for (int32_t b0 = 0; b0 < tot; b0 += 32 * SSSP_U) {
-    int32_t u[SSSP_U], w[SSSP_U], d[SSSP_U];
+  for (int32_t b0 = 0; b0 < tot; b0 += 32 * U) {
+    int32_t u[U], w[U], d[U];
 #pragma unroll
-    for (int r = 0; r < SSSP_U; r++) {
+    for (int r = 0; r < U; r++) {
       const int32_t j = b0 + r * 32 + lane;
       int l = 0;
 #pragma unroll
@@ -173,7 +194,7 @@ __device__ __forceinline__ void warp_walk(RelaxCtx &x, WarpStage &st, int32_t v,
       u[r] = ok ? ((sv & hi) | adj[k]) : -1;
       w[r] = ok ? (wt ? wt[k] : 1) : 0;
     }
-    relax_group(x, st, u, w, d);
+    relax_group<U, FAR>(x, st, u, w, d);
   }
 }
 
@@ -233,7 +254,7 @@ __device__ void sssp_level_end(const SsspArgs &a) {
   if (over) c->status = MG_ERR_QUEUE_OVERFLOW;
   __threadfence();
   c->done = done ? 1 : 0;
-  if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+  loop_signal(a.ctl, a.h, a.use_cond, done);
 }
 
 // Adds a block's counters to the control block.
@@ -252,13 +273,18 @@ __device__ __forceinline__ void sssp_counters(DevCtl *c, int64_t *s_sum, int64_t
 }
 
 // Relaxation round, pass 1: each warp takes 32 frontier items, cuts the heavy ones
-// into chunks for pass 2 and walks the edges of the others itself.
+// into chunks for pass 2 and walks the edges of the others itself. Both passes are
+// bound by the latency of dependent loads (R-MAT s21: 34% of the L2's throughput, 16%
+// of the issue slots), so a plain round holds SSSP_P edges per lane in flight and
+// loads what the next step starts from while it relaxes this one.
+template <bool FAR>
 __global__ void __launch_bounds__(SSSP_NT, 4) sssp_relax_kernel(SsspArgs a) {
+  constexpr int U = FAR ? SSSP_U : SSSP_P;
   __shared__ int32_t s_stage[SSSP_NT / 32][WS_CAP];
   __shared__ int64_t s_sum[SSSP_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
@@ -274,15 +300,17 @@ __global__ void __launch_bounds__(SSSP_NT, 4) sssp_relax_kernel(SsspArgs a) {
   // a vertex of their own: hand every vertex of heavy_small edges or more to pass 2.
   const int32_t th = (int64_t)nin < nw * 32 ? a.heavy_small : a.heavy;
   int64_t insp = 0, nexp = 0;
+  int32_t next = gw * 32 + lane_id() < nin ? qin[gw * 32 + lane_id()] : -1;
   for (int64_t base = gw * 32; base < nin; base += nw * 32) {
-    const int64_t i = base + lane_id();
-    const int32_t v = i < nin ? qin[i] : -1;
+    const int32_t v = next;
+    const int64_t i1 = base + nw * 32 + lane_id();
+    next = i1 < nin ? qin[i1] : -1;
     int32_t beg = 0, deg = 0, dv = 0, cb = 0, cdeg = 0;
     if (v >= 0) {
       // Near-far rounds: the whole bitmap of the current frontier is cleared here,
       // one word at a time (nothing sets bits in it during this round). Plain
       // rounds have one bitmap, cleared by the compaction.
-      if (a.delta > 0) inq_cur[v >> 5] = 0u;
+      if (FAR) inq_cur[v >> 5] = 0u;
       nexp++;
       beg = a.ro[v & a.vmask];
       deg = a.ro[(v & a.vmask) + 1] - beg;
@@ -294,10 +322,10 @@ __global__ void __launch_bounds__(SSSP_NT, 4) sssp_relax_kernel(SsspArgs a) {
       insp += deg + cdeg;
     }
     deg = warp_chunks(a, &c->big_len, v, beg, deg, th, 0);
-    warp_walk(x, st, v, dv, beg, deg, a.ci, a.w, hi);
+    warp_walk<U, FAR>(x, st, v, dv, beg, deg, a.ci, a.w, hi);
     if (a.both) {
       cdeg = warp_chunks(a, &c->big_len, v, cb, cdeg, th, INT_MIN);
-      warp_walk(x, st, v, dv, cb, cdeg, a.ri, a.cw, hi);
+      warp_walk<U, FAR>(x, st, v, dv, cb, cdeg, a.ri, a.cw, hi);
     }
   }
   ws_flush(st, x.qout, x.qlen_out, x.qcap, x.overflow);
@@ -305,50 +333,71 @@ __global__ void __launch_bounds__(SSSP_NT, 4) sssp_relax_kernel(SsspArgs a) {
   sssp_counters(c, s_sum, insp, insp, nexp, x.updates);
 }
 
+// A chunk of a heavy vertex: its edges [k0, end), the vertex's item and distance.
+struct SsspChunk {
+  int32_t item, k0, end, dv;
+  bool rev;
+};
+
+// Relaxes a chunk, 32 x U edges at a time.
+template <int U, bool FAR>
+__device__ __forceinline__ void chunk_walk(RelaxCtx &x, WarpStage &st, const SsspArgs &a, const SsspChunk &h) {
+  const int32_t *adj = h.rev ? a.ri : a.ci;
+  const int32_t *wt = h.rev ? a.cw : a.w;
+  const int32_t base = h.item & ~a.vmask;
+  for (int32_t b = h.k0; b < h.end; b += 32 * U) {
+    int32_t u[U], w[U], d[U];
+#pragma unroll
+    for (int r = 0; r < U; r++) {
+      const int32_t k = b + r * 32 + lane_id();
+      u[r] = k < h.end ? (base | adj[k]) : -1;
+      w[r] = wt && k < h.end ? wt[k] : 1;
+      d[r] = h.dv;
+    }
+    relax_group<U, FAR>(x, st, u, w, d);
+  }
+}
+
 // Pass 2: every warp of the grid relaxes chunks of the heavy vertices' edges; the
-// last CTA closes the round.
+// last CTA closes the round. A warp's next chunk is on its way while it relaxes one:
+// its header two chunks ahead, its end and its vertex's distance one ahead (a
+// distance that improves meanwhile has marked its vertex for the next round).
+template <bool FAR>
 __global__ void __launch_bounds__(SSSP_NT, 4) sssp_chunk_kernel(SsspArgs a) {
+  constexpr int U = FAR ? SSSP_U : SSSP_P;
   __shared__ int32_t s_stage[SSSP_NT / 32][WS_CAP];
   __shared__ int64_t s_sum[SSSP_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
   RelaxCtx x = relax_ctx(a, c, cur);
   WarpStage st{s_stage[warp_id()], 0};
-  const int32_t hi = ~a.vmask;
-  const int lane = lane_id();
   const int32_t nch = min(vload(&c->big_len), a.chunk_cap);
   const int32_t nw = gridDim.x * (SSSP_NT / 32);
-  for (int32_t ch = blockIdx.x * (SSSP_NT / 32) + warp_id(); ch < nch; ch += nw) {
-    const int2 e = a.chunks[ch];
-    if (e.x < 0) continue;
-    const bool rev = e.y < 0;
-    const int32_t k0 = e.y & INT_MAX;
-    const int32_t *off = rev ? a.co : a.ro;
-    const int32_t *adj = rev ? a.ri : a.ci;
-    const int32_t *wt = rev ? a.cw : a.w;
-    const int32_t end = min(k0 + SSSP_CH, off[(e.x & a.vmask) + 1]);
-    const int32_t dv = vload(a.dist + e.x);
-    const int32_t base = e.x & hi;
-    for (int32_t b = k0; b < end; b += 32 * SSSP_U) {
-      int32_t u[SSSP_U], w[SSSP_U], d[SSSP_U];
-#pragma unroll
-      for (int r = 0; r < SSSP_U; r++) {
-        const int32_t k = b + r * 32 + lane;
-        const bool ok = k < end;
-        u[r] = ok ? (base | adj[k]) : -1;
-        w[r] = ok ? (wt ? wt[k] : 1) : 0;
-        d[r] = dv;
-      }
-      relax_group(x, st, u, w, d);
+  auto header = [&](int32_t ch) { return ch < nch ? a.chunks[ch] : make_int2(-1, 0); };
+  auto open = [&](const int2 &e) {
+    SsspChunk h{e.x, e.y & INT_MAX, 0, 0, e.y < 0};
+    if (e.x >= 0) {
+      h.end = min(h.k0 + SSSP_CH, (h.rev ? a.co : a.ro)[(e.x & a.vmask) + 1]);
+      h.dv = vload(a.dist + e.x);
     }
+    return h;
+  };
+  int32_t ch = blockIdx.x * (SSSP_NT / 32) + warp_id();
+  SsspChunk h = open(header(ch));
+  int2 e1 = header(ch + nw);
+  for (; ch < nch; ch += nw) {
+    const SsspChunk h1 = open(e1);
+    e1 = header(ch + 2 * nw);
+    chunk_walk<U, FAR>(x, st, a, h);  // an empty slot (item -1) has no edges
+    h = h1;
   }
   ws_flush(st, x.qout, x.qlen_out, x.qcap, x.overflow);
   sssp_counters(c, s_sum, 0, 0, 0, x.updates);
-  if (a.delta > 0 && last_block(&c->blocks_done) && threadIdx.x == 0) sssp_level_end(a);
+  if (FAR && last_block(&c->blocks_done) && threadIdx.x == 0) sssp_level_end(a);
 }
 
 // Plain rounds, pass 3: the next frontier, compacted in item order from the
@@ -360,7 +409,7 @@ __global__ void __launch_bounds__(SSSP_NT) sssp_compact_kernel(SsspArgs a) {
   __shared__ int32_t s_base;
   DevCtl *c = a.ctl;
   if (a.delta > 0 || vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0 && vload(&c->done)) cudaGraphSetConditional(a.h, 0u);
+    if (vload(&c->done)) loop_over(c, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
@@ -409,7 +458,7 @@ __global__ void sssp_reach_kernel(const int32_t *__restrict__ dist, int64_t nite
 __global__ void __launch_bounds__(SSSP_NT) sssp_far_min_kernel(SsspArgs a) {
   DevCtl *c = a.ctl;
   if (vload(&c->done) || !vload(&c->split)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0 && vload(&c->done)) cudaGraphSetConditional(a.h, 0u);
+    if (vload(&c->done)) loop_over(c, a.h, a.use_cond);
     return;
   }
   const int fc = vload(&c->far_cur);
@@ -431,7 +480,7 @@ __global__ void __launch_bounds__(SSSP_NT) sssp_far_min_kernel(SsspArgs a) {
 __global__ void __launch_bounds__(SSSP_NT) sssp_far_split_kernel(SsspArgs a) {
   DevCtl *c = a.ctl;
   if (vload(&c->done) || !vload(&c->split)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0 && vload(&c->done)) cudaGraphSetConditional(a.h, 0u);
+    if (vload(&c->done)) loop_over(c, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
@@ -487,10 +536,11 @@ __global__ void __launch_bounds__(SSSP_NT) sssp_far_split_kernel(SsspArgs a) {
   if (over) c->status = MG_ERR_QUEUE_OVERFLOW;
   __threadfence();
   c->done = done ? 1 : 0;
-  if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+  loop_signal(a.ctl, a.h, a.use_cond, done);
 }
 
-// All rounds of a near-far run in one cooperative launch. A high-diameter graph
+// All rounds of a near-far run, or of a plain run on a small graph, in one
+// cooperative launch. A high-diameter graph
 // takes hundreds of rounds of a few thousand vertices (4096^2 lattice: 437), where
 // a sequence of four launches per round cost 41 us a round, most of it in kernels
 // with nothing to do. Here a round is the relaxation and one grid barrier; rounds
@@ -504,6 +554,10 @@ __global__ void __launch_bounds__(SSSP_NT) sssp_far_split_kernel(SsspArgs a) {
 // to its own slot and block 0 clears the next step's, which was last read two steps
 // ago, so at least one barrier lies between.
 constexpr int NF_NT = 1024;
+// Plain rounds in one launch up to this many edges: R-MAT of mean degree 32, 0.5 M /
+// 4 M / 8 M edges 260 / 487 / 824 us against 363 / 525 / 712 for the per-round kernels
+// (uniform: 489 / 777 / 1041 against 734 / 1050 / 1298).
+constexpr int64_t NF_PLAIN_M = 1 << 22;
 constexpr unsigned long long NF_WAIT = 1ull << 22;  // barrier polls (seconds at most) before giving up
 
 __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
@@ -523,7 +577,7 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
   int32_t nin = vload(&c->qlen[0]);
   int sel = 0, fc = 0, step = 0, splits = 0;
   int32_t lvl = 0;
-  int64_t thr = vload(&c->thr);
+  int64_t thr = a.plain ? INT64_MAX : vload(&c->thr);
   int64_t insp = 0, nexp = 0, upd = 0;
   bool ok = true, done = false, over = false;
   unsigned arrivals = 0;  // what bar_count reaches at the current barrier (it only grows)
@@ -590,10 +644,10 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
         edges += deg + cdeg;
       }
       deg = warp_chunks(a, &c->sc[slot], v, beg, deg, th, 0);
-      warp_walk(x, st, v, dv, beg, deg, a.ci, a.w, hi);
+      warp_walk<SSSP_U, true>(x, st, v, dv, beg, deg, a.ci, a.w, hi);
       if (a.both) {
         cdeg = warp_chunks(a, &c->sc[slot], v, cb, cdeg, th, INT_MIN);
-        warp_walk(x, st, v, dv, cb, cdeg, a.ri, a.cw, hi);
+        warp_walk<SSSP_U, true>(x, st, v, dv, cb, cdeg, a.ri, a.cw, hi);
       }
     }
     ws_flush(st, x.qout, x.qlen_out, x.qcap, x.overflow);
@@ -606,25 +660,10 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
       for (int32_t ch = gw; ch < nch; ch += nw) {
         const int2 e = __ldcg(a.chunks + ch);
         if (e.x < 0) continue;
-        const bool rev = e.y < 0;
-        const int32_t k0 = e.y & INT_MAX;
-        const int32_t *off = rev ? a.co : a.ro;
-        const int32_t *adj = rev ? a.ri : a.ci;
-        const int32_t *wt = rev ? a.cw : a.w;
-        const int32_t end = min(k0 + SSSP_CH, off[(e.x & a.vmask) + 1]);
-        const int32_t dv = vload(a.dist + e.x);
-        for (int32_t b = k0; b < end; b += 32 * SSSP_U) {
-          int32_t u[SSSP_U], w[SSSP_U], d[SSSP_U];
-#pragma unroll
-          for (int r = 0; r < SSSP_U; r++) {
-            const int32_t k = b + r * 32 + lane;
-            const bool in = k < end;
-            u[r] = in ? ((e.x & hi) | adj[k]) : -1;
-            w[r] = in ? (wt ? wt[k] : 1) : 0;
-            d[r] = dv;
-          }
-          relax_group(x, st, u, w, d);
-        }
+        SsspChunk h{e.x, e.y & INT_MAX, 0, 0, e.y < 0};
+        h.end = min(h.k0 + SSSP_CH, (h.rev ? a.co : a.ro)[(e.x & a.vmask) + 1]);
+        h.dv = vload(a.dist + e.x);
+        chunk_walk<SSSP_U, true>(x, st, a, h);
       }
       ws_flush(st, x.qout, x.qlen_out, x.qcap, x.overflow);
       if (!(ok = barrier(slot))) break;
@@ -868,7 +907,7 @@ __device__ void mss_level_end(const MssArgs &a) {
   if (over) c->status = MG_ERR_QUEUE_OVERFLOW;
   __threadfence();
   c->done = done ? 1 : 0;
-  if (a.use_cond) cudaGraphSetConditional(a.h, done ? 0u : 1u);
+  loop_signal(a.ctl, a.h, a.use_cond, done);
 }
 
 // Pass 1: each warp reads 32 frontier items' headers (one per lane), cuts the
@@ -1003,7 +1042,7 @@ __global__ void __launch_bounds__(SSSP_NT) mss_compact_kernel(MssArgs a, int64_t
   __shared__ int32_t s_base;
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
@@ -1177,6 +1216,16 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
       delta = (int32_t)std::max(1.0, std::min(1e9, std::round(8.0 * g->mean_weight)));
     }
   }
+  // One cooperative launch for all rounds where a CTA of it fits every SM; the
+  // per-round kernels serve plain rounds of larger graphs (or counted ones), the
+  // CUDA-graph and the host-driven loop.
+  bool persist = o.use_graph == 0 && (delta > 0 || (o.iter_num <= 0 && g->m <= NF_PLAIN_M));
+  if (persist) {
+    int occ = 0;
+    persist = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sssp_persist_kernel, NF_NT, 0) == cudaSuccess && occ > 0;
+    cudaGetLastError();
+  }
+  const bool plain = persist && delta <= 0;
   const size_t far_items = delta > 0 ? (size_t)qcap : 0;
   // Chunk list: a round's heavy vertices hold at most (edges / SSSP_CH + vertices of
   // heavy_small edges or more) chunks; each instance's frontier holds a vertex once,
@@ -1208,7 +1257,8 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
   a.chunk_cap = chunk_cap;
   a.heavy = heavy;
   a.heavy_small = heavy_small;
-  a.delta = delta > 0 ? delta : 0;
+  a.delta = delta > 0 ? delta : plain ? 1 : 0;
+  a.plain = plain ? 1 : 0;
   a.far0 = delta > 0 ? cv.take<int32_t>(far_items) : nullptr;
   a.far1 = delta > 0 ? cv.take<int32_t>(far_items) : nullptr;
   a.infar = delta > 0 ? cv.take<uint32_t>(nwords) : nullptr;
@@ -1255,30 +1305,25 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
     SsspArgs b = a;
     b.h = h;
     b.use_cond = use_cond;
-    sssp_relax_kernel<<<grid, SSSP_NT, 0, st>>>(b);
-    sssp_chunk_kernel<<<grid, SSSP_NT, 0, st>>>(b);
-    if (b.delta <= 0) sssp_compact_kernel<<<cgrid, SSSP_NT, 0, st>>>(b);
-    if (b.delta > 0) {
+    if (b.delta <= 0) {
+      sssp_relax_kernel<false><<<grid, SSSP_NT, 0, st>>>(b);
+      sssp_chunk_kernel<false><<<grid, SSSP_NT, 0, st>>>(b);
+      sssp_compact_kernel<<<cgrid, SSSP_NT, 0, st>>>(b);
+    } else {
+      sssp_relax_kernel<true><<<grid, SSSP_NT, 0, st>>>(b);
+      sssp_chunk_kernel<true><<<grid, SSSP_NT, 0, st>>>(b);
       sssp_far_min_kernel<<<grid, SSSP_NT, 0, st>>>(b);
       sssp_far_split_kernel<<<grid, SSSP_NT, 0, st>>>(b);
     }
   };
-  // Near-far rounds in one cooperative launch where a CTA of it fits every SM; the
-  // per-round kernels serve plain rounds and the host-driven loop.
-  bool persist = false;
-  if (a.delta > 0 && o.use_graph >= 0) {
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sssp_persist_kernel, NF_NT, 0) == cudaSuccess && occ > 0) {
-      SsspArgs pa = a;
-      void *params[] = {&pa};
-      persist = cudaLaunchCooperativeKernel((const void *)sssp_persist_kernel, dim3(g->num_sms), dim3(NF_NT), params, 0,
-                                            s) == cudaSuccess;
-    }
-    cudaGetLastError();
-  }
-  if (!persist)
+  if (persist) {
+    SsspArgs pa = a;
+    void *params[] = {&pa};
+    MG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)sssp_persist_kernel, dim3(g->num_sms), dim3(NF_NT), params, 0, s));
+  } else {
     MG_TRY(run_loop(g, vmask == -1 ? SLOT_SSSP : SLOT_BSSSP, &sig, sizeof(sig), o.use_graph, body,
                     (int64_t)iter_cap + 2));
+  }
   sssp_reach_kernel<<<g->num_sms * 4, 256, 0, s>>>(dist, nitems, vmask, g->ro, g->ctl);
   MG_CUDA_TRY(cudaGetLastError());
   MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
@@ -1293,9 +1338,9 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     stats->kernel_ms = ms;
-    const int64_t per = a.delta > 0 ? 4 : 3;
+    const int64_t per = delta > 0 ? 4 : 3;
     stats->launches = 3 + (persist ? 1 : loop_launches(g, per));
-    stats->status_detail = a.delta > 0 ? a.delta : 0;
+    stats->status_detail = delta > 0 ? delta : 0;
   }
   if (hc.status == MG_ERR_TIMEOUT) {
     mg_set_error("mg_sssp: a grid barrier of the near-far rounds timed out");
