@@ -831,24 +831,67 @@ struct MssArgs {
   int32_t use_cond;
 };
 
-// Relaxes edges [k0, k1) of adj/wt from the vertex whose row this lane's instance
-// reads as dv (act: the lane's instance improved that vertex last round). An edge
-// that improves on the distance read before the atomicMin sets the instance's bit
-// in the head's next mask; neither atomic's old value is waited for (the frontier
-// is compacted from the masks after the round), so a warp keeps one memory round
-// trip per MSS_U edges. A bit set by an improvement that a concurrent smaller one
-// overtook only re-expands that vertex once more.
+// Relaxes MSS_U staged edges (head, weight) from the vertex whose row this lane's
+// instance reads as dv (act: the lane's instance improved that vertex last round;
+// INT_MAX otherwise). Dl: this lane's column of the group's distance rows, mg: the
+// group's next masks. An edge that improves on the distance read before the atomicMin
+// sets the instance's bit in the head's next mask; neither atomic's old value is
+// waited for (the frontier is compacted from the masks after the round). A bit set by
+// an improvement that a concurrent smaller one overtook only re-expands that vertex
+// once more.
 //
-// The edges are staged MSS_CH at a time in the warp's shared buffer `se` as
-// (head, weight) pairs, read back two per 16-byte broadcast load; slots past the
-// end hold (0, INT_MAX), an edge that can never improve a distance. Inactive lanes
-// compare against 0. Every lane of the warp calls it with the same edge range.
+// The traffic of the rows from the L2 bounds it (5.1 TB/s on the chunks of R-MAT s19),
+// with 17 instructions per edge next to it. Most edges improve nothing: the first look
+// goes through L1 (an older, larger distance there only costs the second look), one
+// vote covers the MSS_U edges, and only if it passes are they looked at in the L2 and
+// voted on one by one.
+__device__ __forceinline__ void mss_step(const int2 *se, int32_t *Dl, uint32_t *mg, bool act, uint32_t dv,
+                                         int64_t &updates) {
+  int32_t u[MSS_U];
+  uint32_t nd[MSS_U], cu[MSS_U];
+#pragma unroll
+  for (int r = 0; r < MSS_U; r += 2) {
+    const int4 p = *reinterpret_cast<const int4 *>(se + r);
+    u[r] = p.x;
+    nd[r] = dv + (uint32_t)p.y;  // below 2^32; an improvement is below INT_MAX
+    u[r + 1] = p.z;
+    nd[r + 1] = dv + (uint32_t)p.w;
+  }
+#pragma unroll
+  for (int r = 0; r < MSS_U; r++) cu[r] = act ? (uint32_t)__ldca(Dl + ((uint32_t)u[r] << 5)) : 0u;
+  bool any = false;
+#pragma unroll
+  for (int r = 0; r < MSS_U; r++) any |= nd[r] < cu[r];
+  if (!__any_sync(FULL, any)) return;
+#pragma unroll
+  for (int r = 0; r < MSS_U; r++) cu[r] = nd[r] < cu[r] ? (uint32_t)__ldcg(Dl + ((uint32_t)u[r] << 5)) : 0u;
+  uint32_t myb = 0;
+  int32_t myv = 0;
+#pragma unroll
+  for (int r = 0; r < MSS_U; r++) {
+    const bool tr = nd[r] < cu[r];
+    if (tr) red_min(Dl + ((uint32_t)u[r] << 5), (int32_t)nd[r]);
+    const uint32_t bits = __ballot_sync(FULL, tr);
+    if (lane_id() == r) {
+      myb = bits;
+      myv = u[r];
+    }
+  }
+  if (myb) {
+    updates += __popc(myb);
+    red_or(mg + myv, myb);
+  }
+}
+
+// Edges [k0, k1) of adj/wt, staged MSS_CH at a time in the warp's shared buffer `se`
+// as (head, weight) pairs, read back two per 16-byte broadcast load; slots past the
+// end hold (0, INT_MAX), an edge that can never improve a distance. Every lane of the
+// warp calls it with the same edge range.
 __device__ __forceinline__ void mss_edges(const MssArgs &a, int2 *se, uint32_t *mnext, int64_t gbase, bool act,
                                           int32_t dv, const int32_t *__restrict__ adj,
                                           const int32_t *__restrict__ wt, int32_t k0, int32_t k1, int64_t &updates) {
   const int lane = lane_id();
-  int32_t *Dl = a.D + (gbase << 5) + lane;  // this lane's column of the group's rows
-  uint32_t *mg = mnext + gbase;
+  int32_t *Dl = a.D + (gbase << 5) + lane;
   for (int32_t b = k0; b < k1; b += MSS_CH) {
     const int32_t cnt = min(MSS_CH, k1 - b);
 #pragma unroll
@@ -857,36 +900,7 @@ __device__ __forceinline__ void mss_edges(const MssArgs &a, int2 *se, uint32_t *
       se[j] = j < cnt ? make_int2(adj[b + j], wt ? wt[b + j] : 1) : make_int2(0, INT_MAX);
     }
     __syncwarp();
-    for (int32_t e0 = 0; e0 < cnt; e0 += MSS_U) {
-      int32_t u[MSS_U], w[MSS_U], cu[MSS_U];
-#pragma unroll
-      for (int r = 0; r < MSS_U; r += 2) {
-        const int4 p = *reinterpret_cast<const int4 *>(se + e0 + r);
-        u[r] = p.x;
-        w[r] = p.y;
-        u[r + 1] = p.z;
-        w[r + 1] = p.w;
-      }
-#pragma unroll
-      for (int r = 0; r < MSS_U; r++) cu[r] = act ? __ldcg(Dl + ((uint32_t)u[r] << 5)) : 0;
-      uint32_t myb = 0;
-      int32_t myv = 0;
-#pragma unroll
-      for (int r = 0; r < MSS_U; r++) {
-        const int32_t nd = (int32_t)min((uint32_t)dv + (uint32_t)w[r], (uint32_t)INT_MAX);
-        const bool tr = nd < cu[r];
-        if (tr) red_min(Dl + ((uint32_t)u[r] << 5), nd);
-        const uint32_t bits = __ballot_sync(FULL, tr);
-        if (lane == r) {
-          myb = bits;
-          myv = u[r];
-        }
-      }
-      if (myb) {
-        updates += __popc(myb);
-        red_or(mg + myv, myb);
-      }
-    }
+    for (int32_t e0 = 0; e0 < cnt; e0 += MSS_U) mss_step(se + e0, Dl, mnext + gbase, act, (uint32_t)dv, updates);
     __syncwarp();
   }
 }
@@ -917,7 +931,7 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_relax_kernel(MssArgs a) {
   __shared__ int64_t s_sum[SSSP_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
@@ -979,7 +993,40 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_relax_kernel(MssArgs a) {
         else deg = 0;
       }
     }
-    // light items, one at a time by the whole warp
+    // Items of up to 32 edges, four at a time: their rows' and their edges' loads are
+    // issued together (one at a time, a warp waited for two round trips per item).
+    unsigned few = __ballot_sync(FULL, deg > 0 && deg <= 32 && cdeg == 0);
+    while (few) {
+      int32_t sit[4], sd[4];
+      int32_t dv[4];
+      uint32_t sm[4];
+      int2 *se = s_edges[warp_id()];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int j = few ? __ffs(few) - 1 : 0;
+        const bool have = few != 0;
+        few &= few - 1;
+        sit[q] = __shfl_sync(FULL, it, j);
+        sm[q] = __shfl_sync(FULL, mask, j);
+        const int64_t srow = __shfl_sync(FULL, row, j);
+        const int32_t sb = __shfl_sync(FULL, beg, j);
+        const int32_t d = __shfl_sync(FULL, deg, j);
+        sd[q] = have ? d : 0;
+        dv[q] = have && ((sm[q] >> lane) & 1u) ? __ldcg(a.D + (srow << 5) + lane) : INT_MAX;
+        const bool in = lane < sd[q];
+        se[q * 32 + lane] = make_int2(in ? a.ci[sb + lane] : 0, in ? (a.w ? a.w[sb + lane] : 1) : INT_MAX);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int64_t gbase = (int64_t)(sit[q] >> a.shift) * a.n;
+        for (int32_t e0 = 0; e0 < sd[q]; e0 += MSS_U)
+          mss_step(se + q * 32 + e0, a.D + (gbase << 5) + lane, mnext + gbase, (sm[q] >> lane) & 1u, (uint32_t)dv[q], upd);
+      }
+      __syncwarp();
+    }
+    if (deg <= 32 && cdeg == 0) deg = 0;
+    // the others one at a time by the whole warp
     unsigned todo = __ballot_sync(FULL, deg + cdeg > 0);
     while (todo) {
       const int j = __ffs(todo) - 1;
@@ -1008,7 +1055,7 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_chunk_kernel(MssArgs a) {
   __shared__ int64_t s_sum[SSSP_NT / 32 + 1];
   DevCtl *c = a.ctl;
   if (vload(&c->done)) {
-    if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.h, 0u);
+    loop_over(a.ctl, a.h, a.use_cond);
     return;
   }
   const int cur = vload(&c->cur);
@@ -1017,18 +1064,31 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_chunk_kernel(MssArgs a) {
   int64_t upd = 0;
   const int32_t nch = min(vload(&c->big_len), a.chunk_cap);
   const int32_t nw = gridDim.x * (SSSP_NT / 32);
-  for (int32_t ch = blockIdx.x * (SSSP_NT / 32) + warp_id(); ch < nch; ch += nw) {
-    const int4 e = a.chunks[ch];
-    if (e.x < 0) continue;
-    const bool rev = e.y < 0;
-    const int32_t k0 = e.y & INT_MAX;
+  // the next chunk's header and row are on their way while this one is relaxed
+  auto header = [&](int32_t ch) { return ch < nch ? a.chunks[ch] : make_int4(-1, 0, 0, 0); };
+  auto open = [&](const int4 &e, int32_t &end, int32_t &dv) {
+    end = 0;
+    dv = INT_MAX;
+    if (e.x < 0) return;
     const int32_t v = e.x & a.vmask;
-    const int64_t gbase = (int64_t)(e.x >> a.shift) * a.n;
-    const int32_t *off = rev ? a.co : a.ro;
-    const int32_t end = min(k0 + MSS_CH, off[v + 1]);
-    const bool act = ((uint32_t)e.z >> lane) & 1u;
-    const int32_t dv = act ? __ldcg(a.D + ((gbase + v) << 5) + lane) : INT_MAX;
-    mss_edges(a, s_edges[warp_id()], mnext, gbase, act, dv, rev ? a.ri : a.ci, rev ? a.cw : a.w, k0, end, upd);
+    end = min((e.y & INT_MAX) + MSS_CH, (e.y < 0 ? a.co : a.ro)[v + 1]);
+    if (((uint32_t)e.z >> lane) & 1u) dv = __ldcg(a.D + (((int64_t)(e.x >> a.shift) * a.n + v) << 5) + lane);
+  };
+  int32_t ch = blockIdx.x * (SSSP_NT / 32) + warp_id();
+  int4 e = header(ch), e1 = header(ch + nw);
+  int32_t end, dv;
+  open(e, end, dv);
+  for (; ch < nch; ch += nw) {
+    int32_t end1, dv1;
+    open(e1, end1, dv1);
+    const int4 e2 = header(ch + 2 * nw);
+    const bool rev = e.y < 0;
+    mss_edges(a, s_edges[warp_id()], mnext, (int64_t)(e.x >> a.shift) * a.n, ((uint32_t)e.z >> lane) & 1u, dv,
+              rev ? a.ri : a.ci, rev ? a.cw : a.w, e.y & INT_MAX, end, upd);  // an empty slot has no edges
+    e = e1;
+    e1 = e2;
+    end = end1;
+    dv = dv1;
   }
   sssp_counters(c, s_sum, 0, 0, 0, upd);
 }
