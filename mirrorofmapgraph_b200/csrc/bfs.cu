@@ -147,18 +147,32 @@ __device__ void bfs_level_end(const BfsArgs &a) {
   loop_signal(a.ctl, a.h, a.use_cond, done);
 }
 
-// Early exit shared by both kernels: when the run is already over, make sure
-// the WHILE node stops.
-__device__ __forceinline__ bool bfs_skip(const BfsArgs &a, int want_dir) {
-  DevCtl *c = a.ctl;
-  if (vload(&c->done)) {
-    loop_over(a.ctl, a.h, a.use_cond);
-    return true;
-  }
-  return vload(&c->dir) != want_dir;
-}
+// What a level kernel reads from the control block: by one thread per block, since
+// every warp of the grid reading one L2 sector queues for microseconds (more than an
+// empty kernel takes otherwise).
+struct BfsEnter {
+  int32_t skip, cur, nin, level;
+  uint32_t *vis, *vis_out;  // the visited bitmap as the level found it, and the one it writes
+};
 
-__device__ __forceinline__ uint32_t *bfs_vis(const BfsArgs &a) { return vload(&a.ctl->vsel) ? a.vis2 : a.vis; }
+// Early exit shared by the level kernels: true if the run is over (then it makes sure
+// the loop stops) or the level goes the other way. Every thread of the block calls it.
+__device__ __forceinline__ bool bfs_skip(const BfsArgs &a, int want_dir, BfsEnter &en) {
+  DevCtl *c = a.ctl;
+  if (threadIdx.x == 0) {
+    const int32_t done = vload(&c->done), dir = vload(&c->dir), cur = vload(&c->cur), vsel = vload(&c->vsel);
+    en.level = vload(&c->level);
+    const int32_t q0 = vload(&c->qlen[0]), q1 = vload(&c->qlen[1]);
+    en.cur = cur;
+    en.nin = cur ? q1 : q0;
+    en.vis = vsel ? a.vis2 : a.vis;
+    en.vis_out = a.vis2 ? (vsel ? a.vis : a.vis2) : a.vis;
+    en.skip = done || dir != want_dir;
+    if (done) loop_over(a.ctl, a.h, a.use_cond);
+  }
+  __syncthreads();
+  return en.skip != 0;
+}
 
 // Per-thread state of a push level (plain copies, so nothing is read through
 // the kernel-parameter block).
@@ -194,13 +208,13 @@ __global__ void __launch_bounds__(BFS_NT) bfs_push_kernel(BfsArgs a) {
   __shared__ ExpandSmem<BFS_NT> sm;
   __shared__ BlockQueue bq;
   __shared__ int64_t s_sum[BFS_NT / 32 + 1];
-  if (bfs_skip(a, 0)) return;
+  __shared__ BfsEnter en;
+  if (bfs_skip(a, 0, en)) return;
   DevCtl *c = a.ctl;
-  const int cur = vload(&c->cur);
-  const int32_t nin = vload(&c->qlen[cur]);
+  const int cur = en.cur;
+  const int32_t nin = en.nin;
   const int32_t *qin = cur ? a.q1 : a.q0;
-  uint32_t *vis = bfs_vis(a);
-  PushCtx x{a.label, vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, vload(&c->level), 0};
+  PushCtx x{a.label, en.vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, en.level, 0};
   bq_init(bq);
   x.bq = &bq;
   int64_t insp = 0, nexp = 0;
@@ -246,17 +260,66 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
   } sm;
   __shared__ BlockQueue bq;
   __shared__ int64_t s_sum[BFS_NT / 32 + 1];
+  // Read by one thread per block (at entry, and behind each barrier): every warp of
+  // the grid reading one L2 sector queues for microseconds.
+  __shared__ struct {
+    int32_t lvl, sel, nin, cap, skip, pq, pb, over, ok;
+    int64_t mf, vdeg, pm;
+    uint32_t *vis;
+  } s_c;
   DevCtl *c = a.ctl;
+  unsigned gen = 0;  // thread 0: the barrier's generation, moved by nobody else's arrival alone
   // Entry state, as the seed kernel or the last per-level kernel left it; every
   // block reads the same values and then takes the same decisions level by level.
-  const int32_t l0 = vload(&c->level);
-  int32_t lvl = l0, sel = vload(&c->cur);
-  int32_t nin = vload(&c->qlen[sel]);
-  int64_t mf = vload(&c->mf_front), vdeg = vload(&c->visited_deg);
-  const int32_t iter_cap = vload(&c->iter_cap);
-  if (vload(&c->done) || vload(&c->dir) != 0 || nin > a.persist_max || mf > a.persist_edges) return;
+  if (threadIdx.x == 0) {
+    gen = vload(&c->bar_gen);
+    const int32_t done = vload(&c->done), dir = vload(&c->dir), q0 = vload(&c->qlen[0]), q1 = vload(&c->qlen[1]);
+    s_c.lvl = vload(&c->level);
+    s_c.sel = vload(&c->cur);
+    s_c.mf = vload(&c->mf_front);
+    s_c.vdeg = vload(&c->visited_deg);
+    s_c.cap = vload(&c->iter_cap);
+    s_c.vis = vload(&c->vsel) ? a.vis2 : a.vis;
+    s_c.nin = s_c.sel ? q1 : q0;
+    s_c.skip = done || dir != 0 || s_c.nin > a.persist_max || s_c.mf > a.persist_edges;
+  }
+  __syncthreads();
+  if (s_c.skip) return;
+  const int32_t l0 = s_c.lvl, iter_cap = s_c.cap;
+  int32_t lvl = l0, sel = s_c.sel, nin = s_c.nin;
+  int64_t mf = s_c.mf, vdeg = s_c.vdeg;
+  uint32_t *vis = s_c.vis;
+  // Grid barrier (bounded) that ends with the counters of slot `out` in s_c.
+  auto barrier = [&](int out) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int ok = 1;
+      __threadfence();
+      if (atomicAdd(&c->bar_count, 1u) + 1 == gridDim.x + a.bar_extra) {
+        c->bar_count = 0;
+        __threadfence();
+        atomicAdd(&c->bar_gen, 1u);
+      } else {
+        unsigned long long it = 0;
+        while (vload(&c->bar_gen) == gen) {
+          if (++it > a.bar_limit) {
+            ok = 0;
+            break;
+          }
+        }
+      }
+      gen++;
+      __threadfence();
+      s_c.pq = vload(&c->pq[out]);
+      s_c.pb = vload(&c->pb[out]);
+      s_c.pm = vload(&c->pm[out]);
+      s_c.over = vload(&c->overflow);
+      s_c.ok = ok;
+    }
+    __syncthreads();
+    return s_c.ok != 0;
+  };
   bq_init(bq);
-  uint32_t *vis = bfs_vis(a);
   for (;;) {
     // Per-level counters rotate over three slots: this level appends to `out`;
     // `zero` is the slot the next level appends to (nobody touches it now).
@@ -291,21 +354,21 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
       if (bins) atomicAdd((unsigned long long *)&c->edges_inspected, (unsigned long long)bins);
       if (bexp) atomicAdd((unsigned long long *)&c->vertices_expanded, (unsigned long long)bexp);
     }
-    if (!grid_barrier(&c->bar_count, &c->bar_gen, a.bar_limit, a.bar_extra)) {
+    if (!barrier(out)) {
       if (threadIdx.x == 0) {
         c->status = MG_ERR_TIMEOUT;
         c->done = 1;
       }
       return;
     }
-    if (vload(&c->pb[out]) > 0) {
+    if (s_c.pb > 0) {
       // The deferred vertices' edges, spread over the whole grid.
       x.mf = 0;
       expand_big<BFS_NT>(sm.b, a.ro, big, [&](int32_t, int32_t k) { bfs_visit(x, ci[k]); });
       bq_flush(bq, x.qout, x.qlen_out, x.qcap, x.overflow);
       const int64_t bmf2 = block_sum<BFS_NT>(x.mf, s_sum);
       if (threadIdx.x == 0 && bmf2) atomicAdd((unsigned long long *)&c->pm[out], (unsigned long long)bmf2);
-      if (!grid_barrier(&c->bar_count, &c->bar_gen, a.bar_limit, a.bar_extra)) {
+      if (!barrier(out)) {
         if (threadIdx.x == 0) {
           c->status = MG_ERR_TIMEOUT;
           c->done = 1;
@@ -315,12 +378,12 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
     }
     // Level end (bfs_level_end's rules), computed alike in every block.
     if (blockIdx.x == 0 && threadIdx.x == 0) trace_level(c, lvl, MG_DIR_PUSH, nin, mf, 0.0);
-    const int32_t nf = vload(&c->pq[out]);
-    mf = vload(&c->pm[out]);
+    const int32_t nf = s_c.pq;
+    mf = s_c.pm;
     vdeg += mf;
     lvl += 1;
     sel ^= 1;
-    const bool over = vload(&c->overflow) != 0;
+    const bool over = s_c.over != 0;
     const bool done = nf == 0 || lvl >= iter_cap || over;
     int dir = 0;
     if (a.mode == MG_DIR_PULL) dir = a.can_pull ? 1 : 0;
@@ -356,11 +419,11 @@ __global__ void __launch_bounds__(BFS_NT) bfs_push_big_kernel(BfsArgs a) {
   __shared__ BigSmem<BFS_NT> sm;
   __shared__ BlockQueue bq;
   __shared__ int64_t s_sum[BFS_NT / 32 + 1];
-  if (bfs_skip(a, 0)) return;
+  __shared__ BfsEnter en;
+  if (bfs_skip(a, 0, en)) return;
   DevCtl *c = a.ctl;
-  const int cur = vload(&c->cur);
-  uint32_t *vis = bfs_vis(a);
-  PushCtx x{a.label, vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, vload(&c->level), 0};
+  const int cur = en.cur;
+  PushCtx x{a.label, en.vis, a.ro, cur ? a.q0 : a.q1, &c->qlen[cur ^ 1], &c->overflow, a.qcap, en.level, 0};
   bq_init(bq);
   x.bq = &bq;
   const int32_t *ci = a.ci;
@@ -379,19 +442,20 @@ __global__ void __launch_bounds__(BFS_NT) bfs_push_big_kernel(BfsArgs a) {
 // of vertices of middling degree, a lane per vertex up to the longest row); and
 // discoveries are staged per warp (one queue atomic per word queued 130,000 of them on
 // one address). Largest level of R-MAT s22: 191 us one edge and one depth load at a
-// time, 136 us now.
+// time, 115 us now.
 // BITS: the test reads the bitmap the level found (else the depth, and the one bitmap
 // is updated in place).
 template <bool BITS>
 __global__ void __launch_bounds__(BFS_NT, 6) bfs_pull_kernel(BfsArgs a) {
   __shared__ int64_t s_sum[BFS_NT / 32 + 1];
   __shared__ int32_t s_stage[BFS_NT / 32][WS_CAP];
-  if (bfs_skip(a, 1)) return;
+  __shared__ BfsEnter en;
+  if (bfs_skip(a, 1, en)) return;
   DevCtl *c = a.ctl;
-  const int cur = vload(&c->cur);
-  const int32_t level = vload(&c->level);
-  const uint32_t *vis = bfs_vis(a);
-  uint32_t *vout = BITS ? (vload(&c->vsel) ? a.vis : a.vis2) : a.vis;
+  const int cur = en.cur;
+  const int32_t level = en.level;
+  const uint32_t *vis = en.vis;
+  uint32_t *vout = en.vis_out;
   int32_t *qout = cur ? a.q0 : a.q1;
   int32_t *qlen_out = &c->qlen[cur ^ 1];
   WarpStage st{s_stage[warp_id()], 0};
@@ -460,15 +524,13 @@ __global__ void __launch_bounds__(BFS_NT, 6) bfs_pull_kernel(BfsArgs a) {
         if (!f && e < en && e + 8 > b) f = sector(e, b, en);
         f = (__ballot_sync(FULL, f) & mine) != 0;
       }
-      // back to the vertices' lanes
-      for (int q = 0; q < 8 && pend; q++) {
-        const int t = __ffs(pend) - 1;
-        pend &= pend - 1;
-        const bool fq = __shfl_sync(FULL, f, 4 * q);
-        const bool more = __shfl_sync(FULL, en0 > en, 4 * q);
-        if (lane == t) found = fq;
-        if (!fq && more) far |= 1u << t;
-      }
+      // back to the vertices' lanes: the r-th waiting vertex was quad r's
+      const unsigned fq = __ballot_sync(FULL, f), mq = __ballot_sync(FULL, en0 > en);
+      const int r = 4 * __popc(pend & lanemask_lt());
+      const bool served = ((pend >> lane) & 1u) && r < 32;
+      if (served) found = (fq >> r) & 1u;
+      far |= __ballot_sync(FULL, served && !found && ((mq >> r) & 1u));
+      pend = __ballot_sync(FULL, ((pend >> lane) & 1u) && !served);
     }
     while (far) {
       const int l = __ffs(far) - 1;
