@@ -1991,8 +1991,7 @@ static mg_status pagerank_ppr(mg_graph *g, const float *tele_dev, int32_t nvec, 
                                    sizeof(float) * nw, sizeof(float) * ((size_t)n + 8), sizeof(double) * W,
                                    sizeof(double) * 2 * W * (size_t)gpart,
                                    sizeof(Comp) * W * (size_t)std::max<int64_t>(nchunks, 1),
-                                   sizeof(int32_t) * (size_t)(std::max<int64_t>(nheavy, 1) + 1),
-                                   sizeof(double) * 2 * W * (size_t)std::max<int64_t>(nheavy, 1),
+                                   sizeof(int32_t) * (size_t)(std::max<int64_t>(nheavy, 1) + 1), (size_t)n,
                                    out_is_device ? 0 : sizeof(float) * (size_t)kmax * n});
   MG_TRY(ws_reserve(g, g->ws_main, need));
   Carve cv(g->ws_main.ptr);
@@ -2009,13 +2008,15 @@ static mg_status pagerank_ppr(mg_graph *g, const float *tele_dev, int32_t nvec, 
   a.hpart = cv.take<Comp>((size_t)W * std::max<int64_t>(nchunks, 1));
   a.hcount = cv.take<int32_t>(std::max<int64_t>(nheavy, 1) + 1);
   a.grab = a.hcount + std::max<int64_t>(nheavy, 1);
-  a.hres = cv.take<double>(2 * (size_t)W * std::max<int64_t>(nheavy, 1));
+  uint8_t *tflag = cv.take<uint8_t>(n);
+  a.tflag = tflag;
   float *stage = out_is_device ? nullptr : cv.take<float>((size_t)kmax * n);
   a.off = g->co;
   a.idx = g->ri;
   a.wts = weighted ? (const float *)g->cvals : nullptr;
   a.rows = bins->rows;
   a.nlight = bins->boff[PRB_HUB];
+  a.nempty = bins->boff[1];
   a.hrows = bins->hrows;
   a.hbase = bins->hbase;
   a.nheavy = nheavy;
@@ -2044,7 +2045,8 @@ static mg_status pagerank_ppr(mg_graph *g, const float *tele_dev, int32_t nvec, 
   for (int32_t c0 = 0; c0 < nvec; c0 += kmax) {
     const int32_t k = std::min<int32_t>(kmax, nvec - c0);
     MG_CUDA_TRY(cudaEventRecord(g->ev0, s));
-    ppr_pack_kernel<<<tgrid, tblk, 0, s>>>(tele_dev ? tele_dev + (size_t)c0 * n : nullptr, k, n, W, tele);
+    MG_CUDA_TRY(cudaMemsetAsync(tflag, 0, (size_t)n, s));
+    ppr_pack_kernel<<<tgrid, tblk, 0, s>>>(tele_dev ? tele_dev + (size_t)c0 * n : nullptr, k, n, W, tele, tflag);
     MG_CUDA_TRY(cudaMemsetAsync(g->ctl, 0, sizeof(DevCtl), s));
     switch (vpl) {
       case 1: ppr_launch_init<1>(a, ginit, s); break;
@@ -2052,7 +2054,7 @@ static mg_status pagerank_ppr(mg_graph *g, const float *tele_dev, int32_t nvec, 
       case 4: ppr_launch_init<4>(a, ginit, s); break;
       default: ppr_launch_init<8>(a, ginit, s); break;
     }
-    ppr_init_reduce_kernel<<<1, 256, 0, s>>>(a, ginit);
+    ppr_init_reduce_kernel<<<(W + PPR_NT / 32 - 1) / (PPR_NT / 32), PPR_NT, 0, s>>>(a, ginit);
     MG_CUDA_TRY(cudaGetLastError());
     struct Sig {
       PprArgs a;

@@ -10,9 +10,13 @@
 // Per column the update is the single-vector one,
 //   x'_v = alpha (sum_u a_uv g_u + d t_v) + (1 - alpha) t_v,  g'_v = x'_v / s_v,
 // accumulated with compensated FP32 sums; the per-column L1 residual and dangling
-// mass are reduced in FP64 in a fixed order (per-CTA partials, per-hub
-// contributions, then the last CTA), and the loop stops when every column's
-// residual is below tol.
+// mass are reduced in FP64 (per-CTA partials, then the last CTA), and the loop stops
+// when every column's residual is below tol.
+//
+// The gathered rows bound it (R-MAT s20, 256 vectors: 34 GB per iteration), then the
+// rows' own traffic, 4 KB each at 256 vectors. Teleport vectors are sparse: a row
+// whose teleport entries are all 0 does not read them, and one that has no in-edges
+// either stays 0 and is not touched at all (38% of the rows of an R-MAT graph).
 #pragma once
 
 #include "common.cuh"
@@ -27,13 +31,13 @@ struct PprArgs {
   const int32_t *off, *idx;  // CSC (gathered adjacency)
   const float *wts;          // its edge weights (nullptr: unit)
   const int32_t *rows;       // non-hub rows of the bin plan (bins 0..5), plan order
-  int64_t nlight;
+  int64_t nlight, nempty;  // rows; the first nempty of them have no in-edges
+  const uint8_t *tflag;      // per row: some teleport entry of the group is not 0
   const int32_t *hrows, *hbase;  // hub rows and their first chunk
   int64_t nheavy, nchunks;
   int32_t *hcount;  // arrival counters of the hubs (nheavy)
   int32_t *grab;    // work-item counter of the dynamic schedule (reset by the last CTA)
   Comp *hpart;      // hub chunk partial sums (nchunks x W)
-  double *hres;     // per-hub FP64 contributions: residual (W) then dangling (W)
   const float *srow;  // s_u (0: dangling)
   const float *tele;  // n x W
   float *x0, *x1, *g0, *g1;  // n x W ping-pong
@@ -149,7 +153,9 @@ __device__ __forceinline__ void ppr_update(const PprArgs &a, int64_t row, const 
   const int64_t W = a.W;
   const double s = (double)__ldg(a.srow + row);
   float t[VPL], xold[VPL], xnew[VPL], gnew[VPL];
-  ppr_load<VPL>(a.tele + row * W, lane, t);
+#pragma unroll
+  for (int j = 0; j < VPL; j++) t[j] = 0.f;
+  if (a.tflag[row]) ppr_load<VPL>(a.tele + row * W, lane, t);
   ppr_load<VPL>(xo + row * W, lane, xold);
 #pragma unroll
   for (int j = 0; j < VPL; j++) {
@@ -175,13 +181,10 @@ __device__ void ppr_iteration_end(const PprArgs &a, int cur, double *s_max) {
   double mx = 0.0;
   for (int col = threadIdx.x; col < a.W; col += blockDim.x) {
     double r = 0.0, d = 0.0;
+#pragma unroll 8
     for (int b = 0; b < a.grid; b++) {
       r += __ldcg(a.part + (int64_t)b * 2 * a.W + col);
       d += __ldcg(a.part + (int64_t)b * 2 * a.W + a.W + col);
-    }
-    for (int64_t h = 0; h < a.nheavy; h++) {
-      r += __ldcg(a.hres + h * 2 * a.W + col);
-      d += __ldcg(a.hres + h * 2 * a.W + a.W + col);
     }
     a.dang[col] = d;
     mx = fmax(mx, r);
@@ -211,7 +214,7 @@ __device__ void ppr_iteration_end(const PprArgs &a, int cur, double *s_max) {
 // R-MAT s20, 256 vectors, 5.15 ms an iteration against 5.00); each warp takes the next
 // item from a shared counter, so faster SMs take more.
 template <int VPL, bool WEIGHTED>
-__global__ void __launch_bounds__(PPR_NT) ppr_iter_kernel(PprArgs a) {
+__global__ void __launch_bounds__(PPR_NT, VPL == 8 ? 2 : 1) ppr_iter_kernel(PprArgs a) {
   __shared__ double s_red[2][PPR_NT / 32][32 * VPL];
   __shared__ double s_max[PPR_NT];
   __shared__ int s_last;
@@ -233,8 +236,28 @@ __global__ void __launch_bounds__(PPR_NT) ppr_iter_kernel(PprArgs a) {
     rs[j] = 0.0;
     ds[j] = 0.0;
   }
-  const int64_t total = a.nchunks + a.nlight;
+  // a dangling mass that is no number makes every row of its column none
+  bool wild = false;
+#pragma unroll
+  for (int j = 0; j < VPL; j++) wild |= !isfinite(dj[j]);
+  wild = __any_sync(FULL, wild);
+  const int64_t nrows = a.nlight - a.nempty;
+  const int64_t total = a.nchunks + nrows + (a.nempty + 31) / 32;
   auto item = [&](int64_t it) {
+    if (it >= a.nchunks + nrows) {  // 32 rows without in-edges: those with a teleport entry
+      const int64_t i = (it - a.nchunks - nrows) * 32 + lane;
+      const int32_t mine = i < a.nempty ? a.rows[i] : -1;
+      unsigned todo = __ballot_sync(FULL, mine >= 0 && (wild || a.tflag[mine]));
+      Comp zero[VPL];
+#pragma unroll
+      for (int j = 0; j < VPL; j++) zero[j] = Comp{0.f, 0.f};
+      while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1;
+        ppr_update<VPL>(a, __shfl_sync(FULL, mine, l), zero, xo, xn, gn, dj, rs, ds);
+      }
+      return;
+    }
     Comp acc[VPL];
 #pragma unroll
     for (int j = 0; j < VPL; j++) acc[j] = Comp{0.f, 0.f};
@@ -280,20 +303,7 @@ __global__ void __launch_bounds__(PPR_NT) ppr_iter_kernel(PprArgs a) {
       }
     }
     if (lane == 0) a.hcount[lo] = 0;
-    double hr[VPL], hd[VPL];
-#pragma unroll
-    for (int j = 0; j < VPL; j++) {
-      hr[j] = 0.0;
-      hd[j] = 0.0;
-    }
-    ppr_update<VPL>(a, row, tot, xo, xn, gn, dj, hr, hd);
-    double *hc = a.hres + lo * 2 * (int64_t)a.W;
-#pragma unroll
-    for (int j = 0; j < VPL; j++) {
-      hc[ppr_col<VPL>(lane, j)] = hr[j];
-      hc[a.W + ppr_col<VPL>(lane, j)] = hd[j];
-    }
-    __threadfence();
+    ppr_update<VPL>(a, row, tot, xo, xn, gn, dj, rs, ds);
   };
   for (;;) {
     int64_t it = 0;
@@ -354,6 +364,10 @@ __global__ void __launch_bounds__(PPR_NT) ppr_init_kernel(PprArgs a) {
     }
     ppr_store<VPL>(a.x0 + v * W, lane, t);
     ppr_store<VPL>(a.g0 + v * W, lane, gv);
+    if (!a.tflag[v] && a.off[v] == a.off[v + 1]) {  // 0 in both buffers from now on
+      ppr_store<VPL>(a.x1 + v * W, lane, t);
+      ppr_store<VPL>(a.g1 + v * W, lane, t);
+    }
   }
 #pragma unroll
   for (int j = 0; j < VPL; j++) s_red[warp][ppr_col<VPL>(lane, j)] = ds[j];
@@ -365,14 +379,18 @@ __global__ void __launch_bounds__(PPR_NT) ppr_init_kernel(PprArgs a) {
   }
 }
 
-// dang[col] = sum of the init partials (fixed order); control block reset.
-__global__ void ppr_init_reduce_kernel(PprArgs a, int32_t nparts) {
-  for (int col = threadIdx.x; col < a.W; col += blockDim.x) {
+// dang[col] = sum of the init partials (fixed order: a warp per column); control
+// block reset.
+__global__ void __launch_bounds__(PPR_NT) ppr_init_reduce_kernel(PprArgs a, int32_t nparts) {
+  const int lane = threadIdx.x & 31;
+  const int col = blockIdx.x * (PPR_NT / 32) + (threadIdx.x >> 5);
+  if (col < a.W) {
     double d = 0.0;
-    for (int b = 0; b < nparts; b++) d += a.part[(int64_t)b * 2 * a.W + col];
-    a.dang[col] = d;
+    for (int b = lane; b < nparts; b += 32) d += a.part[(int64_t)b * 2 * a.W + col];
+    d = warp_sum(d);
+    if (lane == 0) a.dang[col] = d;
   }
-  if (threadIdx.x == 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     DevCtl *c = a.ctl;
     c->level = 0;
     c->cur = 0;
@@ -383,8 +401,10 @@ __global__ void ppr_init_reduce_kernel(PprArgs a, int32_t nparts) {
 }
 
 // Teleport rows (k x n, row i for column c0 + i; nullptr: uniform 1/n) into the
-// vertex-major n x W block; columns past k are 0.
-__global__ void ppr_pack_kernel(const float *__restrict__ src, int32_t k, int64_t n, int32_t W, float *__restrict__ dst) {
+// vertex-major n x W block; columns past k are 0. Sets the rows' teleport flags (0
+// before).
+__global__ void ppr_pack_kernel(const float *__restrict__ src, int32_t k, int64_t n, int32_t W, float *__restrict__ dst,
+                                uint8_t *__restrict__ tflag) {
   __shared__ float tile[32][33];
   const int64_t v0 = (int64_t)blockIdx.x * 32;
   const int c0 = blockIdx.y * 32;
@@ -398,7 +418,9 @@ __global__ void ppr_pack_kernel(const float *__restrict__ src, int32_t k, int64_
   __syncthreads();
   for (int r = threadIdx.y; r < 32; r += blockDim.y) {
     const int64_t v = v0 + r;
-    if (v < n) dst[v * W + c0 + threadIdx.x] = tile[threadIdx.x][r];
+    const float x = tile[threadIdx.x][r];
+    if (v < n) dst[v * W + c0 + threadIdx.x] = x;
+    if (__any_sync(FULL, x != 0.f) && threadIdx.x == 0 && v < n) tflag[v] = 1;
   }
 }
 
