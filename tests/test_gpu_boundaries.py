@@ -213,3 +213,18 @@ def test_loop_modes_agree():
             assert len({r[1]["iterations"] for r in res}) == 1
             for r in res[1:]:
                 assert np.abs(r[0] - res[0][0]).sum() <= 1e-9 * max(1.0, float(np.abs(res[0][0]).sum()))
+
+
+@pytest.mark.parametrize("n,m", [(300, 100), (300, 1200), (300, 1201), (20000, 10000), (20000, 20000), (20000, 60000),
+                                 (700000, 700000)])
+@pytest.mark.parametrize("sym", [False, True])
+def test_cc_sparse(n, m, sym):
+    """Trees and small cycles, on both sides of 4 edges per vertex."""
+    rng = np.random.default_rng(m)
+    src, dst = rng.integers(0, n, m), rng.integers(0, n, m)
+    if sym:
+        src, dst = np.concatenate([src, dst[: m // 2]])[:m], np.concatenate([dst, src[: m // 2]])[:m]
+        src, dst = np.concatenate([src[: m // 2], dst[: m // 2]]), np.concatenate([dst[: m // 2], src[: m // 2]])
+    ro, ci, _ = _csr(n, src, dst)
+    with mg.Graph(ro, ci, symmetric=sym) as g:
+        np.testing.assert_array_equal(g.cc()[0], oracle.cc(ro, ci))
