@@ -441,7 +441,20 @@ __device__ void solve_iteration_end(const SolveArgs &a, int cur, const double *h
       const double tl = vload(&c->dprev[1]) + vload(&c->dsum[2]);
       small = r < a.tol * c->dprev[2] && vload(&c->dsum[1]) < 0.36 * a.tol * a.tol * vload(&c->dprev[3]);
       c->dsum[1] = 0.0;
-      c->dsum[2] = a.alpha / (1.0 - a.alpha) * (d - tl);
+      // Near the end the change no longer falls faster than the constant would by itself
+      // (0.85 per iteration): either other parts are as slow, or what is left is FP32
+      // rounding, which a shift keeps stirring so that the iterates never settle
+      // (tolerances of 3e-8 and below ran to max_iter). No more shifts from there on
+      // (dsum[3] > 0). What the iterates settle on may be a cycle of two values an ulp
+      // apart (bipartite graphs): the change is then the same every time, and after four
+      // such iterations the solve is over.
+      const double rp = vload(&c->dsum[0]);
+      double end = vload(&c->dsum[3]);
+      if (end > 0.0) end = fabs(r - rp) <= 1e-9 * r ? end + 1.0 : 1.0;
+      else if (lvl > 1 && r < 1e-5 * c->dprev[2] && r > 0.8 * rp) end = 1.0;
+      c->dsum[3] = end;
+      small = small || end >= 5.0;
+      c->dsum[2] = end > 0.0 ? 0.0 : a.alpha / (1.0 - a.alpha) * (d - tl);
     }
     c->level = lvl;
     c->dsum[0] = r;

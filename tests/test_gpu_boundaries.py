@@ -228,3 +228,65 @@ def test_cc_sparse(n, m, sym):
     ro, ci, _ = _csr(n, src, dst)
     with mg.Graph(ro, ci, symmetric=sym) as g:
         np.testing.assert_array_equal(g.cc()[0], oracle.cc(ro, ci))
+
+
+@pytest.mark.parametrize("shape", ["cut", "sinks", "cycle2"])
+@pytest.mark.parametrize("teleport", [False, True])
+def test_adjoint_settles(shape, teleport):
+    """The adjoint solve shifts by a constant each iteration, exact whatever the graph: closed parts,
+    rows without edges, a slow alternating mode, a sparse right-hand side. It settles at any tolerance."""
+    rng = np.random.default_rng(5)
+    n = 1500
+    if shape == "cut":  # two halves without an edge between them
+        src = rng.integers(0, n // 2, 9000)
+        dst = rng.integers(0, n // 2, 9000)
+        src[::2] += n // 2
+        dst[::2] += n // 2
+    elif shape == "sinks":  # a third of the vertices without out-edges
+        src, dst = rng.integers(0, 2 * n // 3, 6000), rng.integers(0, n, 6000)
+    else:  # bipartite
+        src, dst = rng.integers(0, n // 2, 4000), rng.integers(n // 2, n, 4000)
+        src, dst = np.concatenate([src, dst]), np.concatenate([dst, src])
+    ro, ci, w = _csr(n, src, dst, rng.lognormal(0, 1, src.size).astype(np.float32))
+    t = None
+    if teleport:
+        t = np.zeros(n)
+        t[rng.integers(0, n, 7)] = 1.0
+        t /= t.sum()
+    dl = np.zeros(n)
+    dl[rng.integers(0, n, 5)] = rng.standard_normal(5) + 3
+    x, _, _ = oracle.pr_normalized(ro, ci, w, 0.85, 1e-15, 5000, t)
+    rw, rt, _, _ = oracle.pr_adjoint(ro, ci, w, x, dl, teleport=t)
+    with mg.Graph(ro, ci, w) as g:
+        for gather in ("binned", "cached"):
+            gw, gt, st = g.pagerank_backward(x.astype(np.float32), dl.astype(np.float32),
+                                             teleport=None if t is None else t.astype(np.float32), weighted=True,
+                                             tol=1e-8, max_iter=400, gather=gather)
+            assert st["iterations"] < 400
+            # 1e-8 relative over 1 - alpha, with FP32 ranks, iterates and results
+            assert np.linalg.norm(gt - rt) <= 2e-6 * np.linalg.norm(rt)
+            assert np.linalg.norm(gw - rw) <= 2e-6 * np.linalg.norm(rw) + 1e-12
+
+
+@pytest.mark.parametrize("nvec", [2, 32, 33, 70])
+def test_batched_ranks_sparse_rows(nvec):
+    """Rows with and without in-edges, with and without teleport entries, in every pairing."""
+    rng = np.random.default_rng(nvec)
+    n, m = 3001, 9000
+    src, dst = rng.integers(0, n, m), rng.integers(0, n // 3, m)  # two thirds of the rows have no in-edge
+    ro, ci, w = _csr(n, src, dst, rng.lognormal(0, 1, m).astype(np.float32))
+    tele = np.zeros((nvec, n), dtype=np.float32)
+    for k in range(nvec):
+        s = rng.integers(0, n, 1 + k % 5)
+        np.add.at(tele[k], s, np.float32(1.0 / s.size))
+    tele[0] = 1.0 / n
+    with mg.Graph(ro, ci, w) as g:
+        xs, st = g.pagerank(teleport=tele, nvec=nvec, mode="normalized", weighted=True)
+        ys, _ = g.pagerank(teleport=tele, nvec=nvec, mode="normalized", weighted=True)  # over the first run's state
+        for k in range(nvec):
+            xr, _, _ = oracle.pr_normalized(ro, ci, w, 0.85, 0.0, st["iterations"], tele[k].astype(np.float64))
+            assert np.abs(xs[k] - xr).sum() <= L1_TOL
+            assert np.abs(ys[k] - xr).sum() <= L1_TOL
+        tele[1, n - 1] = np.inf
+        zs, st = g.pagerank(teleport=tele, nvec=nvec, mode="normalized", weighted=True, max_iter=5)
+        assert np.isfinite(zs[0]).all() and not np.isfinite(zs[1]).all()
