@@ -152,6 +152,7 @@ __device__ void bfs_level_end(const BfsArgs &a) {
 // empty kernel takes otherwise).
 struct BfsEnter {
   int32_t skip, cur, nin, level;
+  int64_t mf;
   uint32_t *vis, *vis_out;  // the visited bitmap as the level found it, and the one it writes
 };
 
@@ -165,6 +166,7 @@ __device__ __forceinline__ bool bfs_skip(const BfsArgs &a, int want_dir, BfsEnte
     const int32_t q0 = vload(&c->qlen[0]), q1 = vload(&c->qlen[1]);
     en.cur = cur;
     en.nin = cur ? q1 : q0;
+    en.mf = vload(&c->mf_front);
     en.vis = vsel ? a.vis2 : a.vis;
     en.vis_out = a.vis2 ? (vsel ? a.vis : a.vis2) : a.vis;
     en.skip = done || dir != want_dir;
@@ -219,9 +221,10 @@ __global__ void __launch_bounds__(BFS_NT) bfs_push_kernel(BfsArgs a) {
   x.bq = &bq;
   int64_t insp = 0, nexp = 0;
   const BigList big{a.big_v, &c->big_len, defer_threshold<BFS_NT>(nin, a.cta_th, a.grid_th, a.defer_warp)};
-  for (int64_t tile = (int64_t)blockIdx.x * BFS_NT; tile < nin; tile += (int64_t)gridDim.x * BFS_NT) {
-    const int64_t i = tile + threadIdx.x;
-    const int32_t v = i < nin ? qin[i] : -1;
+  const int tl = tile_lanes<BFS_NT>(nin, en.mf), tn = tl * (BFS_NT / 32);
+  for (int64_t tile = (int64_t)blockIdx.x * tn; tile < nin; tile += (int64_t)gridDim.x * tn) {
+    const int64_t i = tile + warp_id() * tl + lane_id();
+    const int32_t v = lane_id() < tl && i < nin ? qin[i] : -1;
     nexp += v >= 0;
     const int32_t *ci = a.ci, *ri = a.ri;
     expand_tile<BFS_NT, BFS_CTA_TH>(sm, a.ro, v, insp, [&](int32_t, int32_t k) { bfs_visit(x, ci[k]); }, &big, -1,
@@ -335,9 +338,10 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
     const BigList big{a.big_v, &c->pb[out], defer_threshold<BFS_NT>(nin, a.cta_th, a.grid_th, a.defer_warp)};
     const int32_t *ci = a.ci, *ri = a.ri;
     int64_t insp = 0, nexp = 0;
-    for (int64_t tile = (int64_t)blockIdx.x * BFS_NT; tile < nin; tile += (int64_t)gridDim.x * BFS_NT) {
-      const int64_t i = tile + threadIdx.x;
-      const int32_t v = i < nin ? qin[i] : -1;
+    const int tl = tile_lanes<BFS_NT>(nin, mf), tn = tl * (BFS_NT / 32);
+    for (int64_t tile = (int64_t)blockIdx.x * tn; tile < nin; tile += (int64_t)gridDim.x * tn) {
+      const int64_t i = tile + warp_id() * tl + lane_id();
+      const int32_t v = lane_id() < tl && i < nin ? qin[i] : -1;
       nexp += v >= 0;
       expand_tile<BFS_NT, BFS_CTA_TH>(sm.e, a.ro, v, insp, [&](int32_t, int32_t k) { bfs_visit(x, ci[k]); }, &big,
                                       -1, a.cta_th);

@@ -230,6 +230,61 @@ def test_cc_sparse(n, m, sym):
         np.testing.assert_array_equal(g.cc()[0], oracle.cc(ro, ci))
 
 
+@pytest.mark.parametrize("wide,deg", [(37, 9000), (5000, 40), (5000, 200), (40000, 20)])
+def test_bfs_skewed_frontier(wide, deg):
+    """A sparse graph whose second level holds most of the edges: few vertices per warp,
+    hubs beyond the deferral list's 4096, and full tiles."""
+    rng = np.random.default_rng(wide)
+    n = max(1 << 18, wide * deg // 6)
+    src = np.concatenate([np.zeros(wide, np.int64), np.repeat(np.arange(1, wide + 1), deg)])
+    dst = np.concatenate([np.arange(1, wide + 1), rng.integers(0, n, wide * deg)])
+    ro, ci, _ = _csr(n, src, dst)
+    ref = oracle.bfs(ro, ci, [0])
+    with mg.Graph(ro, ci) as g:
+        for mode in (True, False):
+            d, st = g.bfs([0], use_graph=mode)
+            np.testing.assert_array_equal(d, ref)
+            assert st["edges_traversed"] == int(np.diff(ro)[ref >= 0].sum())
+        np.testing.assert_array_equal(g.bfs([0], direction="push")[0], ref)
+        np.testing.assert_array_equal(g.bfs_batch([0, 1], direction="push")[0][0], ref)
+
+
+@pytest.mark.parametrize("n", [33, 8191, 140001])
+def test_bottom_up_degrees(n):
+    """In-degrees at the ends of the shares of a bottom-up level: one lane, four, the warp; with and
+    without a parent in the last edge."""
+    rng = np.random.default_rng(n)
+    degs = np.array([0, 1, 7, 8, 9, 10, 263, 264, 265, 266, 511, 512, 4097])
+    rows = np.arange(min(n - 2, 16 * degs.size)) + 1
+    indeg = degs[rng.integers(0, degs.size, rows.size)]
+    dst = np.repeat(rows, indeg)
+    src = np.full(dst.size, n - 1)  # a vertex nothing reaches
+    last = np.cumsum(indeg)[(indeg > 0) & (rng.random(rows.size) < 0.7)] - 1
+    src[last] = rng.integers(0, rows.size, last.size)  # its parent, in the row's last edge
+    pos = np.arange(dst.size)
+    order = np.lexsort((pos, src))
+    ro = np.searchsorted(src[order], np.arange(n + 1)).astype(np.int32)
+    ci = dst[order].astype(np.int32)
+    with mg.Graph(ro, ci) as g:
+        for srcs in ([0], [0, 5, n - 2], [n - 1]):
+            ref = oracle.bfs(ro, ci, srcs)
+            for kw in (dict(direction="pull"), dict(direction="pull", use_graph=False), dict()):
+                np.testing.assert_array_equal(g.bfs(srcs, **kw)[0], ref)
+        np.testing.assert_array_equal(g.bfs_batch([0, 5], direction="pull")[0][1], oracle.bfs(ro, ci, [5]))
+
+
+@pytest.mark.parametrize("m", [(1 << 22) - 1, 1 << 22, (1 << 22) + 1])
+def test_plain_sssp_one_launch_limit(m):
+    rng = np.random.default_rng(m & 7)
+    n = 300001
+    src, dst = rng.integers(0, n, m), rng.integers(0, n, m)
+    ro, ci, w = _csr(n, src, dst, rng.integers(0, 100, m).astype(np.int32))
+    ref = oracle.sssp(ro, ci, w, [3, 70000])
+    with mg.Graph(ro, ci, w) as g:
+        for kw in (dict(), dict(use_graph=False), dict(use_graph="graph"), dict(delta=64)):
+            np.testing.assert_array_equal(g.sssp([3, 70000], **kw)[0], ref)
+
+
 @pytest.mark.parametrize("shape", ["cut", "sinks", "cycle2"])
 @pytest.mark.parametrize("teleport", [False, True])
 def test_adjoint_settles(shape, teleport):
