@@ -37,6 +37,8 @@ namespace mg {
 constexpr int MS_NT = 256;
 constexpr int MS_CTA_TH = 512;
 constexpr int MS_WIDTH = 64;        // sources per bit-parallel group
+constexpr int MS_PLANES = 5;         // digits of the depths kept by vertex
+constexpr int MS_FV = 4;             // vertices a thread commits at a time
 constexpr int64_t MS_ALPHA = 14;    // bottom-up when the union frontier's out-edges exceed m / MS_ALPHA
 
 struct MsArgs {
@@ -47,6 +49,7 @@ struct MsArgs {
   int32_t qcap;
   int32_t *big_v;  // grid-strided bin (BIG_CAP vertices)
   int32_t *depth;  // the group's first depth row (k rows of n)
+  uint64_t *plane[MS_PLANES];  // depths by their binary digits, while the level is below 1 << MS_PLANES
   int64_t n, m_total;
   uint64_t full;   // mask of the group's sources
   int32_t mode, can_pull, both;
@@ -65,6 +68,7 @@ __device__ void ms_level_end(const MsArgs &a) {
   c->level = lvl;
   c->qlen[cur] = 0;
   c->cur = cur ^ 1;
+  c->mf_front = mf;
   c->mf_next = 0;
   c->blocks_done = 0;
   c->big_len = 0;
@@ -84,13 +88,86 @@ __device__ void ms_level_end(const MsArgs &a) {
   loop_signal(a.ctl, a.h, a.use_cond, done);
 }
 
-__device__ __forceinline__ bool ms_skip(const MsArgs &a, int want_dir) {
+// What a level kernel reads from the control block: by one thread per block, since
+// every warp of the grid reading one L2 sector queues for microseconds.
+struct MsEnter {
+  int32_t skip, cur, nin, level;
+  int64_t mf;
+};
+
+// Early exit of the level kernels: true if the run is over (then it makes sure the loop
+// stops) or the level goes the other way (want_dir -1: either way is right). Every
+// thread of the block calls it.
+__device__ __forceinline__ bool ms_skip(const MsArgs &a, int want_dir, MsEnter &en) {
   DevCtl *c = a.ctl;
-  if (vload(&c->done)) {
-    loop_over(a.ctl, a.h, a.use_cond);
-    return true;
+  if (threadIdx.x == 0) {
+    const int32_t done = vload(&c->done), dir = vload(&c->dir), cur = vload(&c->cur);
+    const int32_t q0 = vload(&c->qlen[0]), q1 = vload(&c->qlen[1]);
+    en.level = vload(&c->level);
+    en.mf = vload(&c->mf_front);
+    en.cur = cur;
+    en.nin = cur ? q1 : q0;
+    en.skip = done || (want_dir >= 0 && dir != want_dir);
+    if (done) loop_over(a.ctl, a.h, a.use_cond);
   }
-  return vload(&c->dir) != want_dir;
+  __syncthreads();
+  return en.skip != 0;
+}
+
+// Depths while the levels are few (fewer than 1 << MS_PLANES). A level that stores
+// its new depths writes each row in pieces, the sector of a row at several levels, and
+// the rows had to be set to -1 first: R-MAT s20, 64 sources, 268 MB of rows, clearing 43 us and most of
+// the finishing passes.
+// Instead digit b of a vertex's 64 depths is kept in one word, plane[b][v]; a level
+// ORs its new bits into the planes of its own digits, and the rows are written once,
+// complete, at the end of the run (or at level 1 << MS_PLANES, from where on
+// ms_write_depths stores them): 56 us.
+__device__ __forceinline__ void ms_plane(const MsArgs &a, int64_t w, uint64_t nw, int32_t d) {
+#pragma unroll
+  for (int b = 0; b < MS_PLANES; b++) {
+    if (d == 1 << b) a.plane[b][w] = nw;  // first level with this digit: no other bit yet
+    else if (((d >> b) & 1) && nw) a.plane[b][w] |= nw;
+  }
+}
+
+// The rows of vertex v, complete: reached (`seen`) sources' depths from the planes of
+// levels up to `top`, 1 << MS_PLANES for those in `nw`, -1 for the others. Sources
+// i, i + 8, i + 16, i + 24 are decoded at a time, a byte each.
+__device__ __forceinline__ void ms_emit_rows(const MsArgs &a, int64_t v, uint64_t seen, uint64_t nw, int32_t top) {
+  uint64_t pl[MS_PLANES];
+#pragma unroll
+  for (int b = 0; b < MS_PLANES; b++) pl[b] = top >> b ? __ldcs(a.plane[b] + v) : 0;
+  seen |= nw;
+  const int k = 64 - __clzll((long long)a.full);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const unsigned s = (unsigned)(seen >> (32 * h)), w = (unsigned)(nw >> (32 * h));
+    unsigned p[MS_PLANES];
+#pragma unroll
+    for (int b = 0; b < MS_PLANES; b++) p[b] = (unsigned)(pl[b] >> (32 * h));
+    const int kh = k - 32 * h;
+    int32_t *row = a.depth + (int64_t)(32 * h) * a.n + v;
+    for (int i = 0; i < 8 && i < kh; i++, row += a.n) {
+      unsigned x = ((w >> i) & 0x01010101u) << MS_PLANES;
+#pragma unroll
+      for (int b = 0; b < MS_PLANES; b++) x |= ((p[b] >> i) & 0x01010101u) << b;
+      x |= (~(s >> i) & 0x01010101u) * 0xffu;
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (i + 8 * j < kh) __stcs(row + 8 * j * a.n, (int32_t)(x << (24 - 8 * j)) >> 24);
+    }
+  }
+}
+
+// After the last level: the rows, unless level 1 << MS_PLANES wrote them.
+__global__ void __launch_bounds__(MS_NT) ms_rows_kernel(MsArgs a) {
+  __shared__ int32_t s_top;
+  if (threadIdx.x == 0) s_top = vload(&a.ctl->level);
+  __syncthreads();
+  const int32_t top = s_top;
+  if (top >= 1 << MS_PLANES) return;
+  for (int64_t v = (int64_t)blockIdx.x * MS_NT + threadIdx.x; v < a.n; v += (int64_t)gridDim.x * MS_NT)
+    ms_emit_rows(a, v, a.seen[v], 0, top);
 }
 
 // Writes depth d of every lane's vertex v for each source bit in its `nw`.
@@ -111,10 +188,11 @@ __device__ __forceinline__ void ms_write_depths(int32_t *depth, int64_t n, int64
 __global__ void __launch_bounds__(MS_NT) ms_push_kernel(MsArgs a) {
   __shared__ ExpandSmem<MS_NT, uint64_t> sm;
   __shared__ int64_t s_sum[MS_NT / 32 + 1];
-  if (ms_skip(a, 0)) return;
+  __shared__ MsEnter en;
+  if (ms_skip(a, 0, en)) return;
   DevCtl *c = a.ctl;
-  const int cur = vload(&c->cur);
-  const int32_t nin = vload(&c->qlen[cur]);
+  const int cur = en.cur;
+  const int32_t nin = en.nin;
   const int32_t *qin = cur ? a.q1 : a.q0;
   const uint64_t *fcur = cur ? a.f1 : a.f0;
   const uint64_t *seen = a.seen;
@@ -126,9 +204,10 @@ __global__ void __launch_bounds__(MS_NT) ms_push_kernel(MsArgs a) {
     const uint64_t add = f & ~__ldg(seen + w);
     if (add) atomicOr(acc + w, (unsigned long long)add);
   };
-  for (int64_t tile = (int64_t)blockIdx.x * MS_NT; tile < nin; tile += (int64_t)gridDim.x * MS_NT) {
-    const int64_t i = tile + threadIdx.x;
-    const int32_t v = i < nin ? qin[i] : -1;
+  const int tl = tile_lanes<MS_NT>(nin, en.mf), tn = tl * (MS_NT / 32);
+  for (int64_t tile = (int64_t)blockIdx.x * tn; tile < nin; tile += (int64_t)gridDim.x * tn) {
+    const int64_t i = tile + warp_id() * tl + lane_id();
+    const int32_t v = lane_id() < tl && i < nin ? qin[i] : -1;
     nexp += v >= 0;
     const uint64_t f = v >= 0 ? __ldg(fcur + v) : 0;  // the sender's frontier mask, once per vertex
     expand_tile_p<MS_NT, MS_CTA_TH>(sm, a.ro, v, f, insp,
@@ -149,9 +228,10 @@ __global__ void __launch_bounds__(MS_NT) ms_push_kernel(MsArgs a) {
 // over every CTA.
 __global__ void __launch_bounds__(MS_NT) ms_push_big_kernel(MsArgs a) {
   __shared__ BigSmem<MS_NT> sm;
-  if (ms_skip(a, 0)) return;
+  __shared__ MsEnter en;
+  if (ms_skip(a, 0, en)) return;
   DevCtl *c = a.ctl;
-  const int cur = vload(&c->cur);
+  const int cur = en.cur;
   const uint64_t *fcur = cur ? a.f1 : a.f0;
   const uint64_t *seen = a.seen;
   unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc);
@@ -164,43 +244,59 @@ __global__ void __launch_bounds__(MS_NT) ms_push_big_kernel(MsArgs a) {
 }
 
 // Commits a level: new bits = accumulated & ~seen; rewrites every vertex's
-// next-frontier mask and clears the accumulators it read. In vertex order, so the
-// stores of a depth row are coalesced whichever way the level ran.
+// next-frontier mask and clears the accumulators it read, in vertex order. Latency
+// bounds it (three dependent loads per new vertex), so a thread has MS_FV vertices in
+// flight and a warp stages its appends. R-MAT s20, 64 sources, the fullest level: 44 us
+// with one vertex in flight and an atomic on the queue's length per 32 vertices, 34 us now.
 __global__ void __launch_bounds__(MS_NT) ms_finish_kernel(MsArgs a) {
   __shared__ int64_t s_sum[MS_NT / 32 + 1];
+  __shared__ int32_t s_stage[MS_NT / 32][WS_CAP];
+  __shared__ MsEnter en;
+  if (ms_skip(a, -1, en)) return;
   DevCtl *c = a.ctl;
-  if (vload(&c->done)) {
-    loop_over(a.ctl, a.h, a.use_cond);
-    return;
-  }
-  const int cur = vload(&c->cur);
-  const int32_t d = vload(&c->level) + 1;
+  const int cur = en.cur;
+  const int32_t d = en.level + 1;
   uint64_t *fnext = cur ? a.f0 : a.f1;
   int32_t *qout = cur ? a.q0 : a.q1;
   int32_t *qlen_out = &c->qlen[cur ^ 1];
+  WarpStage st{s_stage[warp_id()], 0};
   int64_t mf = 0, vdeg = 0;
   const int64_t stride = (int64_t)gridDim.x * MS_NT;
-  for (int64_t base = (int64_t)blockIdx.x * MS_NT; base < a.n; base += stride) {
-    const int64_t w = base + threadIdx.x;
-    uint64_t nw = 0;
-    if (w < a.n) {
-      const uint64_t ac = a.acc[w];
-      if (ac) {
-        a.acc[w] = 0;
-        const uint64_t s = a.seen[w];
-        nw = ac & ~s;
-        if (nw) {
-          a.seen[w] = s | nw;
-          const int64_t deg = a.ro[w + 1] - a.ro[w];
-          mf += deg;
-          vdeg += deg * __popcll(nw);
-        }
-      }
-      fnext[w] = nw;
+  for (int64_t base = (int64_t)blockIdx.x * MS_NT; base < a.n; base += MS_FV * stride) {
+    uint64_t ac[MS_FV], s[MS_FV];
+    int32_t r0[MS_FV], r1[MS_FV];
+#pragma unroll
+    for (int j = 0; j < MS_FV; j++) {
+      const int64_t w = base + j * stride + threadIdx.x;
+      ac[j] = w < a.n ? a.acc[w] : 0;
     }
-    ms_write_depths(a.depth, a.n, w, nw, d);
-    warp_append(nw != 0, (int32_t)w, qout, qlen_out, a.qcap, &c->overflow);
+#pragma unroll
+    for (int j = 0; j < MS_FV; j++) {
+      const int64_t w = base + j * stride + threadIdx.x;
+      s[j] = ac[j] || (d == 1 << MS_PLANES && w < a.n) ? a.seen[w] : 0;
+      r0[j] = ac[j] ? __ldg(a.ro + w) : 0;
+      r1[j] = ac[j] ? __ldg(a.ro + w + 1) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < MS_FV; j++) {
+      const int64_t w = base + j * stride + threadIdx.x;
+      const uint64_t nw = ac[j] & ~s[j];
+      if (w < a.n) {
+        if (ac[j]) a.acc[w] = 0;
+        if (nw) {
+          a.seen[w] = s[j] | nw;
+          mf += r1[j] - r0[j];
+          vdeg += (int64_t)(r1[j] - r0[j]) * __popcll(nw);
+        }
+        fnext[w] = nw;
+        if (d < 1 << MS_PLANES) ms_plane(a, w, nw, d);
+        else if (d == 1 << MS_PLANES) ms_emit_rows(a, w, s[j], nw, d - 1);
+      }
+      if (d > 1 << MS_PLANES) ms_write_depths(a.depth, a.n, w, nw, d);
+      ws_push(st, nw != 0, (int32_t)w, qout, qlen_out, a.qcap, &c->overflow);
+    }
   }
+  ws_flush(st, qout, qlen_out, a.qcap, &c->overflow);
   const int64_t bmf = block_sum<MS_NT>(mf, s_sum);
   const int64_t bvd = block_sum<MS_NT>(vdeg, s_sum);
   if (threadIdx.x == 0) {
@@ -222,9 +318,10 @@ __global__ void __launch_bounds__(MS_NT) ms_finish_kernel(MsArgs a) {
 // `second`: the out-edges' pass of an undirected run, on top of the first.
 __global__ void __launch_bounds__(MS_NT) ms_pull_kernel(MsArgs a, PrbArgs p, int second) {
   __shared__ int64_t s_sum[MS_NT / 32 + 1];
-  if (ms_skip(a, 1)) return;
+  __shared__ MsEnter en;
+  if (ms_skip(a, 1, en)) return;
   DevCtl *c = a.ctl;
-  const uint64_t *__restrict__ fcur = vload(&c->cur) ? a.f1 : a.f0;
+  const uint64_t *__restrict__ fcur = en.cur ? a.f1 : a.f0;
   unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc);
   int64_t insp = 0, nexp = 0;
   prb_walk(p, [&](auto lanes, int32_t row, int32_t b, int32_t e, int sub, int64_t task, int64_t) {
@@ -271,8 +368,8 @@ __global__ void __launch_bounds__(MS_NT) ms_pull_kernel(MsArgs a, PrbArgs p, int
   }
 }
 
-// Masks := 0; the group's depth rows := -1.
-__global__ void ms_clear_kernel(MsArgs a, int32_t k) {
+// Masks := 0.
+__global__ void ms_clear_kernel(MsArgs a) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {
     a.seen[i] = 0;
@@ -280,8 +377,6 @@ __global__ void ms_clear_kernel(MsArgs a, int32_t k) {
     a.f1[i] = 0;
     a.acc[i] = 0;
   }
-  const int64_t total = (int64_t)k * a.n;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) a.depth[i] = -1;
 }
 
 // Seeds the group's sources (bit i for srcs[i]; equal sources share a vertex).
@@ -296,7 +391,6 @@ __global__ void ms_seed_kernel(MsArgs a, const int32_t *srcs, int32_t k, int32_t
     const unsigned long long bit = 1ull << i;
     const int64_t deg = a.ro[s + 1] - a.ro[s];
     atomicOr(seen + s, bit);
-    a.depth[(int64_t)i * a.n + s] = 0;
     vdeg += deg;
     if (atomicOr(f0 + s, bit) == 0ull) {
       mf += deg;
@@ -309,6 +403,7 @@ __global__ void ms_seed_kernel(MsArgs a, const int32_t *srcs, int32_t k, int32_t
   const int64_t tv = block_sum<1024>(vdeg, s_sum);
   if (threadIdx.x == 0) {
     c->visited_deg = tv;
+    c->mf_front = tm;
     c->mf_next = 0;
     c->level = 0;
     c->cur = 0;
@@ -340,7 +435,7 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
                                    sizeof(uint64_t) * (size_t)n, sizeof(uint64_t) * (size_t)n,
                                    sizeof(int32_t) * (size_t)n, sizeof(int32_t) * (size_t)n,
                                    sizeof(int32_t) * (size_t)BIG_CAP, sizeof(int32_t) * (size_t)nsrc,
-                                   sizeof(int32_t) * 2});
+                                   sizeof(int32_t) * 2, sizeof(uint64_t) * (size_t)n * MS_PLANES});
   MG_TRY(ws_reserve(g, g->ws_main, need));
   Carve cv(g->ws_main.ptr);
   MsArgs a;
@@ -354,6 +449,8 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
   a.big_v = cv.take<int32_t>(BIG_CAP);
   int32_t *dsrc = cv.take<int32_t>(nsrc);
   a.grab = cv.take<int32_t>(2);
+  uint64_t *planes = cv.take<uint64_t>(n * MS_PLANES);
+  for (int b = 0; b < MS_PLANES; b++) a.plane[b] = planes + b * n;
   a.qcap = (int32_t)n;
   a.ro = g->ro;
   a.ci = g->ci;
@@ -392,7 +489,7 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
     a.full = k == 64 ? ~0ull : ((1ull << k) - 1);
     MG_CUDA_TRY(cudaEventRecord(g->ev0, s));
     MG_CUDA_TRY(cudaMemsetAsync(g->ctl, 0, sizeof(DevCtl), s));
-    ms_clear_kernel<<<g->num_sms * 8, 256, 0, s>>>(a, k);
+    ms_clear_kernel<<<g->num_sms * 8, 256, 0, s>>>(a);
     ms_seed_kernel<<<1, 1024, 0, s>>>(a, dsrc + g0, k, iter_cap, dir0);
     MG_CUDA_TRY(cudaGetLastError());
     struct Sig {
@@ -416,6 +513,8 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
       ms_finish_kernel<<<grid, MS_NT, 0, st>>>(b);
     };
     MG_TRY(run_loop(g, SLOT_MSBFS, &sig, sizeof(sig), o.use_graph, body, n + 2));
+    ms_rows_kernel<<<g->num_sms * 8, MS_NT, 0, s>>>(a);
+    MG_CUDA_TRY(cudaGetLastError());
     MG_CUDA_TRY(cudaEventRecord(g->ev1, s));
     MG_TRY(fetch_ctl(g));
     const DevCtl &hc = *g->ctl_host;
@@ -431,7 +530,7 @@ static mg_status msbfs_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32
     insp += hc.edges_inspected;
     pulls += hc.levels_pull;
     const int64_t per = 3 + (pull ? 1 + a.both : 0);
-    launches += 2 + loop_launches(g, per);
+    launches += 3 + loop_launches(g, per);
   }
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));

@@ -230,6 +230,28 @@ def test_cc_sparse(n, m, sym):
         np.testing.assert_array_equal(g.cc()[0], oracle.cc(ro, ci))
 
 
+@pytest.mark.parametrize("depth", [1, 30, 31, 32, 33, 34, 70])
+@pytest.mark.parametrize("k", [1, 9, 33, 64, 65])
+@pytest.mark.parametrize("directed", [0, 1])
+def test_bfs_batch_levels(depth, k, directed):
+    """The level at which the depth rows are written, with sources that are done by then and some beyond it."""
+    rng = np.random.default_rng(depth)
+    n = depth + 1 + 90
+    src = np.concatenate([np.arange(depth), rng.integers(depth + 1, n, 150)])
+    dst = np.concatenate([np.arange(1, depth + 1), rng.integers(depth + 1, n, 150)])
+    ro, ci, w = _csr(n, src, dst, np.ones(src.size, dtype=np.int32))
+    srcs = [0] + [int(v) for v in rng.integers(0, n, k - 1)]
+    ref = np.stack([oracle.bfs(ro, ci, [s], directed=directed) for s in srcs])
+    with mg.Graph(ro, ci) as g:
+        for direction in ("auto", "push", "pull"):
+            d, st = g.bfs_batch(srcs, directed=directed, direction=direction)
+            np.testing.assert_array_equal(d, ref)
+            assert st["edges_traversed"] == int((np.diff(ro)[None] * (ref >= 0)).sum())
+        for cap in (1, 31, 32, 33):
+            d, _ = g.bfs_batch(srcs, directed=directed, iter_num=cap)
+            np.testing.assert_array_equal(d, np.where(ref <= cap, ref, -1))
+
+
 @pytest.mark.parametrize("wide,deg", [(37, 9000), (5000, 40), (5000, 200), (40000, 20)])
 def test_bfs_skewed_frontier(wide, deg):
     """A sparse graph whose second level holds most of the edges: few vertices per warp,
