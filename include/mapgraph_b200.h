@@ -419,7 +419,8 @@ typedef struct mg_tuning {
   int32_t bfs_tail_max;     /* push levels of at most this many frontier vertices ... [512; 0 .. 2^30] */
   int32_t bfs_tail_edges;   /* ... and out-edges run one after another in a single CTA, one launch for the
                                run of them, wherever they occur (0: never) [16384; 0 .. 2^30] */
-  int32_t cc_rounds;        /* CC: rounds that link every vertex to its next neighbour before the largest sampled
+  int32_t cc_rounds;        /* CC: rounds beyond the first that hook every vertex's tree to its next two
+                               neighbours' (one more on graphs of up to 4 edges per vertex) before the largest
                                component is picked and only the vertices outside it read their other edges
                                [1; 0 .. 8] */
   int32_t reserved[15];
@@ -433,9 +434,9 @@ mg_status mg_graph_get_tuning(mg_graph *g, mg_tuning *t);
  * mg_debug_fail_alloc(k): the k-th device allocation from now, and every later
  *   one, fails as if the device were out of memory (the call in progress returns
  *   MG_ERR_OOM); k = 0 disarms.
- * mg_debug_barrier_skew(extra, poll_limit): the persistent BFS kernel's grid
- *   barriers wait for `extra` arrivals more than there are blocks, polling at
- *   most poll_limit times, so the next mg_bfs that takes the persistent path
+ * mg_debug_barrier_skew(extra, poll_limit): the grid barriers of the persistent
+ *   BFS and SSSP kernels wait for `extra` arrivals more than there are blocks,
+ *   polling at most poll_limit times, so the next call that takes such a kernel
  *   returns MG_ERR_TIMEOUT and leaves the device usable; extra = 0 restores. */
 mg_status mg_debug_fail_alloc(int64_t k);
 mg_status mg_debug_barrier_skew(int32_t extra, int64_t poll_limit);

@@ -116,8 +116,7 @@ __device__ __forceinline__ bool ms_skip(const MsArgs &a, int want_dir, MsEnter &
 
 // Depths while the levels are few (fewer than 1 << MS_PLANES). A level that stores
 // its new depths writes each row in pieces, the sector of a row at several levels, and
-// the rows had to be set to -1 first: R-MAT s20, 64 sources, 268 MB of rows, clearing 43 us and most of
-// the finishing passes.
+// the rows had to be set to -1 first (R-MAT s20, 64 sources, 268 MB of rows: 43 us).
 // Instead digit b of a vertex's 64 depths is kept in one word, plane[b][v]; a level
 // ORs its new bits into the planes of its own digits, and the rows are written once,
 // complete, at the end of the run (or at level 1 << MS_PLANES, from where on
