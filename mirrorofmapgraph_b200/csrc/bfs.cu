@@ -3,7 +3,7 @@
 // Per level one of two kernels does the work and the last CTA to finish closes
 // the level (swap queues, pick the next direction, stop or continue):
 //
-//  push (top-down)  input: vertex queue. Each CTA takes a tile of 256 frontier
+//  push (top-down)  input: vertex queue. Each CTA takes a tile of up to 256 frontier
 //                   vertices and bins them by out-degree: >= CTA_TH edges are
 //                   expanded by the whole CTA, >= 32 by one warp, the rest by a
 //                   block-wide scan over the remaining degrees (thread-level
