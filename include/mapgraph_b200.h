@@ -255,6 +255,9 @@ mg_status mg_bfs_ragged(mg_graph *g, const int32_t *srcs, int32_t *depth, const 
  *   dL/dt_i  = lambda_i * (1 - alpha + alpha * d)                      (n)
  * with a the F32 edge values (unit weights when opts->weighted == 0), s_u their
  * row sums, x = ranks from mg_pagerank with the same options, d its dangling mass.
+ * t need not sum to 1 (a larger sum may leave no solution on graphs with dangling
+ * vertices). tol (default 1e-7) bounds the last change of lambda relative to w; FP32
+ * rounding may end the solve before that.
  * Either gradient pointer may be NULL. nvec must be 1. */
 mg_status mg_pagerank_backward(mg_graph *g, const float *teleport, const float *ranks,
                                const float *dL_dranks, float *dL_dweights, float *dL_dteleport,

@@ -71,6 +71,26 @@ __device__ __forceinline__ T block_sum(T v, T *smem) {
   return r;  // valid in thread 0 only
 }
 
+// K block-wide sums at once, in block_sum's order: thread k < K ends with the k-th in v[0].
+// smem: K * (NT / 32) entries, not in use by an earlier call that no barrier follows.
+template <int NT, int K, typename T>
+__device__ __forceinline__ void block_sums(T (&v)[K], T *smem) {
+  constexpr int W = NT / 32;
+#pragma unroll
+  for (int k = 0; k < K; k++) v[k] = warp_sum(v[k]);
+  if (lane_id() == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k++) smem[k * W + warp_id()] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < K) {
+    T r = T(0);
+#pragma unroll
+    for (int i = 0; i < W; i++) r += smem[threadIdx.x * W + i];
+    v[0] = r;
+  }
+}
+
 // Last-block-done election: every CTA calls this once after finishing its work
 // (all threads). Returns true in every thread of the last CTA to arrive. Writes
 // made by any CTA before its call are visible to the last CTA afterwards.

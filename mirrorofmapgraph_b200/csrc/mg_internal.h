@@ -83,6 +83,14 @@ struct DevCtl {
   int64_t se[3];
   uint32_t reports;  // iterations reported to the host (engine.cuh, launches ahead)
   uint32_t pad;
+  // PageRank adjoint (adjoint_end): sums of the running iteration, and what one iteration
+  // hands to the next
+  double adj_sum[4];
+  double adj_mean;   // expected constant part of the next change
+  double adj_tau;    // sum of the teleport vector
+  double adj_prev;   // 2-norm of the last change without its constant part
+  double adj_floor;  // iterations that left that norm at the FP32 rounding of the iterate
+  double adj_shift;  // constant to add to the final iterate
 };
 
 // Padding of the device graph arrays. Offsets arrays hold n + 1 + MG_OFF_PAD
