@@ -214,6 +214,9 @@ inline volatile unsigned long long *graph_mailbox(mg_graph *g) {
   return reinterpret_cast<volatile unsigned long long *>(reinterpret_cast<char *>(g->ctl_host) + MG_MAIL_OFF);
 }
 
+// Exclusive scan of n int32 counts into n + 1 offsets; tmp: ceil(n / 2048) int64 values.
+mg_status device_exclusive_scan(const int32_t *in, int32_t *out, int64_t n, int64_t *tmp, cudaStream_t s);
+
 // Grows a workspace to at least `bytes` (contents are not preserved).
 mg_status ws_reserve(mg_graph *g, Workspace &w, size_t bytes);
 

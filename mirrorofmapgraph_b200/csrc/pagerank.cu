@@ -784,18 +784,21 @@ __global__ void __launch_bounds__(256) hub_hist_kernel(const int32_t *__restrict
     if (sh[i]) atomicAdd(hist + i, sh[i]);
 }
 
-__global__ void hub_slot_kernel(const int32_t *__restrict__ ro, int64_t n, int32_t thr, int32_t cap, int32_t *slot,
-                                int32_t *hv, unsigned *count) {
+// Slots in vertex order, so that a cache built again for the same capacity is the same
+// cache: the segmented plan holds slot numbers and outlives it. flag[v]: 1 for the cached
+// vertices; first: its exclusive prefix.
+__global__ void hub_flag_kernel(const int32_t *__restrict__ ro, int64_t n, int32_t thr, int32_t *__restrict__ flag) {
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+    flag[v] = ro[v + 1] - ro[v] >= thr;
+}
+
+__global__ void hub_slot_kernel(const int32_t *__restrict__ first, int64_t n, int32_t cap, int32_t *slot,
+                                int32_t *hv) {
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-    int32_t sl = -1;
-    if (ro[v + 1] - ro[v] >= thr) {
-      const unsigned t = atomicAdd(count, 1u);
-      if ((int32_t)t < cap) {
-        sl = (int32_t)t;
-        hv[sl] = (int32_t)v;
-      }
-    }
-    slot[v] = sl;
+    const int32_t t = first[v];
+    const bool in = slot[v] && t < cap;
+    if (in) hv[t] = (int32_t)v;
+    slot[v] = in ? t : -1;
   }
 }
 
@@ -1036,13 +1039,17 @@ static mg_status get_hub_cache(mg_graph *g, int32_t cap, mg::HubCache **out) {
     const int64_t n = g->n, m = g->m;
     cudaStream_t s = g->stream;
     unsigned *hist = nullptr;
-    MG_CUDA_TRY(mg_malloc_async((void **)&hist, sizeof(unsigned) * (65536 + 1), s));
+    const size_t ntiles = (size_t)(n / 2048 + 2);
+    MG_CUDA_TRY(mg_malloc_async((void **)&hist, sizeof(unsigned) * 65536 + sizeof(int64_t) * ntiles +
+                                                    sizeof(int32_t) * (size_t)(n + 1), s));
+    int64_t *tiles = reinterpret_cast<int64_t *>(hist + 65536);
+    int32_t *first = reinterpret_cast<int32_t *>(tiles + ntiles);
     auto alloc = [&](void **q, size_t bytes) -> mg_status {
       const mg_status st = dev_alloc(g, q, bytes);
       if (st != MG_OK) dev_free(g, hist);
       return st;
     };
-    MG_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(unsigned) * (65536 + 1), s));
+    MG_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(unsigned) * 65536, s));
     hub_hist_kernel<<<g->num_sms * 4, 256, 0, s>>>(g->ro, n, hist);
     std::vector<unsigned> h(65536);
     MG_CUDA_TRY(cudaMemcpyAsync(h.data(), hist, sizeof(unsigned) * 65536, cudaMemcpyDeviceToHost, s));
@@ -1057,14 +1064,15 @@ static mg_status get_hub_cache(mg_graph *g, int32_t cap, mg::HubCache **out) {
     MG_TRY(alloc((void **)&hc.slot, sizeof(int32_t) * std::max<int64_t>(n, 1)));
     MG_TRY(alloc((void **)&hc.hv, sizeof(int32_t) * std::max<int64_t>(cap, 1)));
     MG_TRY(alloc((void **)&hc.cidx, sizeof(int32_t) * (m + 8)));
-    unsigned *count = hist + 65536;
-    hub_slot_kernel<<<g->num_sms * 4, 256, 0, s>>>(g->ro, n, thr, cap, hc.slot, hc.hv, count);
+    hub_flag_kernel<<<g->num_sms * 4, 256, 0, s>>>(g->ro, n, thr, hc.slot);
+    MG_TRY(device_exclusive_scan(hc.slot, first, n, tiles, s));
+    hub_slot_kernel<<<g->num_sms * 4, 256, 0, s>>>(first, n, cap, hc.slot, hc.hv);
     hub_remap_kernel<<<g->num_sms * 8, 256, 0, s>>>(g->ri, m, hc.slot, hc.cidx);
-    unsigned k = 0;
-    MG_CUDA_TRY(cudaMemcpyAsync(&k, count, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    int32_t k = 0;
+    MG_CUDA_TRY(cudaMemcpyAsync(&k, first + n, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     MG_CUDA_TRY(cudaStreamSynchronize(s));
     MG_CUDA_TRY(cudaFreeAsync(hist, s));
-    hc.K = (int32_t)std::min<unsigned>(k, (unsigned)cap);
+    hc.K = std::min(k, cap);
     hc.cap = cap;
     hc.ok = true;
   }
@@ -1096,6 +1104,7 @@ static mg_status seg_plan_build(mg_graph *g, int32_t T, int32_t S, bool weighted
   }
   sp.T = T;
   sp.S = S;
+  sp.cap = hc.cap;
   sp.nblocks = (int32_t)B;
   sp.grid = g->num_sms;
   sp.weighted = weighted;
@@ -1320,12 +1329,12 @@ static mg_status seg_plan_build(mg_graph *g, int32_t T, int32_t S, bool weighted
   return MG_OK;
 }
 
-// Segmented plan for (T, S), rebuilt when either changes; a failed build leaves
-// nothing behind.
+// Segmented plan for (T, S) and the column cache's capacity, rebuilt when one of them
+// changes; a failed build leaves nothing behind.
 static mg_status get_seg_plan(mg_graph *g, int32_t T, int32_t S, bool weighted, const mg::HubCache &hc,
                               mg::SegPlan **out) {
   mg::SegPlan &sp = plans_of(g)->seg;
-  if (!sp.ok || sp.T != T || sp.S != S || sp.weighted != weighted) {
+  if (!sp.ok || sp.T != T || sp.S != S || sp.cap != hc.cap || sp.weighted != weighted) {
     seg_plan_release(g, sp);
     const mg_status st = seg_plan_build(g, T, S, weighted, hc, sp);
     if (st != MG_OK) {

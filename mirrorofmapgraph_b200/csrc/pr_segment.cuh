@@ -83,7 +83,8 @@ __host__ __device__ __forceinline__ int32_t seg_swz(int32_t c) {
 // Plan of the forward (CSC) gather, built once per graph and (T, S).
 struct SegPlan {
   int32_t T = 0, S = 0, nblocks = 0, grid = 0;
-  BinPlan bins;              // rows below T in bins 0..5; rows of >= T edges are its hubs;
+  int32_t cap = 0;           // capacity of the column cache whose slots the plan holds
+  BinPlan bins;              // rows below T in bins 0..11; rows of >= T edges are its hubs;
                              // hbase / hpart count fragments instead of fixed chunks
   int32_t *sidx = nullptr;   // m + 8 indices: rows below T with cached columns as
                              // (slot | 0x80000000); hub rows block-grouped (plan scratch)

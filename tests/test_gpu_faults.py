@@ -54,6 +54,34 @@ def test_allocation_failures_surface_as_oom_and_leave_the_library_usable():
     np.testing.assert_array_equal(clean["bfs"], oracle.bfs(h.row_offsets, h.col_idx, [0]))
 
 
+def test_segmented_plan_outlives_its_column_cache():
+    """The segmented plan holds slot numbers of the column cache. A tuning run drops the cache for one of
+    another capacity and fails on the way: the cache that the next segmented solve builds must be the one
+    the plan knows."""
+    lib = L.load()
+    h = mg.gen_rmat(17, 8, 5, symmetrize=False)
+    ref = oracle.pr_normalized(h.row_offsets, h.col_idx, None, 0.85, 0.0, 2)[0]
+    kw = dict(mode="normalized", gather="segmented", seg_hub_edges=64, max_iter=2, tol=1e-30)
+    dropped = 0
+    with mg.Graph(h.row_offsets, h.col_idx) as g:
+        try:
+            for k in range(1, 30):
+                assert np.abs(g.pagerank(**kw)[0] - ref).sum() <= 1e-6
+                lib.mg_debug_fail_alloc(k)
+                try:
+                    g.pagerank(mode="normalized", autotune=True)
+                    break  # the tuning run got by with fewer allocations
+                except mg.MapGraphError as e:
+                    assert e.status == L.MG_ERR_OOM
+                    dropped += 1
+                finally:
+                    lib.mg_debug_fail_alloc(0)
+                assert np.abs(g.pagerank(**kw)[0] - ref).sum() <= 1e-6
+        finally:
+            lib.mg_debug_fail_alloc(0)
+    assert dropped >= 3
+
+
 def test_barrier_that_cannot_complete_times_out_and_the_device_stays_usable():
     lib = L.load()
     h = mg.gen_lattice(300, 200, 0.0, 5)  # small frontiers: the persistent BFS kernel runs
