@@ -93,6 +93,10 @@ struct DevCtl {
   double adj_shift;  // constant to add to the final iterate
 };
 
+// Batched SSSP keeps 32 distances per vertex and group: the first one of row `row`
+// (past 2^31 from row 2^26 on, past 2^32 from 2^27).
+__host__ __device__ inline int64_t mss_row(int64_t row) { return row << 5; }
+
 // Padding of the device graph arrays. Offsets arrays hold n + 1 + MG_OFF_PAD
 // entries (the pad is INT_MAX) and edge arrays m + MG_EDGE_PAD entries (the pad is
 // 0), so 16-byte-aligned bulk copies that round a range outwards stay inside the

@@ -831,6 +831,15 @@ struct MssArgs {
   int32_t use_cond;
 };
 
+// Dl + mss_row(u): one multiply-add where it is used. Volatile, or the compiler keeps
+// eight 64-bit addresses from the first look to the last and spills (R-MAT s20, 64
+// sources: 11.1 against 14.1 ms).
+__device__ __forceinline__ int32_t *mss_at(int32_t *Dl, int32_t u) {
+  uint64_t p;
+  asm volatile("mad.wide.u32 %0, %1, 128, %2;" : "=l"(p) : "r"(u), "l"(Dl));
+  return reinterpret_cast<int32_t *>(p);
+}
+
 // Relaxes MSS_U staged edges (head, weight) from the vertex whose row this lane's
 // instance reads as dv (act: the lane's instance improved that vertex last round;
 // INT_MAX otherwise). Dl: this lane's column of the group's distance rows, mg: the
@@ -858,19 +867,19 @@ __device__ __forceinline__ void mss_step(const int2 *se, int32_t *Dl, uint32_t *
     nd[r + 1] = dv + (uint32_t)p.w;
   }
 #pragma unroll
-  for (int r = 0; r < MSS_U; r++) cu[r] = act ? (uint32_t)__ldca(Dl + ((uint32_t)u[r] << 5)) : 0u;
+  for (int r = 0; r < MSS_U; r++) cu[r] = act ? (uint32_t)__ldca(mss_at(Dl, u[r])) : 0u;
   bool any = false;
 #pragma unroll
   for (int r = 0; r < MSS_U; r++) any |= nd[r] < cu[r];
   if (!__any_sync(FULL, any)) return;
 #pragma unroll
-  for (int r = 0; r < MSS_U; r++) cu[r] = nd[r] < cu[r] ? (uint32_t)__ldcg(Dl + ((uint32_t)u[r] << 5)) : 0u;
+  for (int r = 0; r < MSS_U; r++) cu[r] = nd[r] < cu[r] ? (uint32_t)__ldcg(mss_at(Dl, u[r])) : 0u;
   uint32_t myb = 0;
   int32_t myv = 0;
 #pragma unroll
   for (int r = 0; r < MSS_U; r++) {
     const bool tr = nd[r] < cu[r];
-    if (tr) red_min(Dl + ((uint32_t)u[r] << 5), (int32_t)nd[r]);
+    if (tr) red_min(mss_at(Dl, u[r]), (int32_t)nd[r]);
     const uint32_t bits = __ballot_sync(FULL, tr);
     if (lane_id() == r) {
       myb = bits;
@@ -891,7 +900,7 @@ __device__ __forceinline__ void mss_edges(const MssArgs &a, int2 *se, uint32_t *
                                           int32_t dv, const int32_t *__restrict__ adj,
                                           const int32_t *__restrict__ wt, int32_t k0, int32_t k1, int64_t &updates) {
   const int lane = lane_id();
-  int32_t *Dl = a.D + (gbase << 5) + lane;
+  int32_t *Dl = a.D + mss_row(gbase) + lane;
   for (int32_t b = k0; b < k1; b += MSS_CH) {
     const int32_t cnt = min(MSS_CH, k1 - b);
 #pragma unroll
@@ -1012,7 +1021,7 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_relax_kernel(MssArgs a) {
         const int32_t sb = __shfl_sync(FULL, beg, j);
         const int32_t d = __shfl_sync(FULL, deg, j);
         sd[q] = have ? d : 0;
-        dv[q] = have && ((sm[q] >> lane) & 1u) ? __ldcg(a.D + (srow << 5) + lane) : INT_MAX;
+        dv[q] = have && ((sm[q] >> lane) & 1u) ? __ldcg(a.D + mss_row(srow) + lane) : INT_MAX;
         const bool in = lane < sd[q];
         se[q * 32 + lane] = make_int2(in ? a.ci[sb + lane] : 0, in ? (a.w ? a.w[sb + lane] : 1) : INT_MAX);
       }
@@ -1021,7 +1030,7 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_relax_kernel(MssArgs a) {
       for (int q = 0; q < 4; q++) {
         const int64_t gbase = (int64_t)(sit[q] >> a.shift) * a.n;
         for (int32_t e0 = 0; e0 < sd[q]; e0 += MSS_U)
-          mss_step(se + q * 32 + e0, a.D + (gbase << 5) + lane, mnext + gbase, (sm[q] >> lane) & 1u, (uint32_t)dv[q], upd);
+          mss_step(se + q * 32 + e0, a.D + mss_row(gbase) + lane, mnext + gbase, (sm[q] >> lane) & 1u, (uint32_t)dv[q], upd);
       }
       __syncwarp();
     }
@@ -1036,7 +1045,7 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_relax_kernel(MssArgs a) {
       const uint32_t sm = __shfl_sync(FULL, mask, j);
       const int64_t gbase = (int64_t)(sit >> a.shift) * a.n;
       const bool act = (sm >> lane) & 1u;
-      const int32_t dv = act ? __ldcg(a.D + (srow << 5) + lane) : INT_MAX;
+      const int32_t dv = act ? __ldcg(a.D + mss_row(srow) + lane) : INT_MAX;
       const int32_t sb = __shfl_sync(FULL, beg, j), sd = __shfl_sync(FULL, deg, j);
       int2 *se = s_edges[warp_id()];
       if (sd) mss_edges(a, se, mnext, gbase, act, dv, a.ci, a.w, sb, sb + sd, upd);
@@ -1072,7 +1081,7 @@ __global__ void __launch_bounds__(SSSP_NT, 4) mss_chunk_kernel(MssArgs a) {
     if (e.x < 0) return;
     const int32_t v = e.x & a.vmask;
     end = min((e.y & INT_MAX) + MSS_CH, (e.y < 0 ? a.co : a.ro)[v + 1]);
-    if (((uint32_t)e.z >> lane) & 1u) dv = __ldcg(a.D + (((int64_t)(e.x >> a.shift) * a.n + v) << 5) + lane);
+    if (((uint32_t)e.z >> lane) & 1u) dv = __ldcg(a.D + mss_row((int64_t)(e.x >> a.shift) * a.n + v) + lane);
   };
   int32_t ch = blockIdx.x * (SSSP_NT / 32) + warp_id();
   int4 e = header(ch), e1 = header(ch + nw);
@@ -1162,7 +1171,7 @@ __global__ void mss_seed_kernel(MssArgs a, const int32_t *srcs, int32_t nsrc, in
     const int32_t s = srcs[i];
     const int32_t g = i >> 5;
     const int64_t row = (int64_t)g * a.n + s;
-    a.D[(row << 5) + (i & 31)] = 0;
+    a.D[mss_row(row) + (i & 31)] = 0;
     if (atomicOr(a.m0 + row, 1u << (i & 31)) == 0u) {
       const int pos = atomicAdd(&c->qlen[0], 1);
       if (pos < a.qcap) a.q0[pos] = (g << a.shift) | s;
@@ -1190,7 +1199,7 @@ __global__ void __launch_bounds__(1024) mss_unpack_kernel(MssArgs a, int32_t *di
     const int64_t v0 = (tile % vtiles) << 5;
     const int64_t v = v0 + wy;
     __syncthreads();
-    t[wy][lane] = v < a.n ? a.D[(((int64_t)g * a.n + v) << 5) + lane] : INT_MAX;
+    t[wy][lane] = v < a.n ? a.D[mss_row((int64_t)g * a.n + v) + lane] : INT_MAX;
     __syncthreads();
     // thread (wy, lane): instance g * 32 + wy, vertex v0 + lane
     const int32_t inst = g * 32 + wy;

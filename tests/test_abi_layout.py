@@ -51,3 +51,21 @@ def test_ctypes_structs_match_the_header(tmp_path):
         assert got[(cname, "size")] == C.sizeof(cls), cname
         for fname, _ in cls._fields_:
             assert got[(cname, fname)] == getattr(cls, fname).offset, (cname, fname)
+
+
+def test_batched_sssp_row_offsets_past_32_bits(tmp_path):
+    """Offsets into the interleaved distance rows (mss_row), and that the kernels use nothing else: a
+    vertex from 2^27 on lies past 2^32 distances, on a graph too large for a test."""
+    rows = [0, 1, 2**26 - 1, 2**26, 2**27 - 1, 2**27, 140_000_000, 2**31 - 1, 2**33]
+    src = tmp_path / "rows.cu"
+    src.write_text('#include "mg_internal.h"\nint main() {\n' +
+                   "".join(f'  printf("%lld\\n", (long long)mss_row({r}ll));\n' for r in rows) + "}\n")
+    exe = tmp_path / "rows"
+    r = subprocess.run([_build.NVCC] + _build.NVCC_FLAGS + [str(src), "-o", str(exe)], capture_output=True, text=True)
+    if r.returncode != 0:
+        pytest.fail("row offset probe did not compile:\n" + r.stderr)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout
+    assert [int(x) for x in out.split()] == [32 * r for r in rows]
+    with open(os.path.join(_build.CSRC, "sssp.cu")) as f:
+        text = f.read()
+    assert text.count("<< 5") == text.count("(tile % vtiles) << 5")  # a tile's first vertex
