@@ -331,6 +331,9 @@ __global__ void __launch_bounds__(MS_NT) ms_pull_kernel(MsArgs a, PrbArgs p, int
       // bits an earlier chunk or pass has brought already
       if (miss && (task >= 0 || second)) miss &= ~__ldcg(a.acc + row);
     }
+    // The other chunks of a hub add to its accumulator meanwhile, so the lanes may have
+    // read different words, and the loop below, which the warp leaves together, ends by it.
+    if constexpr (L == 32) miss = __shfl_sync(FULL, miss, 0);
     if (sub == 0 && miss && task < 0 && !second) nexp++;
     if (!miss) e = b;
     uint64_t got = 0;

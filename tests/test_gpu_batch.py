@@ -255,3 +255,27 @@ def test_ppr_group_width_and_autotuned_width(width):
         assert np.abs(xa - xs).sum() <= 1e-9 * 150
         with pytest.raises(mg.MapGraphError):
             g.pagerank(teleport=tele, nvec=150, mode="normalized", group_width=48)
+
+
+@pytest.mark.parametrize("directed", [0, 1])
+@pytest.mark.parametrize("k", [1, 33, 64, 65])
+def test_bfs_batch_hubs_of_many_chunks(directed, k):
+    """Bottom-up levels in which many warps add to one hub's accumulator at a time: hubs of 40 to 400 chunks
+    in both directions, sources that reach them through different chunks."""
+    rng = np.random.default_rng(k)
+    n, hubs = 30000, 5
+    src, dst = [], []
+    for h in range(hubs):
+        m = 2048 * (40 + 90 * h) + h
+        src += [rng.integers(hubs, n, m), np.full(m, h)]
+        dst += [np.full(m, h), rng.integers(hubs, n, m)]
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    order = np.argsort(src, kind="stable")
+    ro = np.searchsorted(src[order], np.arange(n + 1)).astype(np.int32)
+    ci = dst[order].astype(np.int32)
+    srcs = [int(v) for v in rng.integers(hubs, n, k)]
+    ref = np.stack([oracle.bfs(ro, ci, [s], directed=directed) for s in srcs])
+    with mg.Graph(ro, ci) as g:
+        for direction in ("pull", "auto", "pull"):
+            d, st = g.bfs_batch(srcs, directed=directed, direction=direction)
+            np.testing.assert_array_equal(d, ref)
