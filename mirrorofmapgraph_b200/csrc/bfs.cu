@@ -683,7 +683,7 @@ __global__ void __cluster_dims__(SB_CLUSTER, 1, 1) __launch_bounds__(SB_NT, 1)
   cl.sync();
   int32_t nin = len[0];
   int32_t lvl = 0, sel = 0;
-  bool over = vload(&c->overflow) != 0;
+  bool over = nin > a.qcap;  // from the level's own length, see its end
   bool done = over || sb.iter_cap <= 0;
   int64_t insp = 0, nexp = 0, vdeg = 0;
   // claims the items u (-1: none) of a lane, issued together
@@ -787,10 +787,12 @@ __global__ void __cluster_dims__(SB_CLUSTER, 1, 1) __launch_bounds__(SB_NT, 1)
     }
     bq_flush(bq, qout, qlen, a.qcap, &c->overflow);
     cl.sync();
-    // Level end, alike in every CTA.
+    // Level end, alike in every CTA: a CTA that leaves takes its shared memory with it. So
+    // an overflow shows in the level's length, which counts what did not fit; the flag in
+    // the control block may be a faster CTA's, from the next level.
     const int64_t mf = (int64_t)mfs[out];
     const int32_t nf = len[out];
-    over = vload(&c->overflow) != 0;
+    over = nf > a.qcap;
     if (lead) {
       trace_level(c, lvl, MG_DIR_PUSH, nin, mf, 0.0);
       vdeg += mf;

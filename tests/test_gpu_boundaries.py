@@ -7,6 +7,7 @@ import pytest
 
 import oracle
 import mirrorofmapgraph_b200 as mg
+from mirrorofmapgraph_b200 import _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -367,3 +368,28 @@ def test_batched_ranks_sparse_rows(nvec):
         tele[1, n - 1] = np.inf
         zs, st = g.pagerank(teleport=tele, nvec=nvec, mode="normalized", weighted=True, max_iter=5)
         assert np.isfinite(zs[0]).all() and not np.isfinite(zs[1]).all()
+
+
+def _capacities(run, ref, widths, n):
+    """Runs with queues of just the widest frontier, and of one less than every frontier."""
+    def sized(cap):
+        return run(queue_sizing=(cap - 0.5) / n)  # rounded up
+
+    for _ in range(20):
+        np.testing.assert_array_equal(sized(int(widths.max())), ref)
+        for cap in sorted({int(w) - 1 for w in widths if w > 1}):
+            with pytest.raises(mg.MapGraphError) as e:
+                sized(cap)
+            assert e.value.status == L.MG_ERR_QUEUE_OVERFLOW
+        np.testing.assert_array_equal(run(), ref)
+
+
+@pytest.mark.parametrize("directed", [0, 1])
+def test_small_bfs_queue_capacity(directed):
+    """The run ends in every CTA alike, at any level, and the next one is right."""
+    rng = np.random.default_rng(2)
+    n, m = 20000, 50000
+    ro, ci, _ = _csr(n, rng.integers(0, n, m), rng.integers(0, n, m))
+    ref = oracle.bfs(ro, ci, [0], directed=directed)
+    with mg.Graph(ro, ci) as g:
+        _capacities(lambda **kw: g.bfs([0], directed=directed, **kw)[0], ref, np.bincount(ref[ref >= 0]), n)
