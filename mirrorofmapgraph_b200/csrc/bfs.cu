@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
   // Read by one thread per block (at entry, and behind each barrier): every warp of
   // the grid reading one L2 sector queues for microseconds.
   __shared__ struct {
-    int32_t lvl, sel, nin, cap, skip, pq, pb, over, ok;
+    int32_t lvl, sel, nin, cap, skip, pq, pb, ok;
     int64_t mf, vdeg, pm;
     uint32_t *vis;
   } s_c;
@@ -316,7 +316,6 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
       s_c.pq = vload(&c->pq[out]);
       s_c.pb = vload(&c->pb[out]);
       s_c.pm = vload(&c->pm[out]);
-      s_c.over = vload(&c->overflow);
       s_c.ok = ok;
     }
     __syncthreads();
@@ -387,7 +386,7 @@ __global__ void __launch_bounds__(BFS_NT) bfs_persist_kernel(BfsArgs a) {
     vdeg += mf;
     lvl += 1;
     sel ^= 1;
-    const bool over = s_c.over != 0;
+    const bool over = nf > a.qcap;  // not the flag: a faster block may have set it in the next level
     const bool done = nf == 0 || lvl >= iter_cap || over;
     int dir = 0;
     if (a.mode == MG_DIR_PULL) dir = a.can_pull ? 1 : 0;

@@ -393,3 +393,11 @@ def test_small_bfs_queue_capacity(directed):
     ref = oracle.bfs(ro, ci, [0], directed=directed)
     with mg.Graph(ro, ci) as g:
         _capacities(lambda **kw: g.bfs([0], directed=directed, **kw)[0], ref, np.bincount(ref[ref >= 0]), n)
+
+
+def test_persistent_bfs_queue_capacity():
+    h = mg.gen_lattice(400, 500, 0.001, 4)  # past the cluster BFS; every level within the one-launch limits
+    ref = oracle.bfs(h.row_offsets, h.col_idx, [0])
+    widths = np.bincount(ref)
+    with mg.Graph(h.row_offsets, h.col_idx, symmetric=True) as g:
+        _capacities(lambda **kw: g.bfs([0], **kw)[0], ref, widths[np.argsort(widths)[-3:]], h.n)
