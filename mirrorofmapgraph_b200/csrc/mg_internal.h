@@ -76,7 +76,9 @@ struct DevCtl {
   uint32_t bar_count;
   uint32_t bar_gen;
   // persistent near-far SSSP: per-step counters in a ring of three (near items
-  // appended, chunks, edges of the frontier, smallest waiting distance)
+  // appended, chunks, edges of the frontier, smallest waiting distance, whether an
+  // append ran past capacity)
+  int32_t so[3];
   int32_t sq[3];
   int32_t sc[3];
   int32_t smin[3];

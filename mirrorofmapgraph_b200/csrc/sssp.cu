@@ -552,7 +552,8 @@ __global__ void __launch_bounds__(SSSP_NT) sssp_far_split_kernel(SsspArgs a) {
 //
 // Counters rotate over three slots, one per step (a round or a split): a step adds
 // to its own slot and block 0 clears the next step's, which was last read two steps
-// ago, so at least one barrier lies between.
+// ago, so at least one barrier lies between. That goes for the overflow flag too: a
+// block past the barrier may run over in the next step before the last one has read it.
 constexpr int NF_NT = 1024;
 // Plain rounds in one launch up to this many edges: R-MAT of mean degree 32, 0.5 M /
 // 4 M / 8 M edges 260 / 487 / 824 us against 363 / 525 / 712 for the per-round kernels
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
       s_c.smin = vload(&c->smin[slot]);
       s_c.far[0] = vload(&c->far_len[0]);
       s_c.far[1] = vload(&c->far_len[1]);
-      s_c.over = vload(&c->overflow);
+      s_c.over = vload(&c->so[slot]);
       s_c.ok = in;
     }
     __syncthreads();
@@ -611,6 +612,7 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
     const int slot = step % 3, z = (step + 1) % 3;
     step++;
     if (lead) {
+      c->so[z] = 0;
       c->sq[z] = 0;
       c->sc[z] = 0;
       c->se[z] = 0;
@@ -622,7 +624,7 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
     const int slot = next_slot();
     const int32_t *qin = sel ? a.q1 : a.q0;
     uint32_t *inq_cur = sel ? a.inq1 : a.inq0;
-    RelaxCtx x{a.dist, sel ? a.inq0 : a.inq1, a.ro, sel ? a.q0 : a.q1, &c->sq[slot], &c->overflow, a.qcap, a.vmask, 0,
+    RelaxCtx x{a.dist, sel ? a.inq0 : a.inq1, a.ro, sel ? a.q0 : a.q1, &c->sq[slot], &c->so[slot], a.qcap, a.vmask, 0,
                a.delta, thr, a.infar, fc ? a.far1 : a.far0, &c->far_len[fc]};
     WarpStage st{s_stage[warp_id()], 0};
     const int32_t th = nin < nw * 32 ? a.heavy_small : a.heavy;
@@ -711,8 +713,8 @@ __global__ void __launch_bounds__(NF_NT, 1) sssp_persist_kernel(SsspArgs a) {
           }
         }
         __syncwarp();
-        warp_append(to_near, u, qnear, &c->sq[sp], a.qcap, &c->overflow);
-        warp_append(keep, u, keep_to, &c->far_len[fc ^ 1], a.qcap, &c->overflow);
+        warp_append(to_near, u, qnear, &c->sq[sp], a.qcap, &c->so[sp]);
+        warp_append(keep, u, keep_to, &c->far_len[fc ^ 1], a.qcap, &c->so[sp]);
       }
       if (!(ok = barrier(sp))) break;
       nf = s_c.sq;
@@ -1412,7 +1414,7 @@ static mg_status sssp_core(mg_graph *g, const int32_t *seeds, int32_t nseed, int
     stats->status_detail = delta > 0 ? delta : 0;
   }
   if (hc.status == MG_ERR_TIMEOUT) {
-    mg_set_error("mg_sssp: a grid barrier of the near-far rounds timed out");
+    mg_set_error("mg_sssp: a grid barrier of the one-launch rounds timed out");
     return MG_ERR_TIMEOUT;
   }
   if (hc.status != 0) {

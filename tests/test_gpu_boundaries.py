@@ -401,3 +401,29 @@ def test_persistent_bfs_queue_capacity():
     widths = np.bincount(ref)
     with mg.Graph(h.row_offsets, h.col_idx, symmetric=True) as g:
         _capacities(lambda **kw: g.bfs([0], **kw)[0], ref, widths[np.argsort(widths)[-3:]], h.n)
+
+
+@pytest.mark.parametrize("kind", ["near_far", "plain", "per_round", "batch"])
+def test_sssp_queue_capacity(kind):
+    """Queues too small for a round: in the one-launch rounds, near-far and plain (near frontier, far pile),
+    in the per-round kernels, and with several instances per run. Each is followed by a correct run."""
+    if kind == "plain":
+        h = mg.gen_rmat(14, 16, 6, symmetrize=True, weights="int", p0=1, p1=50)
+    else:
+        h = mg.gen_lattice(300, 200, 0.001, 4, weights="int", p0=1, p1=1000)
+    srcs = [0, 7] if kind == "batch" else [0]
+    kw = dict(use_graph="graph") if kind == "per_round" else {}
+    if kind == "batch":
+        kw["delta"] = 500
+    ref = np.stack([oracle.sssp(h.row_offsets, h.col_idx, h.weights_i32, [s]) for s in srcs])
+    with mg.Graph(h.row_offsets, h.col_idx, h.weights_i32, symmetric=True) as g:
+        for _ in range(10):
+            for size in (0.5 / h.n, 3.5 / h.n, 20.5 / h.n, 0.002):
+                with pytest.raises(mg.MapGraphError) as e:
+                    if kind == "batch":
+                        g.sssp_batch(srcs, queue_sizing=size, **kw)
+                    else:
+                        g.sssp(srcs, queue_sizing=size, **kw)
+                assert e.value.status == L.MG_ERR_QUEUE_OVERFLOW
+            d = g.sssp_batch(srcs, **kw)[0] if kind == "batch" else g.sssp(srcs, **kw)[0][None]
+            np.testing.assert_array_equal(d, ref)

@@ -101,6 +101,22 @@ def test_barrier_that_cannot_complete_times_out_and_the_device_stays_usable():
     assert lib.mg_debug_fail_alloc(-3) == L.MG_ERR_ARG
 
 
+@pytest.mark.parametrize("delta", [0, -1])
+def test_sssp_barrier_that_cannot_complete_times_out(delta):
+    lib = L.load()
+    h = mg.gen_lattice(120, 100, 0.0, 5, weights="int", p0=1, p1=100)  # near-far and plain rounds in one launch
+    ref = oracle.sssp(h.row_offsets, h.col_idx, h.weights_i32, [0])
+    with mg.Graph(h.row_offsets, h.col_idx, h.weights_i32, symmetric=True) as g:
+        try:
+            assert lib.mg_debug_barrier_skew(1, 1 << 12) == L.MG_OK
+            with pytest.raises(mg.MapGraphError) as ei:
+                g.sssp([0], delta=delta)
+            assert ei.value.status == L.MG_ERR_TIMEOUT
+        finally:
+            lib.mg_debug_barrier_skew(0, 1)
+        np.testing.assert_array_equal(g.sssp([0], delta=delta)[0], ref)
+
+
 def test_repeated_runs_are_bit_identical():
     # Integer outputs are bit-identical run to run. PageRank rows are too, except
     # that its FP64 residual and dangling-mass sums add per-CTA partials whose
