@@ -112,7 +112,8 @@ typedef struct mg_pr_opts {
   double alpha;          /* NORMALIZED damping [0.85] */
   double tol;            /* NORMALIZED: stop when the L1 change < tol [1e-6]; REFCOMPAT: active
                             while |dx| >= tol [0.01] */
-  int32_t compensated;   /* 1: two-sum compensated FP32 accumulation [1]; -1 plain FP32 sums */
+  int32_t compensated;   /* 1: two-sum compensated FP32 accumulation [1]; -1 plain FP32 sums (REFCOMPAT; the
+                            NORMALIZED solves always compensate) */
   int32_t device_output; /* 1: ranks/teleport/gradient arrays are device pointers */
   int32_t use_graph;     /* as mg_opts.use_graph */
   int32_t gather_kernel; /* NORMALIZED/adjoint gather: 0 degree-binned warps [default]; 1 merge-path tiles

@@ -1623,8 +1623,9 @@ struct RefArgs {
   int32_t use_cond;
 };
 
-// PASS 0: the only pass of a sweep; 1, 2: the two of a split one.
-template <int PASS>
+// PASS 0: the only pass of a sweep; 1, 2: the two of a split one. COMP: compensated sums
+// (mg_pr_opts.compensated), else a lane adds in plain FP32.
+template <int PASS, bool COMP>
 __global__ void __launch_bounds__(PRB_NT, PRR_MIN_BLOCKS) prr_sweep_kernel(RefArgs a) {
   __shared__ int64_t s_sum[PRB_NT / 32 + 1];
   DevCtl *c = a.ctl;
@@ -1679,7 +1680,7 @@ __global__ void __launch_bounds__(PRB_NT, PRR_MIN_BLOCKS) prr_sweep_kernel(RefAr
   prb_walk(p, [&](auto lanes, int32_t row, int32_t b, int32_t e, int sub, int64_t task, int64_t h) {
     constexpr int L = decltype(lanes)::value;
     any = false;
-    Comp acc = prb_range<L, false>(p, b, e, sub, gather);
+    Comp acc = prb_range<L, false, COMP>(p, b, e, sub, gather);
     bool act = any;
     if (L == 32) act = __any_sync(FULL, any);
     if (L == 4) act = (__ballot_sync(FULL, any) >> (lane_id() & ~3)) & 0xfu;
@@ -1800,20 +1801,23 @@ static mg_status pagerank_refcompat(mg_graph *g, float *ranks, const mg_pr_opts 
   const int grid = g->num_sms * PRR_MIN_BLOCKS;
   struct Sig {
     RefArgs a;
-    int grid;
+    int grid, comp;
   } sig;
   std::memset(&sig, 0, sizeof(sig));
   sig.a = a;
   sig.grid = grid;
-  LoopBody body = [a, grid](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) {
+  const bool comp = o.compensated >= 0;
+  sig.comp = comp;
+  LoopBody body = [a, grid, comp](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) {
     RefArgs b = a;
     b.h = h;
     b.use_cond = use_cond;
+    const auto sweep = [&](auto *with, auto *without) { (comp ? with : without)<<<grid, PRB_NT, 0, st>>>(b); };
     if (b.split) {
-      prr_sweep_kernel<1><<<grid, PRB_NT, 0, st>>>(b);
-      prr_sweep_kernel<2><<<grid, PRB_NT, 0, st>>>(b);
+      sweep(prr_sweep_kernel<1, true>, prr_sweep_kernel<1, false>);
+      sweep(prr_sweep_kernel<2, true>, prr_sweep_kernel<2, false>);
     } else {
-      prr_sweep_kernel<0><<<grid, PRB_NT, 0, st>>>(b);
+      sweep(prr_sweep_kernel<0, true>, prr_sweep_kernel<0, false>);
     }
   };
   MG_TRY(run_loop(g, SLOT_PR_REF, &sig, sizeof(sig), o.use_graph, body, (int64_t)cap + 2, true));

@@ -321,7 +321,7 @@ __device__ __forceinline__ float cached_gather(uint32_t cache, uint32_t zero, co
 // a load of 32 random columns, and lookups bound this kernel: 32-byte loads make it
 // an eighth of a lookup per index against a quarter with 16-byte loads (weighted
 // R-MAT s22 iteration 380 us with those, 338 with these).
-template <int L, bool WEIGHTED, typename Gather>
+template <int L, bool WEIGHTED, bool COMP, typename Gather>
 __device__ __forceinline__ Comp prb_group_range(const PrbArgs &p, int32_t b, int32_t e, int sub, Gather &gather) {
   Comp acc{0.f, 0.f};
   for (int32_t k0 = (b & ~7) + 8 * sub; k0 < e; k0 += 8 * L) {
@@ -341,8 +341,10 @@ __device__ __forceinline__ Comp prb_group_range(const PrbArgs &p, int32_t b, int
         const float pr = w[j] * x[j];
         two_sum_add(acc, pr);
         acc.lo += __fmaf_rn(w[j], x[j], -pr);
-      } else {
+      } else if (COMP) {
         two_sum_add(acc, x[j]);
+      } else {
+        acc.hi += x[j];
       }
     }
   }
@@ -351,7 +353,7 @@ __device__ __forceinline__ Comp prb_group_range(const PrbArgs &p, int32_t b, int
 }
 
 // Rows of up to 2 edges, one lane each, plain index loads.
-template <bool WEIGHTED, typename Gather>
+template <bool WEIGHTED, bool COMP, typename Gather>
 __device__ __forceinline__ Comp prb_short_range(const PrbArgs &p, int32_t b, int32_t e, Gather &gather) {
   Comp acc{0.f, 0.f};
   int32_t c[2];
@@ -369,8 +371,10 @@ __device__ __forceinline__ Comp prb_short_range(const PrbArgs &p, int32_t b, int
       const float pr = w[j] * x[j];
       two_sum_add(acc, pr);
       acc.lo += __fmaf_rn(w[j], x[j], -pr);
-    } else {
+    } else if (COMP) {
       two_sum_add(acc, x[j]);
+    } else {
+      acc.hi += x[j];
     }
   }
   return acc;
@@ -441,11 +445,12 @@ __device__ __forceinline__ void prb_walk(const PrbArgs &p, Body &&body) {
   });
 }
 
-// A lane's share (prb_walk's L and sub) of the compensated sum of edges [b, e).
-template <int L, bool WEIGHTED, typename Gather>
+// A lane's share (prb_walk's L and sub) of the compensated sum of edges [b, e); COMP
+// false: its own additions are plain FP32 (unweighted sums only).
+template <int L, bool WEIGHTED, bool COMP = true, typename Gather>
 __device__ __forceinline__ Comp prb_range(const PrbArgs &p, int32_t b, int32_t e, int sub, Gather &gather) {
-  if constexpr (L == 0) return prb_short_range<WEIGHTED>(p, b, e, gather);
-  else return prb_group_range<L, WEIGHTED>(p, b, e, sub, gather);
+  if constexpr (L == 0) return prb_short_range<WEIGHTED, COMP>(p, b, e, gather);
+  else return prb_group_range<L, WEIGHTED, COMP>(p, b, e, sub, gather);
 }
 
 // A hub chunk's partial: stored, and the lane that stores the last one of hub h

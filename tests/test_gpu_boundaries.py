@@ -148,6 +148,23 @@ def test_refcompat_sweep(directed, sym):
             assert np.abs(x - xr).max() <= 1e-5 * max(1.0, np.abs(xr).max())
 
 
+@pytest.mark.parametrize("directed,sym", [(1, False), (0, False), (0, True)])
+def test_refcompat_plain_sums(directed, sym):
+    """compensated=False: plain FP32 sums, in the sweep's three forms."""
+    n, ro, ci, _ = _in_degrees(BIN_DEGREES * 9, 8)
+    if sym:
+        src = np.repeat(np.arange(n), np.diff(ro))
+        ro, ci, _ = _csr(n, np.concatenate([src, ci]), np.concatenate([ci, src]))
+    with mg.Graph(ro, ci, symmetric=sym) as g:
+        a, _ = g.pagerank(mode="refcompat", directed=directed, max_iter=1)
+        b, _ = g.pagerank(mode="refcompat", directed=directed, max_iter=1, compensated=False)
+    xr, _ = oracle.pr_refcompat(ro, ci, directed, 1)
+    # ranks, terms and degrees in FP32: a few roundings; a lane adds at most 64 terms in a row
+    assert np.abs(a / xr - 1).max() <= 8 * 2.0**-24
+    assert np.abs(b / xr - 1).max() <= 72 * 2.0**-24
+    assert (a != b).any()  # some of the 234 rows round otherwise
+
+
 @pytest.mark.parametrize("kind", ["lattice", "hubs", "path", "one"])
 @pytest.mark.parametrize("directed", [0, 1])
 def test_near_far_rounds(kind, directed):
