@@ -81,9 +81,13 @@ __global__ void cc_init_kernel(int32_t *p, int64_t n) {
 
 // The first forest: p[v] = min(v, v's first CC_FIRST neighbours). Every vertex
 // writes only its own entry and pointers decrease, so there is no atomic and no
-// cycle.
+// cycle. Counts the edges that it and the hooking passes (hook_reads of every vertex
+// that has any) read.
 __global__ void __launch_bounds__(CC_NT) cc_first_kernel(const int32_t *__restrict__ ro,
-                                                         const int32_t *__restrict__ ci, int64_t n, int32_t *p) {
+                                                         const int32_t *__restrict__ ci, int64_t n, int32_t *p,
+                                                         int hook_reads, unsigned long long *insp_out) {
+  __shared__ int32_t s_insp[CC_NT / 32];
+  int32_t insp = 0;  // a block's share of the vertices keeps within 32 bits
   for (int64_t v = (int64_t)blockIdx.x * CC_NT + threadIdx.x; v < n; v += (int64_t)gridDim.x * CC_NT) {
     const int32_t b = ro[v], e = ro[v + 1];
     int32_t mn = (int32_t)v;
@@ -91,6 +95,14 @@ __global__ void __launch_bounds__(CC_NT) cc_first_kernel(const int32_t *__restri
     for (int k = 0; k < CC_FIRST; k++)
       if (b + k < e) mn = min(mn, ci[b + k]);
     p[v] = mn;
+    if (b < e) insp += min(e - b, CC_FIRST) + hook_reads;
+  }
+  insp = __reduce_add_sync(FULL, insp);
+  if (lane_id() == 0) s_insp[warp_id()] = insp;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < CC_NT / 32; w++) insp += s_insp[w];
+    if (insp) atomicAdd(insp_out, (unsigned long long)insp);
   }
 }
 
@@ -293,7 +305,7 @@ extern "C" mg_status mg_cc(mg_graph *g, int32_t *label, const mg_opts *opts, mg_
   const int64_t per = (int64_t)CC_NT * CC_V;
   const int gv = (int)std::min<int64_t>(std::max<int64_t>((n + per - 1) / per, 1), g->num_sms * 8);
   if (n > 0 && sampling) {
-    cc_first_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent);
+    cc_first_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent, CC_HOOK * (rounds + 1), insp);
     cc_compress_kernel<<<gv, CC_NT, 0, s>>>(parent, nullptr, n);
     for (int r = 0; r <= rounds; r++) {
       cc_hook_kernel<<<grid, CC_NT, 0, s>>>(g->ro, g->ci, n, parent, r * CC_HOOK);
@@ -317,7 +329,7 @@ extern "C" mg_status mg_cc(mg_graph *g, int32_t *label, const mg_opts *opts, mg_
     std::memset(stats, 0, sizeof(*stats));
     stats->iterations = 1;
     stats->edges_traversed = g->m;
-    stats->edges_inspected = g->ctl_host->edges_inspected + (sampling ? (int64_t)(rounds + 1) * n : 0);
+    stats->edges_inspected = g->ctl_host->edges_inspected;
     // offsets and sampled neighbours, the remaining edges actually read, parent
     // init / compress passes
     stats->bytes_compulsory = 4 * (n + 1) + 4 * stats->edges_inspected + 16 * n;

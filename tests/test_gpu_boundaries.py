@@ -133,6 +133,22 @@ def test_cc_forest(shape, sym):
             np.testing.assert_array_equal(g.cc()[0], oracle.cc(ro, ci))
 
 
+@pytest.mark.parametrize("clique,alone,passes", [(12, 3, 2), (40, 5, 2), (3, 50, 3), (2, 1, 3)])
+def test_cc_edges_inspected(clique, alone, passes):
+    """One clique that the first forest joins, and vertices without edges: the edges read are the first four
+    of a row and two per hooking pass (one pass more up to 4 edges per vertex)."""
+    src, dst = np.nonzero(~np.eye(clique, dtype=bool))
+    n = clique + alone
+    ro, ci, _ = _csr(n, src, dst)
+    with mg.Graph(ro, ci, symmetric=True) as g:
+        for rounds in (0, 1, 4):
+            g.set_tuning(cc_rounds=rounds)
+            label, st = g.cc()
+            np.testing.assert_array_equal(label, oracle.cc(ro, ci))
+            reads = min(clique - 1, 4) + 2 * (rounds + passes - 1)
+            assert st["edges_inspected"] == clique * reads
+
+
 @pytest.mark.parametrize("directed", [0, 1])
 @pytest.mark.parametrize("sym", [False, True])
 def test_refcompat_sweep(directed, sym):
