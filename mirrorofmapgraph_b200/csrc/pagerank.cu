@@ -627,9 +627,11 @@ constexpr int SEG_NT = 1024;
 
 template <bool WEIGHTED>
 __global__ void __launch_bounds__(SEG_NT, 1) solve_segment_kernel(SolveArgs a, PrbArgs p, SegArgs sg) {
+  // The block, a zero, the barrier and the counters: static variables take 128 bytes, and
+  // the widest block that fits, 58,080 columns, leaves less than that and the zero.
   extern __shared__ __align__(128) float s_buf[];
-  __shared__ __align__(8) uint64_t s_bar;
-  __shared__ int32_t s_next[2];
+  uint64_t &s_bar = *reinterpret_cast<uint64_t *>(s_buf + sg.S + 4);
+  int32_t *s_next = reinterpret_cast<int32_t *>(s_buf + sg.S + 6);
   if (solve_skip(a)) return;
   DevCtl *c = a.ctl;
   const int cur = vload(&c->cur);
@@ -1405,9 +1407,10 @@ static mg_status solve_setup(mg_graph *g, bool adjoint, bool weighted, const flo
   sp.use_tma = use_tma;
   sp.use_hub = use_hub && !use_seg;
   sp.use_seg = use_seg;
-  // the column cache and a column block, each with a zero behind it
+  // the column cache and a column block, each with a zero behind it (the block with 16
+  // bytes of the kernel's own besides)
   sp.hub_bytes = use_hub ? (int32_t)(sizeof(float) * hubs->K + 16) : 0;
-  sp.seg_bytes = use_seg ? (int32_t)(sizeof(float) * seg->S + 16) : 0;
+  sp.seg_bytes = use_seg ? (int32_t)(sizeof(float) * seg->S + 32) : 0;
   sp.weighted = weighted;
   sp.gather = nullptr;
   if (use_tma) sp.gather = gather_variant(weighted, nr, &occ);

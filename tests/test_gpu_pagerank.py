@@ -9,6 +9,7 @@ import pytest
 
 import oracle
 import mirrorofmapgraph_b200 as mg
+from mirrorofmapgraph_b200 import _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -269,3 +270,16 @@ def test_segmented_gather_rejects_bad_shapes():
         x, st = g.pagerank(mode="normalized", gather="segmented")  # the graph is still usable
     xr, _, _ = oracle.pr_normalized(h.row_offsets, h.col_idx, None, 0.85, 0.0, st["iterations"])
     assert np.abs(x - xr).sum() <= L1_TOL
+
+
+def test_segmented_widest_block():
+    """58,080 columns in a CTA's 227 KB of shared memory, with the kernel's own and the zero behind a block."""
+    h = mg.gen_rmat(18, 8, 4)
+    with mg.Graph(h.row_offsets, h.col_idx) as g:
+        kw = dict(mode="normalized", gather="segmented", seg_hub_edges=32, max_iter=3, tol=1e-30)
+        ref = oracle.pr_normalized(h.row_offsets, h.col_idx, None, 0.85, 0.0, 3)[0]
+        assert np.abs(g.pagerank(seg_block_cols=58080, **kw)[0] - ref).sum() <= 1e-6
+        with pytest.raises(mg.MapGraphError) as e:
+            g.pagerank(seg_block_cols=58112, **kw)
+        assert e.value.status == L.MG_ERR_UNSUPPORTED
+        assert np.abs(g.pagerank(**kw)[0] - ref).sum() <= 1e-6
