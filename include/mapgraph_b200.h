@@ -423,10 +423,10 @@ typedef struct mg_tuning {
   int32_t bfs_tail_max;     /* push levels of at most this many frontier vertices ... [512; 0 .. 2^30] */
   int32_t bfs_tail_edges;   /* ... and out-edges run one after another in a single CTA, one launch for the
                                run of them, wherever they occur (0: never) [16384; 0 .. 2^30] */
-  int32_t cc_rounds;        /* CC: rounds beyond the first that hook every vertex's tree to its next two
-                               neighbours' (one more on graphs of up to 4 edges per vertex) before the largest
-                               component is picked and only the vertices outside it read their other edges
-                               [1; 0 .. 8] */
+  int32_t cc_rounds;        /* CC: passes beyond the first that hook every vertex's tree to two neighbours'
+                               trees, counted round the row from its start (one more on graphs of up to 4 edges
+                               per vertex), before the largest component is picked and only the vertices outside
+                               it read their edges [1; 0 .. 8] */
   int32_t reserved[15];
 } mg_tuning;
 void mg_tuning_defaults(mg_tuning *t);

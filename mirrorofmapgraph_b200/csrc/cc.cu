@@ -15,10 +15,11 @@
 // The forest needs no union to succeed, so it is built without compare-and-swap:
 //   1. every vertex points at the smallest of itself and its first CC_FIRST
 //      neighbours, then the trees are compressed;
-//   2. 1 + mg_tuning.cc_rounds passes (one more on sparse graphs) over the next
-//      CC_HOOK neighbours hook the
-//      larger of the two roots under the smaller one by a fire-and-forget minimum,
-//      each followed by a compression; a root hooked twice keeps the smaller link;
+//   2. 1 + mg_tuning.cc_rounds passes (one more on sparse graphs) over CC_HOOK
+//      neighbours each, from the row's start again (by default the first four, which
+//      step 1 took the smallest of), hook the larger of the two roots under the
+//      smaller one by a fire-and-forget minimum, each followed by a compression; a
+//      root hooked twice keeps the smaller link;
 //   3. one CTA samples 1024 vertices and takes the most frequent root c (on
 //      power-law graphs, the giant component);
 //   4. only vertices outside c unite all their edges (and, without a symmetric
@@ -108,8 +109,8 @@ __global__ void __launch_bounds__(CC_NT) cc_first_kernel(const int32_t *__restri
 
 // Hooking pass over neighbours r0 .. r0 + CC_HOOK - 1 of every vertex, counted round
 // its row (a root keeps one of the links that a pass finds for it, so a short row's
-// neighbours are worth a second look), on compressed trees. Bound by its random parent reads. With atomicCAS unions in its place (one
-// neighbour each) the sampled roots are few and hot: R-MAT s22, rows in edge-list
+// neighbours are worth a second look), on compressed trees. Bound by its random parent
+// reads. With atomicCAS unions in its place (one neighbour each) the sampled roots are few and hot: R-MAT s22, rows in edge-list
 // order, 466 us from singletons and 737 us from the first forest; two passes of
 // this kernel and the whole run take 300 us.
 // Rows whose first neighbours are arbitrary need the minimum to spread: from

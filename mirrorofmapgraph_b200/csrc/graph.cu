@@ -495,13 +495,12 @@ __device__ __forceinline__ int64_t lower_bound_i32(const int32_t *__restrict__ a
   return lo;
 }
 
-// Column offsets from the sorted columns: a CTA brackets its columns first (2,048
-// columns per CTA in place of 256: 68 us against 35, R-MAT s20).
-constexpr int CO_VT = 1;
+// Column offsets from the sorted columns: a CTA brackets its 256 columns first (2,048
+// columns per CTA: 68 us against 35, R-MAT s20).
 __global__ void __launch_bounds__(256) csc_offsets_kernel(const int32_t *__restrict__ key, int64_t m, int64_t n,
                                                           int32_t *__restrict__ co) {
   __shared__ int64_t s_lo, s_hi;
-  const int64_t c0 = (int64_t)blockIdx.x * 256 * CO_VT, c1 = c0 + 256 * CO_VT;
+  const int64_t c0 = (int64_t)blockIdx.x * 256, c1 = c0 + 256;
   if (threadIdx.x == 0) s_lo = lower_bound_i32(key, 0, m, (int32_t)c0);
   if (threadIdx.x == 32) s_hi = c1 <= n ? lower_bound_i32(key, 0, m, (int32_t)(c1 - 1)) : m;
   __syncthreads();
@@ -610,7 +609,7 @@ static mg_status build_csc(mg_graph *g) {
     vin = vo;
     shift += b;
   }
-  csc_offsets_kernel<<<(unsigned)(n / (256 * CO_VT) + 1), 256, 0, s>>>(kin, m, n, g->co);
+  csc_offsets_kernel<<<(unsigned)(n / 256 + 1), 256, 0, s>>>(kin, m, n, g->co);
   // the sorted keys are done with: the pairs take their place
   const unsigned et = (unsigned)((m + 256 * EP_VT - 1) / (256 * EP_VT));
   const int grid = g->num_sms * 8;

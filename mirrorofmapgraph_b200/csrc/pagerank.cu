@@ -4,12 +4,14 @@
 // Two modes:
 //  NORMALIZED  x' = alpha * (P^T x + d t) + (1 - alpha) t over all vertices each
 //              iteration; P_uv = a_uv / s_u (a = 1 unweighted), d = rank mass on
-//              dangling vertices, t = teleport. One iteration is two kernels: the
-//              merge-path gather over the CSC (pr_gather.cuh) with the update fused
-//              into its epilogue (new x, new x/s for the next gather, |dx| and
-//              dangling-mass partials), then the fix-up of rows split across tiles,
-//              whose last CTA sums the FP64 partials in a fixed order and decides
-//              convergence on the device (L1 change < tol or max_iter).
+//              dangling vertices, t = teleport. An iteration gathers over the CSC
+//              with the update fused into the gather's epilogue (new x, new x/s for
+//              the next gather, |dx| and dangling-mass partials), and the last CTA
+//              sums the FP64 partials and decides convergence on the device (L1
+//              change < tol or max_iter). The degree-binned gathers are one kernel
+//              (pr_binned.cuh), the merge-path one has a second for rows split
+//              across tiles (pr_gather.cuh), the segmented one two phases
+//              (pr_segment.cuh).
 //  REFCOMPAT   the reference's program: x' = 0.15 + 0.85 * sum x_u / deg_u over the
 //              in-edges of the frontier, a vertex stays active while |dx| >= 0.01,
 //              the next frontier is the out-neighbourhood of the changed vertices

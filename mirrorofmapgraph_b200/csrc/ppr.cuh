@@ -30,7 +30,7 @@ constexpr int PPR_MAXW = 256;  // vectors per group
 struct PprArgs {
   const int32_t *off, *idx;  // CSC (gathered adjacency)
   const float *wts;          // its edge weights (nullptr: unit)
-  const int32_t *rows;       // non-hub rows of the bin plan (bins 0..5), plan order
+  const int32_t *rows;       // non-hub rows of the bin plan (bins 0..11), plan order
   int64_t nlight, nempty;  // rows; the first nempty of them have no in-edges
   const uint8_t *tflag;      // per row: some teleport entry of the group is not 0
   const int32_t *hrows, *hbase;  // hub rows and their first chunk

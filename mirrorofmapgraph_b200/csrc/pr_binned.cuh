@@ -251,7 +251,7 @@ struct PrbArgs {
   int32_t *hcount;
   Comp *hpart;
   double *hcontrib;
-  // Dynamic schedule: warps take PRB_GRAB work items at a time from this counter
+  // Dynamic schedule: warps take one work item at a time from this counter
   // (heaviest first) instead of a fixed grid stride; the launch's last CTA
   // resets it. nullptr: fixed stride.
   int32_t *grab;

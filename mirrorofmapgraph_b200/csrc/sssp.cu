@@ -6,12 +6,14 @@
 // edge-sized queue), contract (atomicMin into gather_tmp, cull duplicates)
 // (sssp.h:242-402, GASengine/enactor_vertex_centric.cuh:2561-2822).
 //
-// Here one kernel per iteration does all of it: each frontier vertex's edges are
-// expanded with the degree-binned tile expansion; an improving edge lowers
-// dist[u] directly with atomicMin, and the thread whose atomicMin won the
-// improvement claims u's bit in the next frontier's bitmap and appends it with a
-// warp-aggregated atomic. No edge-sized queue exists and duplicates never enter
-// the frontier. Distances are unique fixed points, so the result equals the
+// Here a round relaxes its frontier's edges in place. Warps walk the concatenated edges
+// of 32 frontier vertices; heavy vertices are cut into chunks that any warp takes. In
+// plain rounds an improving edge lowers dist[u] and marks u in the next frontier's bitmap
+// by two atomics nobody waits for, and the bitmap is compacted into the next queue. In
+// near-far rounds the edge whose atomicMin won the improvement claims u's bit and appends
+// it to the near frontier or the far pile; those rounds, and the plain ones of small
+// graphs, run in one cooperative launch. No edge-sized queue exists and duplicates never
+// enter the frontier. Distances are unique fixed points, so the result equals the
 // reference's bit for bit for any schedule.
 #include <algorithm>
 #include <climits>
@@ -167,8 +169,9 @@ __device__ __forceinline__ RelaxCtx relax_ctx(const SsspArgs &a, DevCtl *c, int 
 }
 
 // The edges of the warp's 32 vertices (lane l brings vertex item v, its distance
-// dv, its first edge beg and deg edges), concatenated and walked 32 x U at a time: edge slot j belongs to the last lane whose exclusive degree prefix is <= j
-// (binary search over the lanes' prefixes by shuffles).
+// dv, its first edge beg and deg edges), concatenated and walked 32 x U at a time: edge
+// slot j belongs to the last lane whose exclusive degree prefix is <= j (binary search
+// over the lanes' prefixes by shuffles).
 template <int U, bool FAR>
 __device__ __forceinline__ void warp_walk(RelaxCtx &x, WarpStage &st, int32_t v, int32_t dv, int32_t beg,
                                           int32_t deg, const int32_t *__restrict__ adj,

@@ -151,8 +151,11 @@ def _check_solve(ro, ci, w, t, dl, alpha, tol=1e-7, max_iter=400, gathers=("binn
             assert st["iterations"] <= min(1.1 * iters + 2, max_iter), (st["iterations"], iters)
 
 
-@pytest.mark.parametrize("dangling", [False, True])
-@pytest.mark.parametrize("tau", [0.0, 0.5, 0.8, 0.9, 0.999, 1.0, 1.0 + 1e-5, 1.3, 2.0, 500.0])
+_SUMS = [0.0, 0.5, 0.8, 0.9, 0.999, 1.0, 1.0 + 1e-5]
+
+
+@pytest.mark.parametrize("tau,dangling", [(t, d) for t in _SUMS for d in (False, True)] +
+                         [(1.3, False), (2.0, False), (500.0, False)])
 def test_adjoint_teleport_of_any_sum(tau, dangling):
     """The linear system has no need of a teleport vector that sums to 1, and gradient steps on one
     leave that sum; with rows without edges a larger sum may leave it without a solution that the
@@ -171,8 +174,6 @@ def test_adjoint_teleport_of_any_sum(tau, dangling):
         t /= np.abs(t).sum()
     else:
         t *= tau / t.sum()
-    if dangling and tau > 1.1:
-        pytest.skip("the iteration itself may diverge")
     _check_solve(ro, ci, w, t, rng.standard_normal(n), 0.85, gathers=("binned", "tma"))
 
 

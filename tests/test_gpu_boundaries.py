@@ -344,8 +344,9 @@ def test_plain_sssp_one_launch_limit(m):
 @pytest.mark.parametrize("shape", ["cut", "sinks", "cycle2"])
 @pytest.mark.parametrize("teleport", [False, True])
 def test_adjoint_settles(shape, teleport):
-    """The adjoint solve shifts by a constant each iteration, exact whatever the graph: closed parts,
-    rows without edges, a slow alternating mode, a sparse right-hand side. It settles at any tolerance."""
+    """The adjoint solve where the constant is not the slowest part of its error, or not the only one: closed
+    parts, rows without edges, a slow alternating mode, each with a loss on five vertices, whose tolerance
+    FP32 rounding hides."""
     rng = np.random.default_rng(5)
     n = 1500
     if shape == "cut":  # two halves without an edge between them
