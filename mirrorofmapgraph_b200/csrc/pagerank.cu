@@ -285,12 +285,9 @@ __device__ __forceinline__ double tele_of(const SolveArgs &a, int64_t r) {
   return a.tele ? (double)a.tele[r] : a.tn;
 }
 
-// Per-row update. Forward: x' = alpha (acc + d t) + (1 - alpha) t, g' = x'/s.
-// Adjoint: lambda' = w + alpha * (s > 0 ? acc / s : t.lambda). Partials: |change|
-// and (forward) dangling mass of x' / (adjoint) t . lambda', and adjoint_end's sums.
 // Sums of an adjoint iteration about `mean` (adjoint_end); the FP32 ones run over a
-// thread's own rows only and decide no more than when to stop (all four in FP64: 2% of
-// an iteration of R-MAT s22 directed).
+// thread's own rows only and decide no more than when to stop and which constant to add
+// (all four in FP64: 2% of an iteration of R-MAT s22 directed).
 struct AdjSums {
   double sq = 0.0;                     // (change - mean)^2
   float d1 = 0.f, l1 = 0.f, lam = 0.f;  // change - mean, its magnitude, lambda'^2
@@ -303,6 +300,9 @@ struct AdjSums {
   }
 };
 
+// Per-row update. Forward: x' = alpha (acc + d t) + (1 - alpha) t, g' = x'/s.
+// Adjoint: lambda' = w + alpha * (s > 0 ? acc / s : t.lambda). Partials: |change|
+// and (forward) dangling mass of x' / (adjoint) t . lambda', and adjoint_end's sums.
 // ADJ: 0 forward, 1 adjoint, -1 as the arguments say.
 template <int ADJ = -1>
 struct RowUpdate {
@@ -1003,10 +1003,23 @@ struct SolvePlan {
   const int32_t *ppos = nullptr;  // segmented: position of each row's x in v0 / v1
 };
 
+// Opts a kernel into all the dynamic shared memory that a block can have. The attribute
+// belongs to the kernel, not to a launch: set to what one graph's cache or block needs, it
+// fails the launch of another thread whose graph needs more.
+template <typename Kernel>
+static void allow_dynamic_smem(Kernel *kernel) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa;
+  if (cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+      cudaFuncGetAttributes(&fa, kernel) == cudaSuccess)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+}
+
 template <bool W>
 static int hub_occupancy(int32_t bytes) {
   int occ = 0;
-  cudaFuncSetAttribute(mg::solve_binned_hub_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  allow_dynamic_smem(mg::solve_binned_hub_kernel<W>);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mg::solve_binned_hub_kernel<W>, mg::PRB_HUB_NT, bytes);
   cudaGetLastError();
   return std::max(1, std::min(occ, PRB_HUB_MINB));
@@ -1015,7 +1028,7 @@ static int hub_occupancy(int32_t bytes) {
 template <bool W>
 static int seg_occupancy(int32_t bytes) {
   int occ = 0;
-  cudaFuncSetAttribute(mg::solve_segment_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  allow_dynamic_smem(mg::solve_segment_kernel<W>);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mg::solve_segment_kernel<W>, mg::SEG_NT, bytes);
   cudaGetLastError();
   return occ;
@@ -1426,10 +1439,10 @@ static mg_status solve_setup(mg_graph *g, bool adjoint, bool weighted, const flo
     // phase 1's ranges are cut for one CTA per SM; phase 2 runs one CTA per SM too
     int occ2 = 0;
     if (weighted) {
-      cudaFuncSetAttribute(solve_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.hub_bytes);
+      allow_dynamic_smem(solve_rows_kernel<true>);
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, solve_rows_kernel<true>, SEG_NT, sp.hub_bytes);
     } else {
-      cudaFuncSetAttribute(solve_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.hub_bytes);
+      allow_dynamic_smem(solve_rows_kernel<false>);
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, solve_rows_kernel<false>, SEG_NT, sp.hub_bytes);
     }
     cudaGetLastError();
